@@ -110,10 +110,10 @@ struct fiber_ctx {
     DevBuf d_params, d_inst, d_counters, d_lb, d_range_valid, d_ranges, d_keep, d_inst_visible, d_inst_keep;
     DevBuf d_lut_tree;  // per coarse tile: the slice lookup's search tree (kLutTreeWords)
     DevBuf d_lut, d_tasks, d_projected, d_page_table, d_page_meta, d_counts, d_offsets, d_cursors;
-    DevBuf d_refs, d_ref_keys, d_active_flags, d_active_list, d_work, d_runs, d_big_cells;
-    DevBuf d_visit_rec, d_visit_task, d_visit_rank, d_task_key, d_task_mat, d_cells_small, d_cells_mid, d_cells_large;
+    DevBuf d_active_flags, d_active_list, d_work, d_runs, d_big_cells;
+    DevBuf d_visit_rec, d_visit_task, d_visit_rank, d_task_key, d_cells_small, d_cells_mid, d_cells_large;
     DevBuf d_opaque;  // (covered, farthest depth q) per camera fine tile
-    DevBuf d_task_proj, d_ref_task;  // k_fine's projected end points per task; each reference's task
+    DevBuf d_task_rec, d_ref_task;  // the rasters' record of each task; each reference's task
     DevBuf d_page_nvis, d_page_vbase, d_page_bucket;  // page-CSR backend
     DevBuf d_tel, d_tel_slots;                         // prepass telemetry
     DevBuf d_dom_page_table, d_dom_pool;               // sparse DOM residency
@@ -234,8 +234,6 @@ PrepassArgs prepass_args(fiber_ctx* c) {
     A.counts = dp<uint32_t>(c->d_counts);
     A.offsets = dp<uint32_t>(c->d_offsets);
     A.cursors = dp<uint32_t>(c->d_cursors);
-    A.refs = dp<fiber_fine_seg_ref>(c->d_refs);
-    A.ref_keys = dp<uint32_t>(c->d_ref_keys);
     A.active_flags = dp<uint32_t>(c->d_active_flags);
     A.active_list = dp<uint32_t>(c->d_active_list);
     A.work = dp<fiber_raster_work_item>(c->d_work);
@@ -244,13 +242,12 @@ PrepassArgs prepass_args(fiber_ctx* c) {
     A.visit_rec = dp<uint32_t>(c->d_visit_rec);
     A.visit_task = dp<uint32_t>(c->d_visit_task);
     A.visit_rank = dp<uint32_t>(c->d_visit_rank);
-    A.task_key = dp<unsigned long long>(c->d_task_key);
-    A.task_mat = dp<uint32_t>(c->d_task_mat);
+    A.task_key = dp<uint32_t>(c->d_task_key);
     A.cells_small = dp<uint2>(c->d_cells_small);
     A.cells_mid = dp<uint2>(c->d_cells_mid);
     A.cells_large = dp<uint2>(c->d_cells_large);
     A.opaque_tiles = dp<uint2>(c->d_opaque);
-    A.task_proj = dp<float4>(c->d_task_proj);
+    A.task_rec = dp<float4>(c->d_task_rec);
     A.ref_task = dp<uint32_t>(c->d_ref_task);
     if (c->settings.telemetry_enabled) {
         A.tel = dp<uint32_t>(c->d_tel);
@@ -273,11 +270,10 @@ RenderArgs render_args(fiber_ctx* c) {
     RenderArgs R{};
     R.counters = dp<FrameCounters>(c->d_counters);
     R.tasks = dp<fiber_binning_task>(c->d_tasks);
-    R.refs = dp<fiber_fine_seg_ref>(c->d_refs);
     R.work = dp<fiber_raster_work_item>(c->d_work);
     R.runs = dp<fiber_raster_tile_run>(c->d_runs);
     R.ref_task = dp<uint32_t>(c->d_ref_task);
-    R.task_proj = dp<float4>(c->d_task_proj);
+    R.task_rec = dp<float4>(c->d_task_rec);
     R.dom_depth = dp<float>(c->d_dom_depth);
     R.dom_opacity = dp<float>(c->d_dom_opacity);
     R.dom_page_table = dp<uint32_t>(c->d_dom_page_table);
@@ -585,15 +581,15 @@ fiber_status fiber_ctx_destroy(fiber_ctx* c) {
             if (s.live && s.ptr) cudaFree(s.ptr);
     DevBuf* bufs[] = {&c->d_params, &c->d_inst, &c->d_counters, &c->d_lb, &c->d_range_valid, &c->d_ranges,
                       &c->d_keep, &c->d_inst_visible, &c->d_inst_keep, &c->d_lut, &c->d_lut_tree, &c->d_tasks, &c->d_projected,
-                      &c->d_page_table, &c->d_page_meta, &c->d_counts, &c->d_offsets, &c->d_cursors, &c->d_refs,
-                      &c->d_ref_keys, &c->d_active_flags, &c->d_active_list, &c->d_work, &c->d_runs,
+                      &c->d_page_table, &c->d_page_meta, &c->d_counts, &c->d_offsets, &c->d_cursors,
+                      &c->d_active_flags, &c->d_active_list, &c->d_work, &c->d_runs,
                       &c->d_big_cells, &c->d_dom_depth, &c->d_dom_opacity, &c->d_shadow_map, &c->d_atlas,
                       &c->d_history[0], &c->d_history[1], &c->d_color, &c->d_depth, &c->d_fragments,
                       &c->d_validate, &c->d_host_scene, &c->d_host_depth, &c->d_visit_rec,
-                      &c->d_visit_task, &c->d_visit_rank, &c->d_task_key, &c->d_task_mat,
+                      &c->d_visit_task, &c->d_visit_rank, &c->d_task_key,
                       &c->d_cells_small, &c->d_cells_mid, &c->d_cells_large, &c->d_opaque, &c->d_page_nvis, &c->d_page_vbase,
                       &c->d_page_bucket, &c->d_tel, &c->d_tel_slots, &c->d_dom_page_table, &c->d_dom_pool,
-                      &c->d_task_proj, &c->d_ref_task};
+                      &c->d_task_rec, &c->d_ref_task};
     for (DevBuf* b : bufs) release(c, *b);
     for (int i = 0; i <= kSpanCount; ++i)
         if (c->ev[i]) cudaEventDestroy(c->ev[i]);
@@ -962,8 +958,6 @@ static fiber_status frame_begin_views(fiber_ctx* c, const fiber_view* views, uin
     ENSURE(c->d_counts, page_cap * kPageSize * 4, false);
     ENSURE(c->d_offsets, page_cap * kPageSize * 4, false);
     ENSURE(c->d_cursors, page_cap * kPageSize * 4, false);
-    ENSURE(c->d_refs, ref_cap * sizeof(fiber_fine_seg_ref), false);
-    ENSURE(c->d_ref_keys, ref_cap * 4, false);
     ENSURE(c->d_active_flags, fine_tiles * 4, false);
     ENSURE(c->d_active_list, fine_tiles * 4, false);
     ENSURE(c->d_work, work_cap * sizeof(fiber_raster_work_item), false);
@@ -976,14 +970,13 @@ static fiber_status frame_begin_views(fiber_ctx* c, const fiber_view* views, uin
     ENSURE(c->d_visit_rec, visit_cap * 4, false);
     ENSURE(c->d_visit_task, visit_cap * 4, false);
     ENSURE(c->d_visit_rank, visit_cap * 4, false);
-    ENSURE(c->d_task_key, task_cap * 8, false);
-    ENSURE(c->d_task_mat, task_cap * 4, false);
+    ENSURE(c->d_task_key, task_cap * 4, false);
     // Non-empty cells: at most one per kept reference and one per cell.
     ENSURE(c->d_cells_small, std::min<uint64_t>(ref_cap, page_cap * kPageSize) * sizeof(uint2), false);
     ENSURE(c->d_cells_mid, (ref_cap / 9 + 1) * sizeof(uint2), false);
     ENSURE(c->d_cells_large, (ref_cap / 33 + 1) * sizeof(uint2), false);
     ENSURE(c->d_opaque, (uint64_t)c->camera_fine_tiles * sizeof(uint2), false);
-    ENSURE(c->d_task_proj, task_cap * 2 * sizeof(float4), false);
+    ENSURE(c->d_task_rec, task_cap * kTaskRec * sizeof(float4), false);
     ENSURE(c->d_ref_task, ref_cap * 4, false);
     if (st.telemetry_enabled) {
         ENSURE(c->d_tel, sizeof(fiber_telemetry), false);
@@ -1529,7 +1522,27 @@ fiber_status fiber_dump(fiber_ctx* c, uint32_t what, void* host, uint64_t capaci
         case FIBER_DUMP_PAGE_META: src = c->d_page_meta.p; bytes = (uint64_t)h.pages * 32; break;
         case FIBER_DUMP_COUNTS: src = c->d_counts.p; bytes = (uint64_t)h.pages * kPageSize * 4; break;
         case FIBER_DUMP_OFFSETS: src = c->d_offsets.p; bytes = (uint64_t)h.pages * kPageSize * 4; break;
-        case FIBER_DUMP_REFS: src = c->d_refs.p; bytes = (uint64_t)std::min(h.refs, P.ref_capacity) * 12; break;
+        case FIBER_DUMP_REFS: {
+            const uint64_t n = std::min(h.refs, P.ref_capacity);
+            bytes = n * sizeof(fiber_fine_seg_ref);
+            if (host && capacity >= bytes && n) {
+                // The records live for this call only, outside the frames' buffers.
+                DevBuf refs;
+                if (cudaMalloc(&refs.p, bytes) != cudaSuccess) {
+                    cudaGetLastError();
+                    return FIBER_ENOMEM;
+                }
+                launch_expand_refs(c->last_stream, dp<uint32_t>(c->d_ref_task), dp<float4>(c->d_task_rec),
+                                   std::min(h.tasks, P.task_capacity), n, dp<fiber_fine_seg_ref>(refs));
+                cudaError_t e = cudaGetLastError();
+                if (e == cudaSuccess) e = cudaStreamSynchronize(c->last_stream);
+                if (e == cudaSuccess) e = cudaMemcpy(host, refs.p, bytes, cudaMemcpyDeviceToHost);
+                cudaFree(refs.p);
+                if (written) *written = bytes;
+                return e == cudaSuccess ? FIBER_OK : FIBER_ECUDA;
+            }
+            break;  // the size alone, or a buffer that is too small
+        }
         case FIBER_DUMP_ACTIVE_TILES: src = c->d_active_list.p; bytes = (uint64_t)h.active_tiles * 4; break;
         case FIBER_DUMP_WORK: src = c->d_work.p; bytes = (uint64_t)std::min(h.work_items, P.work_capacity) * 32; break;
         case FIBER_DUMP_RUNS: src = c->d_runs.p; bytes = (uint64_t)h.active_tiles * 32; break;

@@ -109,12 +109,12 @@ struct FrameCounters {
     uint32_t tile_counter[8];     // virtual block ids of the look-back stages
     uint32_t visit_overflow;      // visit records unused this frame (did not fit, or disabled)
     unsigned long long visits;    // visit records appended by k_visit
-    uint32_t small_cells;         // cells of 1..8 references listed for the cell sort
+    uint32_t small_cells;         // cells of 2..8 references listed for the cell sort
     uint32_t large_cells;         // cells of more than 32 references listed for the cell sort
     uint32_t opaque_bound;        // the opaque fine-tile depths of this frame are written
     uint32_t dom_pages;           // DOM pages requested this frame (sparse residency)
     uint32_t mid_cells;           // cells of 9..32 references listed for the cell sort
-    uint32_t pad_counters;
+    uint32_t seg_unordered;       // some instance's strands do not follow one another in its index slab
 };
 static_assert(sizeof(FrameCounters) == 176 + 4 * (kMaxFrusta - 16), "FrameCounters layout");
 

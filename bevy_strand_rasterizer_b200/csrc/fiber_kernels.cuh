@@ -47,6 +47,13 @@ __device__ __forceinline__ uint2 pack_half4(float x, float y, float z, float w) 
     return make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
 }
 
+// A binning task's record for the rasters and the reference dump: its two end
+// points as world_to_screen_raw gave them, then the words (instance, segment,
+// material index, 0). A fine reference (FineSegRef) is a task index into it:
+// 4 B a reference instead of the 12 B record, and one 48 B read instead of the
+// reference, its task and its end points from three arrays.
+constexpr uint32_t kTaskRec = 3;  // float4 words
+
 // Device buffers of the work-preparation stages.
 struct PrepassArgs {
     uint32_t* tile_counter;          // virtual block ids of the current look-back stage
@@ -70,8 +77,6 @@ struct PrepassArgs {
     uint32_t* counts;
     uint32_t* offsets;
     uint32_t* cursors;
-    fiber_fine_seg_ref* refs;
-    uint32_t* ref_keys;
     uint32_t* active_flags;
     uint32_t* active_list;
     fiber_raster_work_item* work;
@@ -80,14 +85,13 @@ struct PrepassArgs {
     uint32_t* visit_rec;    // [ref_capacity] page-table slot << 8 | cell; the count pass rewrites it to the cell index
     uint32_t* visit_task;   // [ref_capacity] binning task of the visit
     uint32_t* visit_rank;   // [ref_capacity] rank of the visit inside its cell
-    unsigned long long* task_key;  // [task_capacity] canonical cell-order key of the task's reference
-    uint32_t* task_mat;            // [task_capacity] material index of the task's reference
-    uint2* cells_small;            // (ref base, count) of cells with 1..8 references
+    uint32_t* task_key;            // [task_capacity] depth key of the task's reference (projected z0 + z1, 17 bits)
+    uint2* cells_small;            // (ref base, count) of cells with 2..8 references
     uint2* cells_mid;              // (ref base, count) of cells with 9..32 references
-    uint2* cells_large;            // (ref base, count) of cells with more than 8
+    uint2* cells_large;            // (ref base, count) of cells with more than 32
     uint2* opaque_tiles;           // [camera fine tiles] (fully covered, quantised farthest opaque depth)
-    float4* task_proj;             // [task_capacity][2] both end points as world_to_screen_raw gave them
-    uint32_t* ref_task;            // [ref_capacity] binning task of each reference (after the cell sort)
+    float4* task_rec;              // [task_capacity][kTaskRec] what the rasters read of a task
+    uint32_t* ref_task;            // [ref_capacity] binning task of each reference (in cell order after the sort)
     // Page-CSR backend only (null otherwise).
     uint32_t* page_nvis;           // [page_capacity] visits per page
     uint32_t* page_vbase;          // [page_capacity] first bucket entry of each page
@@ -112,11 +116,10 @@ __device__ __forceinline__ uint32_t* tel_frustum(uint32_t* tel, uint32_t f, uint
 struct RenderArgs {
     FrameCounters* counters;
     const fiber_binning_task* tasks;
-    const fiber_fine_seg_ref* refs;
     const fiber_raster_work_item* work;
     const fiber_raster_tile_run* runs;
     const uint32_t* ref_task;    // [refs] binning task of each reference
-    const float4* task_proj;     // [tasks][2] the task's end points as k_fine projected them
+    const float4* task_rec;      // [tasks][kTaskRec] end points as k_fine projected them; instance, segment, material
     float* dom_depth;        // [L][D][D] (dense layers)
     float* dom_opacity;      // [L][K][D][D] (dense layers)
     uint32_t* dom_page_table;  // [L][pages_x][pages_x] pool page + 1 (sparse residency)
@@ -199,6 +202,10 @@ void launch_emit(const LaunchCtx& L, const PrepassArgs& A);
 void launch_sort_cells(const LaunchCtx& L, const PrepassArgs& A);
 void launch_sort_big(const LaunchCtx& L, const PrepassArgs& A);
 void launch_telemetry(const LaunchCtx& L, const PrepassArgs& A);
+// The FineSegRef records of references [0, n) as the reference keeps them, from
+// their tasks (tasks >= n_tasks: zeros).
+void launch_expand_refs(cudaStream_t s, const uint32_t* ref_task, const float4* task_rec, uint32_t n_tasks, uint64_t n,
+                        fiber_fine_seg_ref* out);
 
 void launch_shadow(const LaunchCtx& L, const RenderArgs& R, uint32_t K);
 void launch_dom_paging(const LaunchCtx& L, const RenderArgs& R, uint32_t table_entries);

@@ -17,6 +17,8 @@
 // persistent or grid-stride kernel that reads its item count on the device.
 // Append orders that the reference takes from atomics are replaced by
 // decoupled look-back scans, so every output is deterministic.
+#include <algorithm>
+
 #include "fiber_kernels.cuh"
 
 namespace fiber {
@@ -359,12 +361,13 @@ __device__ __forceinline__ bool fine_chunk(const FrameParams& P, const InstanceV
 // The strand g of frustum f: instance, local strand, segment count, first
 // index and the task's packed field; nseg = 0 when the keep tests drop it.
 struct FineStrand {
-    uint32_t i, s, nseg, meta_offset, packed;
+    uint32_t i, s, nseg, meta_offset, packed, material;
+    bool ordered;  // its segments follow the previous strand's in the index slab
 };
 
 __device__ __forceinline__ FineStrand fine_strand(const FrameParams& P, const InstanceView* __restrict__ inst,
                                                   const PrepassArgs& A, uint32_t f, uint32_t g, uint32_t g_end) {
-    FineStrand r{0u, 0u, 0u, 0u, 0u};
+    FineStrand r{0u, 0u, 0u, 0u, 0u, 0u, true};
     if (g >= g_end) return r;
     uint32_t lo = 0, hi = P.I;  // last instance with strand_base <= g
     while (hi - lo > 1u) {
@@ -382,12 +385,17 @@ __device__ __forceinline__ FineStrand fine_strand(const FrameParams& P, const In
     bool ok = in.valid && in.view == P.fview[f] && A.inst_visible[lo] != 0u && r.s < in.strand_count &&
               !(h > A.inst_keep[lo]);
     ok = ok && d.kind <= 1u && r.s < in.n_meta;
+    if (in.valid && r.s > 0u && r.s < in.strand_count) {
+        const fiber_strand_meta a = in.meta[r.s - 1u];
+        r.ordered = (uint64_t)a.offset + max(a.count, 1u) - 1u <= (uint64_t)in.meta[r.s].offset;
+    }
     if (ok) {
         const fiber_strand_meta m = in.meta[r.s];
         ok = m.count >= 2u && !(h > A.keep[lo * P.F + f]) && !(d.kind == 1u && light_layer(P, f) == kInvalid);
         if (ok) {
             r.nseg = m.count - 1u;
             r.meta_offset = m.offset;
+            r.material = m.material_idx;
             r.packed = ((d.kind == 1u ? 1u : 0u) << 2u) | (f << 3u);
         }
     }
@@ -422,6 +430,7 @@ __global__ void __launch_bounds__(kFineThreads, 4) k_fine(const FrameParams* __r
         uint32_t count = 0;
         for (uint32_t k = 0; k < kFineStrandsPerWarp; ++k) {
             const FineStrand fs = fine_strand(P, inst, A, f, g0 + k, g_end);
+            if (!fs.ordered) A.counters->seg_unordered = 1u;
             // FRUSTUM_TELEMETRY_RETAINED_STRANDS (:1085): every strand the
             // keep tests pass.
             if (A.tel && lane == 0 && fs.nseg > 0u) atomicAdd(tel_frustum(A.tel, f, kTelRetainedStrands), 1u);
@@ -463,8 +472,11 @@ __global__ void __launch_bounds__(kFineThreads, 4) k_fine(const FrameParams* __r
                         reinterpret_cast<uint4*>(A.tasks)[dst] = make_uint4(fs.i, fs.s, o.seg, fs.packed);
                         fiber_projected_segment ps{o.p0, o.p1, o.dz};
                         A.projected[dst] = ps;
-                        A.task_proj[2u * (size_t)dst] = o.r0;
-                        A.task_proj[2u * (size_t)dst + 1u] = o.r1;
+                        A.task_key[dst] = (o.dz & 0xFFFFu) + (o.dz >> 16u);
+                        float4* rec = A.task_rec + (size_t)kTaskRec * dst;
+                        rec[0] = o.r0;
+                        rec[1] = o.r1;
+                        reinterpret_cast<uint4*>(rec)[2] = make_uint4(fs.i, o.seg, fs.material, 0u);
                     } else {
                         atomicOr(&A.counters->overflow, 1u);
                     }
@@ -613,7 +625,7 @@ struct FillSink {
         const uint32_t lw = atomicAdd(A->cursors + g, 1u);
         const uint64_t dst = (uint64_t)base + A->offsets[g] + lw;
         if (dst >= (uint64_t)base + count) return;
-        A->ref_keys[dst] = task;  // k_sort_cells turns it into the reference
+        A->ref_task[dst] = task;  // k_sort_cells orders the cell
     }
 };
 
@@ -710,8 +722,6 @@ __device__ __forceinline__ void walk_page(const PrepassArgs& A, F3 p0, const Cli
 struct TaskWalk {
     F3 p0, p1;        // projected endpoints in pixels / depth01
     uint32_t f;       // frustum
-    uint32_t i, strand, seg;
-    uint32_t depths;  // packed projected depths (the sort key source)
     uint32_t min_cx, max_cx, min_cy, max_cy;
 };
 
@@ -739,10 +749,6 @@ __device__ __forceinline__ bool task_walk(const FrameParams& P, const PrepassArg
     w.p0 = p0;
     w.p1 = p1;
     w.f = f;
-    w.i = i;
-    w.strand = t.y;
-    w.seg = t.z;
-    w.depths = pr.depths;
     return true;
 }
 
@@ -808,8 +814,7 @@ __device__ __forceinline__ bool visits_unused(const PrepassArgs& A) {
 // kOpaque: the frame has opaque fine tiles (K0 ran); the variant without them
 // carries no cull code. kTel: count page candidates for the telemetry.
 template <bool kOpaque, bool kTel>
-__global__ void __launch_bounds__(kVisitThreads, 4) k_visit(const FrameParams* __restrict__ Pp,
-                                                            const InstanceView* __restrict__ inst, PrepassArgs A) {
+__global__ void __launch_bounds__(kVisitThreads, 4) k_visit(const FrameParams* __restrict__ Pp, PrepassArgs A) {
     if (frame_failed(A.counters)) return;
     const FrameParams& P = *Pp;
     __shared__ uint32_t s_buf[kVisitSlots * kVisitThreads];
@@ -828,15 +833,7 @@ __global__ void __launch_bounds__(kVisitThreads, 4) k_visit(const FrameParams* _
         TaskWalk w;
         const bool ok = k < n_cap && task_walk(P, A, k, w);
         VisitSink<kTel> vs{A.page_table, s_buf + threadIdx.x, 0u, 0u, records, A.tel_slots};
-        if (ok) {
-            // The task's reference (make_fine_seg_ref, :1313-1327) as its sort
-            // key and material, gathered later by k_sort_cells from these
-            // compact arrays instead of from the task records.
-            const InstanceView& in = inst[w.i];
-            A.task_key[k] = ref_sort_key((w.depths & 0xFFFFu) + (w.depths >> 16u), w.i, w.seg);
-            A.task_mat[k] = w.strand < in.n_meta ? in.meta[w.strand].material_idx : 0u;
-            walk_task(P, A, w, opq, vs);
-        }
+        if (ok) walk_task(P, A, w, opq, vs);
         if (!records) continue;
         uint32_t incl = vs.n;
 #pragma unroll
@@ -889,10 +886,8 @@ __global__ void __launch_bounds__(256) k_count_visits(PrepassArgs A) {
 }
 
 // K11 over visit records: the visit's slot is page base + cell offset + rank.
-// The fill scatters only the binning task index (4 B, into ref_keys, which a
-// frame's L2 holds); k_sort_cells gathers each cell's tasks, builds the
-// references (make_fine_seg_ref, :1313-1327) and writes them in canonical
-// order, contiguously.
+// A reference is its binning task's index (4 B, an array which a frame's L2
+// holds); k_sort_cells puts each cell's into canonical order.
 __global__ void __launch_bounds__(256) k_fill_visits(PrepassArgs A) {
     if (frame_failed(A.counters)) return;
     if (visits_unused(A)) return;
@@ -906,14 +901,13 @@ __global__ void __launch_bounds__(256) k_fill_visits(PrepassArgs A) {
         if (pm.seg_ref_count == 0u) continue;
         const uint64_t dst = (uint64_t)pm.seg_ref_base + A.offsets[g] + __ldcs(A.visit_rank + r);
         if (dst >= (uint64_t)pm.seg_ref_base + pm.seg_ref_count) continue;
-        A.ref_keys[dst] = __ldcs(A.visit_task + r);
+        A.ref_task[dst] = __ldcs(A.visit_task + r);
     }
 }
 
 // K9 / K11 walking form, for frames whose visit records did not fit.
 template <int PASS, bool kOpaque>
-__global__ void __launch_bounds__(256) k_traverse(const FrameParams* __restrict__ Pp,
-                                                  const InstanceView* __restrict__ inst, PrepassArgs A) {
+__global__ void __launch_bounds__(256) k_traverse(const FrameParams* __restrict__ Pp, PrepassArgs A) {
     if (frame_failed(A.counters)) return;
     if (!visits_unused(A)) return;
     const FrameParams& P = *Pp;
@@ -1083,7 +1077,7 @@ __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restr
         for (uint32_t k = 0; k < 8u; ++k) {
             e[k] = sum;
             sum += c[k];
-            nsmall += (c[k] >= 1u && c[k] <= kThreadSortMax) ? 1u : 0u;
+            nsmall += (c[k] >= 2u && c[k] <= kThreadSortMax) ? 1u : 0u;
             nmid += (c[k] > kThreadSortMax && c[k] <= kGroupSortMax) ? 1u : 0u;
             nlarge += c[k] > kGroupSortMax ? 1u : 0u;
             nz |= (c[k] > 0u ? 1u : 0u) << k;
@@ -1124,8 +1118,9 @@ __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restr
         flags = __shfl_sync(0xFFFFFFFFu, flags, 0);
         // A page that lost its references lists no cells and no active tiles.
         if (flags != 0u) continue;
-        // The page's non-empty cells for k_sort_cells: up to 8 references in the
-        // small list, more in the large one, in cell order.
+        // The page's cells for k_sort_cells, in cell order: 2..8 references in
+        // the small list, 9..32 in the middle one, more in the large one (a
+        // single reference is in order).
         uint32_t s_small = 0u, s_mid = 0u, s_large = 0u;
         if (lane == 0u) {
             const uint32_t ns = both & 0x3FFu, nm = (both >> 10) & 0x3FFu, nl = both >> 20;
@@ -1138,7 +1133,7 @@ __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restr
         uint32_t kl = __shfl_sync(0xFFFFFFFFu, s_large, 0) + (list_base >> 20);
 #pragma unroll
         for (uint32_t k = 0; k < 8u; ++k) {
-            if (c[k] >= 1u && c[k] <= kThreadSortMax) A.cells_small[ks++] = make_uint2(base + e[k], c[k]);
+            if (c[k] >= 2u && c[k] <= kThreadSortMax) A.cells_small[ks++] = make_uint2(base + e[k], c[k]);
             else if (c[k] > kThreadSortMax && c[k] <= kGroupSortMax) A.cells_mid[km++] = make_uint2(base + e[k], c[k]);
             else if (c[k] > kGroupSortMax) A.cells_large[kl++] = make_uint2(base + e[k], c[k]);
         }
@@ -1218,96 +1213,63 @@ __global__ void __launch_bounds__(kScanThreads) k_compact_active(const FramePara
 // instance, then segment) is made by k_sort_cells after the fill.
 // ===========================================================================
 
-// One warp sorts a cell of up to 32 * R references in registers: element
-// e = lane * R + r, bitonic network over 32 R keys (padding sorts last).
-// Strides below R compare registers of one lane; larger strides exchange the
-// same register with lane ^ (stride / R).
-// The reference of binning task k (make_fine_seg_ref, :1313-1327) as a sort
-// key (depth key, instance, segment) and its material, as k_visit stored them
-// (12 B per task, which a frame's L2 mostly holds).
-// A cell entry: the task's canonical-order key and the task index; the sort
-// moves the pair, and the store writes the reference (with the task's
-// material), its depth key and its task.
-__device__ __forceinline__ void task_entry(const PrepassArgs& A, const InstanceView* __restrict__ /*inst*/,
-                                           uint32_t k, unsigned long long& key, uint32_t& task) {
-    key = A.task_key[k];
-    task = k;
-}
-
-__device__ __forceinline__ void store_entry(const PrepassArgs& A, uint32_t dst, unsigned long long key, uint32_t task) {
-    A.refs[dst] = fiber_fine_seg_ref{(uint32_t)(key >> 32) & 0x7FFFu, (uint32_t)key, A.task_mat[task]};
-    A.ref_keys[dst] = 0x1FFFFu - (uint32_t)(key >> 47);
-    A.ref_task[dst] = task;
-}
-
-template <int R>
-__device__ __forceinline__ void warp_sort_cell(const PrepassArgs& A, const InstanceView* __restrict__ inst,
-                                               uint32_t base, uint32_t n, int lane) {
-    unsigned long long k[R];
-    uint32_t task[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const uint32_t e = (uint32_t)lane * R + r;
-        k[r] = ~0ull;
-        task[r] = 0u;
-        if (e < n) task_entry(A, inst, A.ref_keys[base + e], k[r], task[r]);
+// A cell's entries are binning task indices; the canonical order is by depth key
+// descending, then instance, then segment. Tasks are in (frustum, instance,
+// strand, segment) order, so where every instance's strands follow one another
+// in its index slab (k_fine checks every strand against the one before it) the
+// task index orders instance and segment, and an entry is one 64-bit word
+// (0x1FFFF - depth key) << 32 | task that sorts alone (ByTask). Otherwise
+// (strands in any order or sharing indices) the word is the full key of
+// ref_sort_key and the task moves beside it (ByRecord). Depth keys repeat inside
+// most cells (a fine cell spans some 100 to 500 of their steps), so the tie
+// order has to be in the word.
+struct ByTask {
+    unsigned long long w;
+    __device__ __forceinline__ void load(const PrepassArgs& A, uint32_t task) {
+        w = ((unsigned long long)(0x1FFFFu - A.task_key[task]) << 32) | task;
     }
-#pragma unroll
-    for (int size = 2; size <= 32 * R; size <<= 1) {
-#pragma unroll
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            if (stride >= R) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int e = lane * R + r;
-                    unsigned long long ok = __shfl_xor_sync(0xFFFFFFFFu, k[r], stride / R);
-                    uint32_t om = __shfl_xor_sync(0xFFFFFFFFu, task[r], stride / R);
-                    const bool up = (e & size) == 0;
-                    const bool lower = (e & stride) == 0;
-                    const bool take_other = lower == up ? (ok < k[r]) : (ok > k[r]);
-                    if (take_other) { k[r] = ok; task[r] = om; }
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int r2 = r ^ stride;
-                    if (r2 > r) {
-                        const int e = lane * R + r;
-                        const bool up = (e & size) == 0;
-                        if (up ? (k[r] > k[r2]) : (k[r] < k[r2])) {
-                            unsigned long long tk = k[r]; k[r] = k[r2]; k[r2] = tk;
-                            uint32_t tt = task[r]; task[r] = task[r2]; task[r2] = tt;
-                        }
-                    }
-                }
-            }
-        }
+    __device__ __forceinline__ void pad() { w = ~0ull; }
+    __device__ __forceinline__ uint32_t task() const { return (uint32_t)w; }
+    __device__ __forceinline__ ByTask other(int mask) const { return ByTask{__shfl_xor_sync(0xFFFFFFFFu, w, mask)}; }
+};
+struct ByRecord {
+    unsigned long long w;
+    uint32_t t;
+    __device__ __forceinline__ void load(const PrepassArgs& A, uint32_t task) {
+        const uint4 r = reinterpret_cast<const uint4*>(A.task_rec)[(size_t)kTaskRec * task + 2u];
+        w = ref_sort_key(A.task_key[task], r.x, r.y);
+        t = task;
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const uint32_t e = (uint32_t)lane * R + r;
-        if (e < n) store_entry(A, base + e, k[r], task[r]);
+    __device__ __forceinline__ void pad() { w = ~0ull; t = 0u; }
+    __device__ __forceinline__ uint32_t task() const { return t; }
+    __device__ __forceinline__ ByRecord other(int mask) const {
+        return ByRecord{__shfl_xor_sync(0xFFFFFFFFu, w, mask), __shfl_xor_sync(0xFFFFFFFFu, t, mask)};
+    }
+};
+template <class E>
+__device__ __forceinline__ void order(E& a, E& b, bool up) {
+    if (up ? (a.w > b.w) : (a.w < b.w)) {
+        const E x = a;
+        a = b;
+        b = x;
     }
 }
 
-
-// A group of G lanes (G-aligned inside the warp) sorts one cell of up to
-// G x R references: the bitonic network of warp_sort_cell over element
-// e = (lane % G) R + r, shuffles exchanging only inside the group. Groups
-// without a cell (n = 0) take part with padding. Every lane of the warp calls
-// it.
-template <int G, int R>
-__device__ __forceinline__ void group_sort_cell(const PrepassArgs& A, const InstanceView* __restrict__ inst,
-                                                uint32_t base, uint32_t n, int lane) {
+// A group of G lanes (G-aligned inside the warp) sorts one cell of up to G x R
+// entries in registers: element e = (lane % G) R + r, a bitonic network over
+// G R words (padding sorts last). Strides below R compare registers of one lane;
+// larger strides exchange the same register with lane ^ (stride / R), inside
+// the group. Groups without a cell (n = 0) take part with padding. Every lane
+// of the warp calls it.
+template <class E, int G, int R>
+__device__ __forceinline__ void group_sort_cell(const PrepassArgs& A, uint32_t base, uint32_t n, int lane) {
     const int gl = lane & (G - 1);
-    unsigned long long k[R];
-    uint32_t task[R];
+    E k[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const uint32_t e = (uint32_t)gl * R + r;
-        k[r] = ~0ull;
-        task[r] = 0u;
-        if (e < n) task_entry(A, inst, A.ref_keys[base + e], k[r], task[r]);
+        k[r].pad();
+        if (e < n) k[r].load(A, A.ref_task[base + e]);
     }
 #pragma unroll
     for (int size = 2; size <= G * R; size <<= 1) {
@@ -1317,52 +1279,37 @@ __device__ __forceinline__ void group_sort_cell(const PrepassArgs& A, const Inst
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     const int e = gl * R + r;
-                    unsigned long long ok = __shfl_xor_sync(0xFFFFFFFFu, k[r], stride / R);
-                    uint32_t om = __shfl_xor_sync(0xFFFFFFFFu, task[r], stride / R);
+                    const E o = k[r].other(stride / R);
                     const bool up = (e & size) == 0;
                     const bool lower = (e & stride) == 0;
-                    const bool take_other = lower == up ? (ok < k[r]) : (ok > k[r]);
-                    if (take_other) { k[r] = ok; task[r] = om; }
+                    if (lower == up ? (o.w < k[r].w) : (o.w > k[r].w)) k[r] = o;
                 }
             } else {
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int r2 = r ^ stride;
-                    if (r2 > r) {
-                        const int e = gl * R + r;
-                        const bool up = (e & size) == 0;
-                        if (up ? (k[r] > k[r2]) : (k[r] < k[r2])) {
-                            unsigned long long tk = k[r]; k[r] = k[r2]; k[r2] = tk;
-                            uint32_t tt = task[r]; task[r] = task[r2]; task[r2] = tt;
-                        }
-                    }
-                }
+                for (int r = 0; r < R; ++r)
+                    if ((r ^ stride) > r) order(k[r], k[r ^ stride], ((gl * R + r) & size) == 0);
             }
         }
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const uint32_t e = (uint32_t)gl * R + r;
-        if (e < n) store_entry(A, base + e, k[r], task[r]);
+        if (e < n) A.ref_task[base + e] = k[r].task();
     }
 }
 
-__device__ __forceinline__ void warp_sort_any(const PrepassArgs& A, const InstanceView* __restrict__ inst,
-                                              uint32_t base, uint32_t n, int lane) {
-    if (n <= 32u) warp_sort_cell<1>(A, inst, base, n, lane);
-    else if (n <= 64u) warp_sort_cell<2>(A, inst, base, n, lane);
-    else if (n <= 128u) warp_sort_cell<4>(A, inst, base, n, lane);
-    else warp_sort_cell<8>(A, inst, base, n, lane);
+template <class E>
+__device__ __forceinline__ void warp_sort_any(const PrepassArgs& A, uint32_t base, uint32_t n, int lane) {
+    if (n <= 32u) group_sort_cell<E, 32, 1>(A, base, n, lane);
+    else if (n <= 64u) group_sort_cell<E, 32, 2>(A, base, n, lane);
+    else if (n <= 128u) group_sort_cell<E, 32, 4>(A, base, n, lane);
+    else group_sort_cell<E, 32, 8>(A, base, n, lane);
 }
 
-// Batcher's odd-even merge network for 8 (key, task) pairs in registers.
-__device__ __forceinline__ void sort8(unsigned long long* k, uint32_t* task) {
-    auto cas = [&](int a, int b) {
-        if (k[a] > k[b]) {
-            const unsigned long long tk = k[a]; k[a] = k[b]; k[b] = tk;
-            const uint32_t tt = task[a]; task[a] = task[b]; task[b] = tt;
-        }
-    };
+// Batcher's odd-even merge network for 8 entries in registers.
+template <class E>
+__device__ __forceinline__ void sort8(E* k) {
+    auto cas = [&](int a, int b) { order(k[a], k[b], true); };
     cas(0, 1); cas(2, 3); cas(4, 5); cas(6, 7);
     cas(0, 2); cas(1, 3); cas(4, 6); cas(5, 7);
     cas(1, 2); cas(5, 6);
@@ -1373,20 +1320,18 @@ __device__ __forceinline__ void sort8(unsigned long long* k, uint32_t* task) {
 
 // One thread sorts a cell of at most 8 references in registers: Batcher's
 // odd-even merge network for 8 inputs (19 comparators); padding sorts last.
-__device__ __forceinline__ void thread_sort_cell(const PrepassArgs& A, const InstanceView* __restrict__ inst,
-                                                 uint32_t base, uint32_t n) {
-    unsigned long long k[8];
-    uint32_t task[8];
+template <class E>
+__device__ __forceinline__ void thread_sort_cell(const PrepassArgs& A, uint32_t base, uint32_t n) {
+    E k[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-        k[e] = ~0ull;
-        task[e] = 0u;
-        if ((uint32_t)e < n) task_entry(A, inst, A.ref_keys[base + e], k[e], task[e]);
+        k[e].pad();
+        if ((uint32_t)e < n) k[e].load(A, A.ref_task[base + e]);
     }
-    sort8(k, task);
+    sort8(k);
 #pragma unroll
     for (int e = 0; e < 8; ++e)
-        if ((uint32_t)e < n) store_entry(A, base + e, k[e], task[e]);
+        if ((uint32_t)e < n) A.ref_task[base + e] = k[e].task();
 }
 
 // One warp per active tile: the tile's 256 depth slots (16 coarse z x 16 fine
@@ -1473,16 +1418,8 @@ __global__ void __launch_bounds__(256) k_emit(const FrameParams* __restrict__ Pp
     }
 }
 
-// A cell longer than a warp sort: its warp writes the references in final
-// form (unsorted) and queues the cell for k_sort_big_cells.
-__device__ __forceinline__ void convert_big_cell(const PrepassArgs& A, const InstanceView* __restrict__ inst,
-                                                 uint32_t b, uint32_t n, uint32_t lane) {
-    for (uint32_t j = lane; j < n; j += 32u) {
-        unsigned long long key;
-        uint32_t task;
-        task_entry(A, inst, A.ref_keys[b + j], key, task);
-        store_entry(A, b + j, key, task);
-    }
+// A cell longer than a warp sort is queued for k_sort_big_cells.
+__device__ __forceinline__ void queue_big_cell(const PrepassArgs& A, uint32_t b, uint32_t n, uint32_t lane) {
     if (lane == 0u) {
         const uint32_t slot = atomicAdd(&A.counters->big_cells, 1u);
         A.big_cells[slot] = make_uint2(b, n);
@@ -1491,36 +1428,37 @@ __device__ __forceinline__ void convert_big_cell(const PrepassArgs& A, const Ins
 
 // 32 consecutive small cells at once. k_prefix_pages lists a page's small
 // cells together, in cell order, so their references usually form one span
-// [lo, hi) of the reference array (holes: the page's larger cells). When the
-// span fits kSortSpan, each lane loads the task index of every 32nd entry of
-// the span (8 independent loads), gathers those tasks' keys and materials (16
-// independent loads), and parks them in shared memory; each lane then sorts
-// its own cell there with the network of thread_sort_cell and the warp writes
-// the span's own entries back coalesced. Otherwise each lane sorts its cell
-// alone.
+// [lo, hi) of the reference array (holes: the page's other cells). When the
+// span fits kSortSpan, each lane loads every 32nd entry of the span (8
+// independent loads, then 8 independent key gathers) and parks the words in
+// shared memory; each lane then sorts its own cell there with sort8 and the
+// warp writes the span's own entries back coalesced. Otherwise each lane sorts
+// its cell alone (as it does for entries that carry their task beside the word).
 constexpr uint32_t kSortSpan = 256;
 constexpr uint32_t kSortPerLane = kSortSpan / 32u;
 struct SortSpanSmem {
-    unsigned long long key[kSortSpan];
-    uint32_t task[kSortSpan];
-    uint32_t mat[kSortSpan];
+    ByTask entry[kSortSpan];
     uint8_t own[kSortSpan];
 };
 
-__device__ __forceinline__ void warp_sort_small_cells(const PrepassArgs& A, const InstanceView* __restrict__ inst,
-                                                      uint32_t i0, uint32_t n_small, uint32_t lane,
-                                                      SortSpanSmem& sm) {
+__device__ __forceinline__ void warp_sort_small_cells(const PrepassArgs& A, uint32_t i0, uint32_t n_small,
+                                                      uint32_t lane, SortSpanSmem* /*sm*/, ByRecord) {
+    if (i0 + lane >= n_small) return;
+    const uint2 e = A.cells_small[i0 + lane];
+    thread_sort_cell<ByRecord>(A, e.x, e.y);
+}
+__device__ __forceinline__ void warp_sort_small_cells(const PrepassArgs& A, uint32_t i0, uint32_t n_small,
+                                                      uint32_t lane, SortSpanSmem* smp, ByTask) {
+    using E = ByTask;
+    SortSpanSmem& sm = *smp;
     const uint32_t i = i0 + lane;
     const bool has = i < n_small;
     const uint2 e = has ? A.cells_small[i] : make_uint2(0u, 0u);
     uint32_t lo = has ? e.x : 0xFFFFFFFFu, hi = has ? e.x + e.y : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
-        hi = max(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
-    }
+    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
     if (hi <= lo || hi - lo > kSortSpan) {
-        if (has) thread_sort_cell(A, inst, e.x, e.y);
+        if (has) thread_sort_cell<E>(A, e.x, e.y);
         return;
     }
     const uint32_t span = hi - lo;
@@ -1534,95 +1472,77 @@ __device__ __forceinline__ void warp_sort_small_cells(const PrepassArgs& A, cons
 #pragma unroll
     for (uint32_t m = 0; m < kSortPerLane; ++m) {
         const uint32_t j = lane + 32u * m;
-        tk[m] = (j < span && sm.own[j]) ? A.ref_keys[lo + j] : kInvalid;
+        tk[m] = (j < span && sm.own[j]) ? A.ref_task[lo + j] : kInvalid;
     }
-    unsigned long long kk[kSortPerLane];
-    uint32_t mt[kSortPerLane];
+    E en[kSortPerLane];
 #pragma unroll
     for (uint32_t m = 0; m < kSortPerLane; ++m) {
-        kk[m] = tk[m] != kInvalid ? A.task_key[tk[m]] : ~0ull;
-        mt[m] = tk[m] != kInvalid ? A.task_mat[tk[m]] : 0u;
+        en[m].pad();
+        if (tk[m] != kInvalid) en[m].load(A, tk[m]);
     }
 #pragma unroll
-    for (uint32_t m = 0; m < kSortPerLane; ++m) {
-        const uint32_t j = lane + 32u * m;
-        sm.key[j] = kk[m];
-        sm.task[j] = tk[m];
-        sm.mat[j] = mt[m];
-    }
+    for (uint32_t m = 0; m < kSortPerLane; ++m) sm.entry[lane + 32u * m] = en[m];
     __syncwarp();
     if (has) {
-        // Sort (key, position); the task and material follow their position.
-        unsigned long long k[8];
-        uint32_t pos[8];
         const uint32_t b = e.x - lo;
 #pragma unroll
         for (uint32_t r = 0; r < 8u; ++r) {
-            k[r] = r < e.y ? sm.key[b + r] : ~0ull;
-            pos[r] = b + min(r, e.y - 1u);
+            en[r].pad();
+            if (r < e.y) en[r] = sm.entry[b + r];
         }
-        sort8(k, pos);
-        uint32_t t[8], mm[8];
-#pragma unroll
-        for (uint32_t r = 0; r < 8u; ++r) {
-            t[r] = sm.task[pos[r]];
-            mm[r] = sm.mat[pos[r]];
-        }
+        sort8(en);
 #pragma unroll
         for (uint32_t r = 0; r < 8u; ++r)
-            if (r < e.y) {
-                sm.key[b + r] = k[r];
-                sm.task[b + r] = t[r];
-                sm.mat[b + r] = mm[r];
-            }
+            if (r < e.y) sm.entry[b + r] = en[r];
     }
     __syncwarp();
 #pragma unroll
     for (uint32_t m = 0; m < kSortPerLane; ++m) {
         const uint32_t j = lane + 32u * m;
-        if (j < span && sm.own[j]) {
-            const unsigned long long key = sm.key[j];
-            A.refs[lo + j] = fiber_fine_seg_ref{(uint32_t)(key >> 32) & 0x7FFFu, (uint32_t)key, sm.mat[j]};
-            A.ref_keys[lo + j] = 0x1FFFFu - (uint32_t)(key >> 47);
-            A.ref_task[lo + j] = sm.task[j];
-        }
+        if (tk[m] != kInvalid) A.ref_task[lo + j] = sm.entry[j].task();
     }
     __syncwarp();
 }
 
-// Canonical order inside every cell (projected depth key descending, then
-// instance, then segment), after the fill, over the cell lists k_prefix_pages
-// made: a warp per 32 cells of up to 8 references (a lane per cell), four
-// cells of 9..32 references per warp (eight lanes each), then a warp per
-// larger cell. A cell longer than a warp sort is converted in place by its
-// warp and queued for k_sort_big_cells.
-__global__ void __launch_bounds__(256, 5) k_sort_cells(const InstanceView* __restrict__ inst, PrepassArgs A) {
-    if (frame_failed(A.counters)) return;
-    __shared__ SortSpanSmem s_span[8];
+template <class E>
+__device__ __forceinline__ void sort_cells(const PrepassArgs& A, SortSpanSmem* s_span) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t n_small = *((volatile uint32_t*)&A.counters->small_cells);
     const uint32_t n_large = *((volatile uint32_t*)&A.counters->large_cells);
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; i0 < n_small; i0 += stride)
-        warp_sort_small_cells(A, inst, i0, n_small, lane, s_span[threadIdx.x >> 5]);
+        warp_sort_small_cells(A, i0, n_small, lane, s_span, E{});
     const uint32_t warps = stride >> 5;
     // Cells of 9..32 references: four per warp, eight lanes each.
     const uint32_t n_mid = *((volatile uint32_t*)&A.counters->mid_cells);
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 4u < n_mid; w += warps) {
         const uint32_t ci = w * 4u + (lane >> 3);
         const uint2 e = ci < n_mid ? A.cells_mid[ci] : make_uint2(0u, 0u);
-        group_sort_cell<8, 4>(A, inst, e.x, e.y, (int)lane);
+        group_sort_cell<E, 8, 4>(A, e.x, e.y, (int)lane);
     }
     // Cells of more than 32: a warp per cell.
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n_large; w += warps) {
         const uint2 e = A.cells_large[w];
-        const uint32_t b = e.x, n = e.y;
-        if (n <= kWarpSortMax) {
-            warp_sort_any(A, inst, b, n, (int)lane);
-        } else {
-            convert_big_cell(A, inst, b, n, lane);
-        }
+        if (e.y <= kWarpSortMax) warp_sort_any<E>(A, e.x, e.y, (int)lane);
+        else queue_big_cell(A, e.x, e.y, lane);
     }
+}
+
+// Canonical order inside every cell, in place, after the fill, over the cell
+// lists k_prefix_pages made: a warp per 32 cells of 2..8 references (a lane per
+// cell), four cells of 9..32 references per warp (eight lanes each), then a
+// warp per larger cell; a cell longer than a warp sort is queued for
+// k_sort_big_cells. Bound by instruction issue (the networks' 64-bit compares)
+// and the L2 latency of the key gathers. Writing 4 B task indices in place
+// instead of 20 B of reference, key and task, and sorting one word instead of
+// a word and its task, took this kernel from 0.57 to 0.37 ms for the 23.5 M
+// references of the medium frame and from 11.8 to 7.6 ms for the large
+// frame's 349 M.
+__global__ void __launch_bounds__(256, 5) k_sort_cells(PrepassArgs A) {
+    if (frame_failed(A.counters)) return;
+    __shared__ SortSpanSmem s_span[8];
+    if (*((volatile uint32_t*)&A.counters->seg_unordered) == 0u) sort_cells<ByTask>(A, s_span + (threadIdx.x >> 5));
+    else sort_cells<ByRecord>(A, s_span + (threadIdx.x >> 5));
 }
 
 // ===========================================================================
@@ -1701,8 +1621,7 @@ __global__ void __launch_bounds__(256) k_page_scatter(PrepassArgs A) {
 }
 
 // One block per page, in page order (the look-back of the page bases).
-__global__ void __launch_bounds__(256) k_build_pages(const FrameParams* __restrict__ Pp,
-                                                     const InstanceView* __restrict__ inst, PrepassArgs A) {
+__global__ void __launch_bounds__(256, 3) k_build_pages(const FrameParams* __restrict__ Pp, PrepassArgs A) {
     if (frame_failed(A.counters)) return;
     if (visits_unused(A)) return;
     const FrameParams& P = *Pp;
@@ -1711,6 +1630,7 @@ __global__ void __launch_bounds__(256) k_build_pages(const FrameParams* __restri
     __shared__ uint32_t s_counts[kPageSize], s_off[kPageSize], s_cur[kPageSize];
     __shared__ uint16_t s_large[kPageSize];
     const uint32_t pages = *((volatile uint32_t*)&A.counters->pages);
+    const bool by_task = *((volatile uint32_t*)&A.counters->seg_unordered) == 0u;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (;;) {
         if (threadIdx.x == 0) {
@@ -1737,17 +1657,20 @@ __global__ void __launch_bounds__(256) k_build_pages(const FrameParams* __restri
             // in L2); the order inside a cell is fixed by the sort below.
             for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
                 const uint2 v = A.page_bucket[vb + e];
-                A.ref_keys[pbase + s_off[v.y] + atomicAdd(&s_cur[v.y], 1u)] = v.x;
+                A.ref_task[pbase + s_off[v.y] + atomicAdd(&s_cur[v.y], 1u)] = v.x;
             }
             __syncthreads();
-            if (c >= 1u && c <= kThreadSortMax) thread_sort_cell(A, inst, pbase + excl, c);
-            else if (c > kThreadSortMax) s_large[atomicAdd(&s_nlarge, 1u)] = (uint16_t)threadIdx.x;
+            if (c >= 2u && c <= kThreadSortMax) {
+                if (by_task) thread_sort_cell<ByTask>(A, pbase + excl, c);
+                else thread_sort_cell<ByRecord>(A, pbase + excl, c);
+            } else if (c > kThreadSortMax) s_large[atomicAdd(&s_nlarge, 1u)] = (uint16_t)threadIdx.x;
             __syncthreads();
             const uint32_t nl = s_nlarge;
             for (uint32_t i = warp; i < nl; i += blockDim.x >> 5) {
                 const uint32_t cell = s_large[i], cb = pbase + s_off[cell], cn = s_counts[cell];
-                if (cn <= kWarpSortMax) warp_sort_any(A, inst, cb, cn, (int)lane);
-                else convert_big_cell(A, inst, cb, cn, lane);
+                if (cn > kWarpSortMax) queue_big_cell(A, cb, cn, lane);
+                else if (by_task) warp_sort_any<ByTask>(A, cb, cn, (int)lane);
+                else warp_sort_any<ByRecord>(A, cb, cn, (int)lane);
             }
             page_active_tiles(P, A, page, s_counts);
         }
@@ -1766,19 +1689,14 @@ constexpr size_t kBigSmemBytes = kBigSmem * (sizeof(unsigned long long) + sizeof
 __device__ __forceinline__ void big_load(const PrepassArgs& A, uint32_t base, uint32_t n, uint32_t i,
                                          unsigned long long& k, uint32_t& m) {
     if (i < n) {
-        fiber_fine_seg_ref r = A.refs[base + i];
-        k = ref_sort_key(A.ref_keys[base + i], r.inst_id, r.seg_id);
-        m = A.ref_task[base + i];
+        ByRecord r;
+        r.load(A, A.ref_task[base + i]);
+        k = r.w;
+        m = r.t;
     } else {
         k = ~0ull;
         m = 0u;
     }
-}
-__device__ __forceinline__ void big_store(const PrepassArgs& A, uint32_t base, uint32_t i, unsigned long long k,
-                                          uint32_t m) {
-    A.refs[base + i] = fiber_fine_seg_ref{(uint32_t)(k >> 32) & 0x7FFFu, (uint32_t)k, A.task_mat[m]};
-    A.ref_keys[base + i] = 0x1FFFFu - (uint32_t)(k >> 47);
-    A.ref_task[base + i] = m;
 }
 // Pair t of a stage: (i, j) with i < j.
 __device__ __forceinline__ void bitonic_pair(uint32_t t, uint32_t size, uint32_t stride, bool flip, uint32_t& i,
@@ -1827,8 +1745,8 @@ __global__ void __launch_bounds__(256) k_sort_big_cells(PrepassArgs A) {
                         big_load(A, base, n, i, ki, mi);
                         big_load(A, base, n, j, kj, mj);
                         if (ki > kj) {
-                            big_store(A, base, i, kj, mj);
-                            big_store(A, base, j, ki, mi);
+                            A.ref_task[base + i] = mj;
+                            A.ref_task[base + j] = mi;
                         }
                     }
                 }
@@ -1836,7 +1754,7 @@ __global__ void __launch_bounds__(256) k_sort_big_cells(PrepassArgs A) {
             }
         }
         if (in_smem) {
-            for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) big_store(A, base, i, s_k[i], s_m[i]);
+            for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) A.ref_task[base + i] = s_m[i];
             __syncthreads();
         }
     }
@@ -1888,6 +1806,19 @@ __global__ void __launch_bounds__(256) k_telemetry(const FrameParams* __restrict
     }
 }
 
+// FineSegRef records of references [0, n), from their tasks' records. References
+// of a page dropped by an overflow hold whatever an earlier frame left there.
+__global__ void __launch_bounds__(256) k_expand_refs(const uint32_t* __restrict__ ref_task,
+                                                     const float4* __restrict__ task_rec, uint32_t n_tasks, uint64_t n,
+                                                     fiber_fine_seg_ref* __restrict__ out) {
+    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t task = ref_task[r];
+        const uint4 w = task < n_tasks ? reinterpret_cast<const uint4*>(task_rec)[(size_t)kTaskRec * task + 2u]
+                                       : make_uint4(0u, 0u, 0u, 0u);
+        out[r] = fiber_fine_seg_ref{w.x, w.y, w.z};
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Launch wrappers
 // ---------------------------------------------------------------------------
@@ -1910,11 +1841,11 @@ void launch_fine(const LaunchCtx& L, const PrepassArgs& A) {
 void launch_visit(const LaunchCtx& L, const PrepassArgs& A) {
     const unsigned grid = L.sm_count * 4;  // the resident blocks (4 per SM), each looping over warps of tasks
     if (L.telemetry) {
-        if (L.opaque) k_visit<true, true><<<grid, kVisitThreads, 0, L.stream>>>(L.P, L.inst, A);
-        else k_visit<false, true><<<grid, kVisitThreads, 0, L.stream>>>(L.P, L.inst, A);
+        if (L.opaque) k_visit<true, true><<<grid, kVisitThreads, 0, L.stream>>>(L.P, A);
+        else k_visit<false, true><<<grid, kVisitThreads, 0, L.stream>>>(L.P, A);
     } else {
-        if (L.opaque) k_visit<true, false><<<grid, kVisitThreads, 0, L.stream>>>(L.P, L.inst, A);
-        else k_visit<false, false><<<grid, kVisitThreads, 0, L.stream>>>(L.P, L.inst, A);
+        if (L.opaque) k_visit<true, false><<<grid, kVisitThreads, 0, L.stream>>>(L.P, A);
+        else k_visit<false, false><<<grid, kVisitThreads, 0, L.stream>>>(L.P, A);
     }
 }
 void launch_alloc(const LaunchCtx& L, const PrepassArgs& A) {
@@ -1925,30 +1856,30 @@ void launch_zero_pages(const LaunchCtx& L, const PrepassArgs& A) {
 }
 void launch_count(const LaunchCtx& L, const PrepassArgs& A) {
     k_count_visits<<<L.sm_count * 8, 256, 0, L.stream>>>(A);
-    if (L.opaque) k_traverse<kCount, true><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, L.inst, A);
-    else k_traverse<kCount, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, L.inst, A);
+    if (L.opaque) k_traverse<kCount, true><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
+    else k_traverse<kCount, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
 }
 void launch_prefix(const LaunchCtx& L, const PrepassArgs& A, bool csr) {
     k_prefix_pages<<<L.sm_count * 6, 256, 0, L.stream>>>(L.P, A, csr);
 }
 void launch_page_csr_count(const LaunchCtx& L, const PrepassArgs& A) {
     k_page_count<<<L.sm_count * 8, 256, 0, L.stream>>>(A);
-    if (L.opaque) k_traverse<kCount, true><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, L.inst, A);
-    else k_traverse<kCount, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, L.inst, A);
+    if (L.opaque) k_traverse<kCount, true><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
+    else k_traverse<kCount, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
     k_page_scan<<<1, 1024, 0, L.stream>>>(A);
     k_page_scatter<<<L.sm_count * 8, 256, 0, L.stream>>>(A);
 }
 void launch_build_pages(const LaunchCtx& L, const PrepassArgs& A) {
-    k_build_pages<<<L.sm_count * 6, 256, 0, L.stream>>>(L.P, L.inst, A);
+    k_build_pages<<<L.sm_count * 6, 256, 0, L.stream>>>(L.P, A);
 }
 void launch_fill_walk(const LaunchCtx& L, const PrepassArgs& A) {
-    if (L.opaque) k_traverse<kFill, true><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, L.inst, A);
-    else k_traverse<kFill, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, L.inst, A);
+    if (L.opaque) k_traverse<kFill, true><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
+    else k_traverse<kFill, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
 }
 void launch_fill(const LaunchCtx& L, const PrepassArgs& A) {
     k_fill_visits<<<L.sm_count * 8, 256, 0, L.stream>>>(A);
-    if (L.opaque) k_traverse<kFill, true><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, L.inst, A);
-    else k_traverse<kFill, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, L.inst, A);
+    if (L.opaque) k_traverse<kFill, true><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
+    else k_traverse<kFill, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
 }
 void launch_compact_active(const LaunchCtx& L, const PrepassArgs& A) {
     k_compact_active<<<L.sm_count * 4, kScanThreads, 0, L.stream>>>(L.P, A);
@@ -1957,10 +1888,14 @@ void launch_emit(const LaunchCtx& L, const PrepassArgs& A) {
     k_emit<<<L.sm_count * 6, 256, 0, L.stream>>>(L.P, A);
 }
 void launch_sort_cells(const LaunchCtx& L, const PrepassArgs& A) {
-    k_sort_cells<<<L.sm_count * 5, 256, 0, L.stream>>>(L.inst, A);  // the resident blocks (5 per SM)
+    k_sort_cells<<<L.sm_count * 5, 256, 0, L.stream>>>(A);  // the resident blocks (5 per SM)
 }
 void launch_telemetry(const LaunchCtx& L, const PrepassArgs& A) {
     k_telemetry<<<L.sm_count * 2, 256, 0, L.stream>>>(L.P, A);
+}
+void launch_expand_refs(cudaStream_t s, const uint32_t* ref_task, const float4* task_rec, uint32_t n_tasks, uint64_t n,
+                        fiber_fine_seg_ref* out) {
+    if (n) k_expand_refs<<<std::min(ceil_div_host(n, 256), 4096u), 256, 0, s>>>(ref_task, task_rec, n_tasks, n, out);
 }
 void launch_sort_big(const LaunchCtx& L, const PrepassArgs& A) {
     static bool configured[64] = {};

@@ -258,16 +258,14 @@ __global__ void __launch_bounds__(kShadowThreads, 14) k_shadow(const FrameParams
     const FrameParams& P = *Pp;
     extern __shared__ float4 s_dyn4[];
     // Per staged entry: the projected end points (x, y, normalised depth, w),
-    // radii and opacity. The radius and opacity words first receive the
-    // entry's task, instance and material index (the first copy level).
+    // radii and opacity. The radius word first receives the entry's task (the
+    // first copy level).
     float4* sa = s_dyn4;
     float4* sb = sa + kShadowCap;
     float* srmin = reinterpret_cast<float*>(sb + kShadowCap);
     float* srmax = srmin + kShadowCap;
     float* sabs = srmax + kShadowCap;
     uint32_t* s_task = reinterpret_cast<uint32_t*>(srmin);
-    uint32_t* s_inst = reinterpret_cast<uint32_t*>(srmax);
-    uint32_t* s_midx = reinterpret_cast<uint32_t*>(sabs);
     // [worker][K][pixel]: a warp's 32 pixels hit 32 banks whatever the slice.
     float* s_partial = sabs + kShadowCap;
     __shared__ uint32_t s_wbase[kMaxRunItems], s_wcount[kMaxRunItems], s_prefix[kMaxRunItems + 1];
@@ -314,27 +312,26 @@ __global__ void __launch_bounds__(kShadowThreads, 14) k_shadow(const FrameParams
 
         // Stage a round (projection, radii, run item and worker of each entry),
         // then build the candidate bits: warp per 32-entry word. The entries'
-        // data arrive by asynchronous copies in two levels: the reference's
-        // task, instance and material index, then the task's projected end
-        // points (as k_fine projected them for this frustum:
-        // world_to_screen_raw of the segment's vertices), so a round waits
-        // for each level's latency once, whatever its entries.
+        // data arrive in two levels: the reference's task, then the task's
+        // record (end points as k_fine projected them for this frustum,
+        // world_to_screen_raw of the segment's vertices; instance and material),
+        // so a round waits for each level's latency once, whatever its entries.
         auto stage = [&](const RoundPlan& rp) {
             for (uint32_t s = threadIdx.x; s < rp.n; s += blockDim.x) {
                 uint32_t item, j;
                 slot_source(s_prefix, rp, s, item, j);
                 const uint32_t g = s_wbase[item] + j;
                 cp_async4(s_task + s, R.ref_task + g);
-                cp_async4(s_inst + s, &R.refs[g].inst_id);
-                cp_async4(s_midx + s, &R.refs[g].material_idx);
                 s_item[s] = (uint16_t)((item << 2) | (j & 3u));
             }
             cp_async_wait_all();
             for (uint32_t s = threadIdx.x; s < rp.n; s += blockDim.x) {
                 const size_t t = s_task[s];
-                cp_async16(sa + s, R.task_proj + 2u * t);
-                cp_async16(sb + s, R.task_proj + 2u * t + 1u);
-                const fiber_strand_material& m = inst[s_inst[s]].materials[s_midx[s]];
+                const float4* rec = R.task_rec + kTaskRec * t;
+                cp_async16(sa + s, rec);
+                cp_async16(sb + s, rec + 1);
+                const uint4 w = __ldg(reinterpret_cast<const uint4*>(rec) + 2);  // instance, segment, material
+                const fiber_strand_material& m = inst[w.x].materials[w.z];
                 const float rmin = wmax(m.min_radius_pixels, 1e-4f);
                 srmin[s] = rmin;
                 srmax[s] = wmax(m.max_radius_pixels, rmin);
@@ -668,9 +665,8 @@ __global__ void __launch_bounds__(kCamThreads, 14) k_raster(const FrameParams* _
     const FrameParams& P = *Pp;
     // Per staged entry: 68 B of projection (x, y, z, w of both end points),
     // radii and shading texels, the run item and position in it (bit 15:
-    // behind the camera, never a candidate). The words of sinv, srmin, srmax
-    // and svis first receive the reference's task, instance, segment and
-    // material index (the first copy level); s_hist receives the history
+    // behind the camera, never a candidate). The sinv word first receives the
+    // reference's task (the first copy level); s_hist receives the history
     // texel pair (visibility, current).
     __shared__ float4 sa[kCamCap], sb[kCamCap];
     __shared__ float sinv[kCamCap], srmin[kCamCap], srmax[kCamCap], svis[kCamCap];
@@ -736,32 +732,28 @@ __global__ void __launch_bounds__(kCamThreads, 14) k_raster(const FrameParams* _
             __syncthreads();
             if (!s_more) break;
             const RoundPlan rp = s_plan;
-            // The entries arrive by asynchronous copies in two levels: the
-            // reference (task, instance, segment, material index), then the
-            // task's projected end points (as k_fine projected them for this
-            // frustum) and the segment's shading and history texels.
+            // The entries arrive in three levels: the reference's task, the
+            // task's record (end points as k_fine projected them for this
+            // frustum; instance, segment, material), then the segment's
+            // shading and history texels.
             uint32_t* s_task = reinterpret_cast<uint32_t*>(sinv);
-            uint32_t* s_inst = reinterpret_cast<uint32_t*>(srmin);
-            uint32_t* s_seg = reinterpret_cast<uint32_t*>(srmax);
-            uint32_t* s_midx = reinterpret_cast<uint32_t*>(svis);
             for (uint32_t s = threadIdx.x; s < rp.n; s += blockDim.x) {
                 uint32_t item, j;
                 slot_source(s_prefix, rp, s, item, j);
                 const uint32_t g = s_wbase[item] + j;
                 cp_async4(s_task + s, R.ref_task + g);
-                cp_async4(s_inst + s, &R.refs[g].inst_id);
-                cp_async4(s_seg + s, &R.refs[g].seg_id);
-                cp_async4(s_midx + s, &R.refs[g].material_idx);
                 s_item[s] = (uint16_t)((item << 2) | (j & 3u));
             }
             cp_async_wait_all();
             for (uint32_t s = threadIdx.x; s < rp.n; s += blockDim.x) {
                 const size_t t = s_task[s];
-                const uint32_t ii = s_inst[s], i0 = min(s_seg[s], cap - 1u), i1 = min(i0 + 1u, cap - 1u);
-                const fiber_strand_material& m = inst[ii].materials[s_midx[s]];
+                const float4* rec = R.task_rec + kTaskRec * t;
+                cp_async16(sa + s, rec);
+                cp_async16(sb + s, rec + 1);
+                const uint4 w = __ldg(reinterpret_cast<const uint4*>(rec) + 2);  // instance, segment, material
+                const uint32_t ii = w.x, i0 = min(w.y, cap - 1u), i1 = min(i0 + 1u, cap - 1u);
+                const fiber_strand_material& m = inst[ii].materials[w.z];
                 const size_t t0 = (size_t)ii * cap + i0, t1 = (size_t)ii * cap + i1;
-                cp_async16(sa + s, R.task_proj + 2u * t);
-                cp_async16(sb + s, R.task_proj + 2u * t + 1u);
                 cp_async8(ss0 + s, R.atlas + t0 * 4);
                 cp_async8(ss1 + s, R.atlas + t1 * 4);
                 cp_async4(s_hist + s, hist + t0 * 2);
