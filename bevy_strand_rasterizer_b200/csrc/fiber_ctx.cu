@@ -285,6 +285,7 @@ RenderArgs render_args(fiber_ctx* c) {
     R.color = dp<__half>(c->d_color);
     R.depth = dp<float>(c->d_depth);
     R.fragments = dp<uint32_t>(c->d_fragments);
+    R.neg_zero2 = 0x8000000080000000ull;
     return R;
 }
 

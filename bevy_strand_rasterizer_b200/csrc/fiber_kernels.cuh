@@ -28,12 +28,6 @@ __device__ __forceinline__ float line_t(float px, float py, float ax, float ay, 
     return ((px - ax) * abx + (py - ay) * aby) / l2;
 }
 
-// blend_over_premult (strand_rasterizer.wgsl:156-162)
-__device__ __forceinline__ float4 over(float4 fg, float4 bg) {
-    float oma = 1.0f - fg.w;
-    return make_float4(fg.x + bg.x * oma, fg.y + bg.y * oma, fg.z + bg.z * oma, fg.w + bg.w * oma);
-}
-
 __device__ __forceinline__ float4 load_half4(const __half* p) {
     uint2 v = *reinterpret_cast<const uint2*>(p);
     __half2 a = *reinterpret_cast<__half2*>(&v.x), b = *reinterpret_cast<__half2*>(&v.y);
@@ -130,6 +124,7 @@ struct RenderArgs {
     __half* color;           // [H][W][4]
     float* depth;            // [H][W]
     uint32_t* fragments;     // [H][W]
+    unsigned long long neg_zero2;  // (-0, -0), a packed addend the assembler cannot see (fiber_raster.cu)
 };
 
 // Sparse DOM pages: DOM_PAGE_XY (src/plugin.rs:68) texels a side.
