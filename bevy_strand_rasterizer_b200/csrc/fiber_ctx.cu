@@ -31,8 +31,8 @@ const char* kSpanNames[kSpanCount] = {
     "strand_prepass/binning",              // count
     "strand_prepass/prefix_fine_pages",
     "strand_prepass/fill_segment_refs",
-    "strand_prepass/compact_active_tiles",
-    "strand_prepass/emit_raster_work",     // emit + canonical cell order
+    "strand_prepass/compact_active_tiles",  // what compaction and emit take beyond the fill they run beside
+    "strand_prepass/emit_raster_work",      // canonical cell order
     "strand_shadow_rasterizer/rasterize",  // incl. fused stampback
     "strand_shading/shade",
     "strand_rasterizer/rasterize",
@@ -110,7 +110,7 @@ struct fiber_ctx {
     DevBuf d_params, d_inst, d_counters, d_lb, d_range_valid, d_ranges, d_keep, d_inst_visible, d_inst_keep;
     DevBuf d_lut_tree;  // per coarse tile: the slice lookup's search tree (kLutTreeWords)
     DevBuf d_lut, d_tasks, d_projected, d_page_table, d_page_meta, d_counts, d_offsets, d_cursors;
-    DevBuf d_active_flags, d_active_list, d_work, d_runs, d_big_cells;
+    DevBuf d_tile_work, d_tile_slot, d_page_items, d_active_list, d_work, d_runs, d_big_cells;
     DevBuf d_visit_rec, d_visit_task, d_visit_rank, d_task_key, d_cells_small, d_cells_mid, d_cells_large;
     DevBuf d_opaque;  // (covered, farthest depth q) per camera fine tile
     DevBuf d_task_rec, d_ref_task;  // the rasters' record of each task; each reference's task
@@ -121,7 +121,7 @@ struct fiber_ctx {
     // beside the frame; ev_in = uploaded, ev_out = the last download queued.
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
-    // The prepass's cell sort runs on this stream beside the emit.
+    // The prepass's active-tile compaction and emit run on this stream beside the fill.
     cudaStream_t side_stream = nullptr;
     cudaStream_t side_override = nullptr;  // fiber_ctx_set_side_stream (request server priorities)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -234,7 +234,9 @@ PrepassArgs prepass_args(fiber_ctx* c) {
     A.counts = dp<uint32_t>(c->d_counts);
     A.offsets = dp<uint32_t>(c->d_offsets);
     A.cursors = dp<uint32_t>(c->d_cursors);
-    A.active_flags = dp<uint32_t>(c->d_active_flags);
+    A.tile_work = dp<uint32_t>(c->d_tile_work);
+    A.tile_slot = dp<uint2>(c->d_tile_slot);
+    A.page_items = dp<uint8_t>(c->d_page_items);
     A.active_list = dp<uint32_t>(c->d_active_list);
     A.work = dp<fiber_raster_work_item>(c->d_work);
     A.runs = dp<fiber_raster_tile_run>(c->d_runs);
@@ -312,7 +314,7 @@ fiber_status check_launch() {
 }
 
 // Per-frame clears of src/plugin.rs:1145-1208 that follow the frame-table
-// upload: counters, page table, active flags, colour / depth / fragment
+// upload: counters, page table, fine tiles' work counts, colour / depth / fragment
 // targets and the DOM depth + stampback target.
 fiber_status frame_resets(fiber_ctx* c, cudaStream_t s) {
     const FrameParams& P = c->P;
@@ -320,7 +322,7 @@ fiber_status frame_resets(fiber_ctx* c, cudaStream_t s) {
     const uint64_t WH = c->out_pixels, L = P.L, D = P.dom_size, S = P.shadow_map_size;
     FIBER_CUDA(cudaMemsetAsync(c->d_counters.p, 0, sizeof(FrameCounters), s));
     FIBER_CUDA(cudaMemsetAsync(c->d_page_table.p, 0, table * 4, s));
-    FIBER_CUDA(cudaMemsetAsync(c->d_active_flags.p, 0, table * 4, s));
+    FIBER_CUDA(cudaMemsetAsync(c->d_tile_work.p, 0, table * 4, s));
     FIBER_CUDA(cudaMemsetAsync(c->d_color.p, 0, WH * 8, s));
     FIBER_CUDA(cudaMemsetAsync(c->d_depth.p, 0, WH * 4, s));
     if (P.fragment_counts) FIBER_CUDA(cudaMemsetAsync(c->d_fragments.p, 0, WH * 4, s));
@@ -391,28 +393,28 @@ fiber_status run_prepass(fiber_ctx* c, cudaStream_t s, const OpaqueSource* opaqu
     set_stage(c, A, kStagePrefix);
     launch_prefix(L, A, csr);
     if (csr) launch_build_pages(L, A);
-    record(c, 6, s);
-    if (csr) launch_fill_walk(L, A);
-    else launch_fill(L, A);
-    record(c, 7, s);
-    // The cell sort needs only the fill; the active-tile compaction and the
-    // emit need only the counts. The sort runs on the side stream beside
-    // them (a branch of the frame graph when captured) and joins before the
-    // rasters.
+    // The active-tile compaction and the emit need only the counts, the fill
+    // and the cell sort only the offsets: the first two run on the side stream
+    // beside the fill (a branch of the frame graph when captured) and join
+    // before the sort, whose blocks would leave them no room.
     cudaStream_t side = c->side_override ? c->side_override : c->side_stream;
     FIBER_CUDA(cudaEventRecord(c->ev_fork, s));
     FIBER_CUDA(cudaStreamWaitEvent(side, c->ev_fork, 0));
     LaunchCtx Ls = L;
     Ls.stream = side;
-    launch_sort_cells(Ls, A);
-    launch_sort_big(Ls, A);
+    PrepassArgs As = A;
+    set_stage(c, As, kStageActive);
+    launch_compact_active(Ls, As, dp<unsigned long long>(c->d_lb) + c->lb_offset[kStageEmit]);
+    launch_emit(Ls, As, c->P.work_capacity);
     FIBER_CUDA(cudaEventRecord(c->ev_join, side));
-    set_stage(c, A, kStageActive);
-    launch_compact_active(L, A);
-    record(c, 8, s);
-    set_stage(c, A, kStageEmit);
-    launch_emit(L, A);
+    record(c, 6, s);
+    if (csr) launch_fill_walk(L, A);
+    else launch_fill(L, A);
+    record(c, 7, s);
     FIBER_CUDA(cudaStreamWaitEvent(s, c->ev_join, 0));
+    record(c, 8, s);
+    launch_sort_cells(L, A);
+    launch_sort_big(L, A);
     if (L.telemetry) launch_telemetry(L, A);
     return check_launch();
 }
@@ -583,7 +585,7 @@ fiber_status fiber_ctx_destroy(fiber_ctx* c) {
     DevBuf* bufs[] = {&c->d_params, &c->d_inst, &c->d_counters, &c->d_lb, &c->d_range_valid, &c->d_ranges,
                       &c->d_keep, &c->d_inst_visible, &c->d_inst_keep, &c->d_lut, &c->d_lut_tree, &c->d_tasks, &c->d_projected,
                       &c->d_page_table, &c->d_page_meta, &c->d_counts, &c->d_offsets, &c->d_cursors,
-                      &c->d_active_flags, &c->d_active_list, &c->d_work, &c->d_runs,
+                      &c->d_tile_work, &c->d_tile_slot, &c->d_page_items, &c->d_active_list, &c->d_work, &c->d_runs,
                       &c->d_big_cells, &c->d_dom_depth, &c->d_dom_opacity, &c->d_shadow_map, &c->d_atlas,
                       &c->d_history[0], &c->d_history[1], &c->d_color, &c->d_depth, &c->d_fragments,
                       &c->d_validate, &c->d_host_scene, &c->d_host_depth, &c->d_visit_rec,
@@ -926,7 +928,7 @@ static fiber_status frame_begin_views(fiber_ctx* c, const fiber_view* views, uin
     // Look-back status regions.
     uint64_t fine_tiles_lb = P.fine_tile_base[P.F];
     uint64_t lb_sizes[kStageCount] = {fine_tiles_lb + 1, table / 1024 + 2, page_cap + 1, table / 1024 + 2,
-                                      fine_tiles + 1};
+                                      table / 1024 + 2};
     uint64_t lb_total = 0;
     for (int i = 0; i < kStageCount; ++i) {
         c->lb_offset[i] = (uint32_t)lb_total;
@@ -959,7 +961,9 @@ static fiber_status frame_begin_views(fiber_ctx* c, const fiber_view* views, uin
     ENSURE(c->d_counts, page_cap * kPageSize * 4, false);
     ENSURE(c->d_offsets, page_cap * kPageSize * 4, false);
     ENSURE(c->d_cursors, page_cap * kPageSize * 4, false);
-    ENSURE(c->d_active_flags, fine_tiles * 4, false);
+    ENSURE(c->d_tile_work, fine_tiles * 4, false);
+    ENSURE(c->d_tile_slot, fine_tiles * sizeof(uint2), false);
+    ENSURE(c->d_page_items, page_cap * 16, false);
     ENSURE(c->d_active_list, fine_tiles * 4, false);
     ENSURE(c->d_work, work_cap * sizeof(fiber_raster_work_item), false);
     ENSURE(c->d_runs, fine_tiles * sizeof(fiber_raster_tile_run), false);

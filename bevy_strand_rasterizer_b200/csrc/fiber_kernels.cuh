@@ -71,7 +71,9 @@ struct PrepassArgs {
     uint32_t* counts;
     uint32_t* offsets;
     uint32_t* cursors;
-    uint32_t* active_flags;
+    uint32_t* tile_work;             // [fine tiles] work items of each on-screen fine tile (0: not active)
+    uint8_t* page_items;             // [pages][16] non-empty cells of each of a page's fine tiles
+    uint2* tile_slot;                // [fine tiles] (active index, first work item) of each active one
     uint32_t* active_list;
     fiber_raster_work_item* work;
     fiber_raster_tile_run* runs;
@@ -192,8 +194,9 @@ void launch_page_csr_count(const LaunchCtx& L, const PrepassArgs& A);
 void launch_build_pages(const LaunchCtx& L, const PrepassArgs& A);
 void launch_fill_walk(const LaunchCtx& L, const PrepassArgs& A);
 void launch_fill(const LaunchCtx& L, const PrepassArgs& A);
-void launch_compact_active(const LaunchCtx& L, const PrepassArgs& A);
-void launch_emit(const LaunchCtx& L, const PrepassArgs& A);
+// lb_work: the look-back words of the work-item sums (stage kStageEmit).
+void launch_compact_active(const LaunchCtx& L, const PrepassArgs& A, unsigned long long* lb_work);
+void launch_emit(const LaunchCtx& L, const PrepassArgs& A, uint32_t work_capacity);
 void launch_sort_cells(const LaunchCtx& L, const PrepassArgs& A);
 void launch_sort_big(const LaunchCtx& L, const PrepassArgs& A);
 void launch_telemetry(const LaunchCtx& L, const PrepassArgs& A);
