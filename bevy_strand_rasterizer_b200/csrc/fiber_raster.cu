@@ -18,7 +18,7 @@
 // Both rasters are bound by instruction issue, so the walk is written for few
 // instructions with the results of the plain binary32 formulas, bit for bit:
 // packed pairs (.f32x2) for what comes in pairs, and quotients and square roots
-// by a reciprocal estimate and fused corrections (see Exact below) instead of
+// by a reciprocal estimate and fused corrections (fiber_device.cuh) instead of
 // the general-range division and square root.
 #include "fiber_kernels.cuh"
 
@@ -68,37 +68,7 @@ __device__ __forceinline__ float sum2(F2 v) {
     return __fadd_rn(x, y);
 }
 
-// ---------------------------------------------------------------------------
-// Exact: correctly rounded reciprocal, quotient and square root from an
-// approximate one and fused corrections (P. Markstein, "IA-64 and Elementary
-// Functions", 2000), for operands whose intermediate values stay in the normal
-// range (staging sends every other case to the plain operators).
-//   rcp   y0 + y0 (1 - x y0): equals the rounded 1 / x for every mantissa.
-//   div   q0 = a y, q0 + y (a - b q0) with y the rounded 1 / b: equals the
-//         rounded a / b. Away from a rounding boundary the corrected quotient's
-//         error (below 6 parts in 2 b 2^24 of an ulp) cannot cross it; the 46.5
-//         million (a, b) whose quotient lies within 8 such parts of one were
-//         enumerated and all agree with the division operator.
-//   sqrt  s0 = x y, s0 + (y / 2)(x - s0^2): equals the rounded root for every
-//         mantissa and exponent parity.
-// rcp and sqrt were compared with the operators over all 1.7e9 binary32 values
-// of magnitude 2^-100 to 2^101.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ float rcp_estimate(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ float rsqrt_estimate(float x) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-// a / b with y = 1 / b rounded.
-__device__ __forceinline__ float div_by_rcp(float a, float b, float y) {
-    const float q = __fmul_rn(a, y);
-    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
-}
+// Two square roots and two quotients at once (see Exact in fiber_device.cuh).
 __device__ __forceinline__ F2 sqrt2_exact(Mul2 mul2, float x0, float x1) {
     const F2 x = pack2(x0, x1), y = pack2(rsqrt_estimate(x0), rsqrt_estimate(x1));
     const F2 s = mul2(x, y);

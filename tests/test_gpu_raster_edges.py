@@ -82,3 +82,16 @@ def test_round_boundaries(strands):
     pos[:, :, 2] = rng.uniform(-0.05, 0.05, (strands, 1))
     _strands(scene, pos)
     _compare(scene)
+
+
+@pytest.mark.parametrize("scale", [1e-6, 1e13])
+def test_scene_scale(scale):
+    # 1e13: clip coordinates beyond the range of the projection's shared
+    # reciprocal (w above 2^40); 1e-6: far below the near plane's distance.
+    scene = build_scene("tiny", settings_overrides=SETTINGS)
+    packed, material, m = scene.assets[0]
+    m = m.copy()
+    m[0] = m[5] = m[10] = scale
+    scene.assets[0] = (packed, material, m)
+    _camera(scene, eye=(0.0, 0.0, 0.6 * max(scale, 1.0)))
+    _compare(scene)
