@@ -111,7 +111,7 @@ struct fiber_ctx {
     DevBuf d_lut_tree;  // per coarse tile: the slice lookup's search tree (kLutTreeWords)
     DevBuf d_lut, d_tasks, d_projected, d_page_table, d_page_meta, d_counts, d_offsets, d_cursors;
     DevBuf d_tile_work, d_tile_slot, d_page_items, d_active_list, d_work, d_runs, d_big_cells;
-    DevBuf d_visit_rec, d_visit_task, d_visit_rank, d_task_key, d_cells_small, d_cells_mid, d_cells_large;
+    DevBuf d_visit_rec, d_visit_task, d_visit_rank, d_task_key, d_cells_small, d_cells_quad, d_cells_mid, d_cells_large;
     DevBuf d_opaque;  // (covered, farthest depth q) per camera fine tile
     DevBuf d_task_rec, d_ref_task;  // the rasters' record of each task; each reference's task
     DevBuf d_page_nvis, d_page_vbase, d_page_bucket;  // page-CSR backend
@@ -246,6 +246,7 @@ PrepassArgs prepass_args(fiber_ctx* c) {
     A.visit_rank = dp<uint32_t>(c->d_visit_rank);
     A.task_key = dp<uint32_t>(c->d_task_key);
     A.cells_small = dp<uint2>(c->d_cells_small);
+    A.cells_quad = dp<uint2>(c->d_cells_quad);
     A.cells_mid = dp<uint2>(c->d_cells_mid);
     A.cells_large = dp<uint2>(c->d_cells_large);
     A.opaque_tiles = dp<uint2>(c->d_opaque);
@@ -590,7 +591,7 @@ fiber_status fiber_ctx_destroy(fiber_ctx* c) {
                       &c->d_history[0], &c->d_history[1], &c->d_color, &c->d_depth, &c->d_fragments,
                       &c->d_validate, &c->d_host_scene, &c->d_host_depth, &c->d_visit_rec,
                       &c->d_visit_task, &c->d_visit_rank, &c->d_task_key,
-                      &c->d_cells_small, &c->d_cells_mid, &c->d_cells_large, &c->d_opaque, &c->d_page_nvis, &c->d_page_vbase,
+                      &c->d_cells_small, &c->d_cells_quad, &c->d_cells_mid, &c->d_cells_large, &c->d_opaque, &c->d_page_nvis, &c->d_page_vbase,
                       &c->d_page_bucket, &c->d_tel, &c->d_tel_slots, &c->d_dom_page_table, &c->d_dom_pool,
                       &c->d_task_rec, &c->d_ref_task};
     for (DevBuf* b : bufs) release(c, *b);
@@ -978,7 +979,8 @@ static fiber_status frame_begin_views(fiber_ctx* c, const fiber_view* views, uin
     ENSURE(c->d_task_key, task_cap * 4, false);
     // Non-empty cells: at most one per kept reference and one per cell.
     ENSURE(c->d_cells_small, std::min<uint64_t>(ref_cap, page_cap * kPageSize) * sizeof(uint2), false);
-    ENSURE(c->d_cells_mid, (ref_cap / 9 + 1) * sizeof(uint2), false);
+    ENSURE(c->d_cells_quad, (ref_cap / 9 + 1) * sizeof(uint2), false);
+    ENSURE(c->d_cells_mid, (ref_cap / 17 + 1) * sizeof(uint2), false);
     ENSURE(c->d_cells_large, (ref_cap / 33 + 1) * sizeof(uint2), false);
     ENSURE(c->d_opaque, (uint64_t)c->camera_fine_tiles * sizeof(uint2), false);
     ENSURE(c->d_task_rec, task_cap * kTaskRec * sizeof(float4), false);

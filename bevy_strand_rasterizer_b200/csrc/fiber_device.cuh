@@ -109,14 +109,15 @@ struct FrameCounters {
     uint32_t tile_counter[8];     // virtual block ids of the look-back stages
     uint32_t visit_overflow;      // visit records unused this frame (did not fit, or disabled)
     unsigned long long visits;    // visit records appended by k_visit
-    uint32_t small_cells;         // cells of 2..8 references listed for the cell sort
-    uint32_t large_cells;         // cells of more than 32 references listed for the cell sort
+    uint32_t list_cells[4];       // cells listed for the cell sort, by size class (CellList)
     uint32_t opaque_bound;        // the opaque fine-tile depths of this frame are written
     uint32_t dom_pages;           // DOM pages requested this frame (sparse residency)
-    uint32_t mid_cells;           // cells of 9..32 references listed for the cell sort
     uint32_t seg_unordered;       // some instance's strands do not follow one another in its index slab
 };
-static_assert(sizeof(FrameCounters) == 176 + 4 * (kMaxFrusta - 16), "FrameCounters layout");
+static_assert(sizeof(FrameCounters) == 184 + 4 * (kMaxFrusta - 16), "FrameCounters layout");
+
+// Size classes of the cell sort's lists: 2..8, 9..16, 17..32 and more references.
+enum CellList : uint32_t { kListSmall = 0, kListQuad = 1, kListMid = 2, kListLarge = 3 };
 
 // Look-back stages (index into FrameCounters::tile_counter and the status regions).
 enum LookbackStage : uint32_t { kStageFine = 0, kStageAlloc = 1, kStagePrefix = 2, kStageActive = 3, kStageEmit = 4, kStageCount = 5 };

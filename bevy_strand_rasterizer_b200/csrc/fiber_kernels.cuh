@@ -83,7 +83,8 @@ struct PrepassArgs {
     uint32_t* visit_rank;   // [ref_capacity] rank of the visit inside its cell
     uint32_t* task_key;            // [task_capacity] depth key of the task's reference (projected z0 + z1, 17 bits)
     uint2* cells_small;            // (ref base, count) of cells with 2..8 references
-    uint2* cells_mid;              // (ref base, count) of cells with 9..32 references
+    uint2* cells_quad;             // (ref base, count) of cells with 9..16 references
+    uint2* cells_mid;              // (ref base, count) of cells with 17..32 references
     uint2* cells_large;            // (ref base, count) of cells with more than 32
     uint2* opaque_tiles;           // [camera fine tiles] (fully covered, quantised farthest opaque depth)
     float4* task_rec;              // [task_capacity][kTaskRec] what the rasters read of a task

@@ -512,6 +512,7 @@ constexpr uint32_t kVisitSlots = 32;  // buffered visits per task; p99 is about 
 // Cell sort sizes: a thread sorts a cell of up to 8 references, a warp one of
 // up to 256 (32 lanes x 8 registers), a block anything longer.
 constexpr uint32_t kThreadSortMax = 8;
+constexpr uint32_t kQuadSortMax = 16;   // 4 lanes x 4 registers: eight cells per warp
 constexpr uint32_t kGroupSortMax = 32;  // 8 lanes x 4 registers: four cells per warp
 constexpr uint32_t kWarpSortMax = 256;
 
@@ -1090,26 +1091,29 @@ __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restr
         const uint4 ca = *reinterpret_cast<const uint4*>(A.counts + g0);
         const uint4 cb = *reinterpret_cast<const uint4*>(A.counts + g0 + 4u);
         const uint32_t c[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
-        uint32_t e[8], sum = 0u, nsmall = 0u, nmid = 0u, nlarge = 0u;
+        uint32_t e[8], sum = 0u, nsmall = 0u, nquad = 0u, nmid = 0u, nlarge = 0u;
 #pragma unroll
         for (uint32_t k = 0; k < 8u; ++k) {
             e[k] = sum;
             sum += c[k];
             nsmall += (c[k] >= 2u && c[k] <= kThreadSortMax) ? 1u : 0u;
-            nmid += (c[k] > kThreadSortMax && c[k] <= kGroupSortMax) ? 1u : 0u;
+            nquad += (c[k] > kThreadSortMax && c[k] <= kQuadSortMax) ? 1u : 0u;
+            nmid += (c[k] > kQuadSortMax && c[k] <= kGroupSortMax) ? 1u : 0u;
             nlarge += c[k] > kGroupSortMax ? 1u : 0u;
         }
-        // One scan carries the reference count (exclusive per cell) and, packed
-        // 10 bits each, the small / mid / large cell counts for the lists.
-        const uint32_t mine = nsmall | (nmid << 10) | (nlarge << 20);
-        uint32_t x = sum, y = mine;
+        // The scans carry the reference count (exclusive per cell) and, packed
+        // 16 bits each, the cell counts of the lists' size classes.
+        const uint32_t mine = nsmall | (nquad << 16), mine2 = nmid | (nlarge << 16);
+        uint32_t x = sum, y = mine, z = mine2;
 #pragma unroll
         for (uint32_t o = 1; o < 32u; o <<= 1) {
             const uint32_t xa = __shfl_up_sync(0xFFFFFFFFu, x, o), ya = __shfl_up_sync(0xFFFFFFFFu, y, o);
-            if (lane >= o) { x += xa; y += ya; }
+            const uint32_t za = __shfl_up_sync(0xFFFFFFFFu, z, o);
+            if (lane >= o) { x += xa; y += ya; z += za; }
         }
         const uint32_t total = __shfl_sync(0xFFFFFFFFu, x, 31), both = __shfl_sync(0xFFFFFFFFu, y, 31);
-        const uint32_t lane_base = x - sum, list_base = y - mine;
+        const uint32_t both2 = __shfl_sync(0xFFFFFFFFu, z, 31);
+        const uint32_t lane_base = x - sum, list_base = y - mine, list_base2 = z - mine2;
 #pragma unroll
         for (uint32_t k = 0; k < 8u; ++k) e[k] += lane_base;
         *reinterpret_cast<uint4*>(A.offsets + g0) = make_uint4(e[0], e[1], e[2], e[3]);
@@ -1143,23 +1147,25 @@ __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restr
             continue;
         }
         // The page's cells for k_sort_cells, in cell order: 2..8 references in
-        // the small list, 9..32 in the middle one, more in the large one (a
-        // single reference is in order).
-        uint32_t s_small = 0u, s_mid = 0u, s_large = 0u;
-        if (lane == 0u) {
-            const uint32_t ns = both & 0x3FFu, nm = (both >> 10) & 0x3FFu, nl = both >> 20;
-            s_small = ns ? atomicAdd(&A.counters->small_cells, ns) : 0u;
-            s_mid = nm ? atomicAdd(&A.counters->mid_cells, nm) : 0u;
-            s_large = nl ? atomicAdd(&A.counters->large_cells, nl) : 0u;
+        // the small list, 9..16 in the quad one, 17..32 in the middle one, more in
+        // the large one (a single reference is in order). Lanes 0..3 reserve the
+        // lists' room at once.
+        uint32_t room = 0u;
+        if (lane < 4u) {
+            const uint32_t w = lane < 2u ? both : both2, want = lane & 1u ? w >> 16 : w & 0xFFFFu;
+            if (want) room = atomicAdd(&A.counters->list_cells[lane], want);
         }
-        uint32_t ks = __shfl_sync(0xFFFFFFFFu, s_small, 0) + (list_base & 0x3FFu);
-        uint32_t km = __shfl_sync(0xFFFFFFFFu, s_mid, 0) + ((list_base >> 10) & 0x3FFu);
-        uint32_t kl = __shfl_sync(0xFFFFFFFFu, s_large, 0) + (list_base >> 20);
+        uint32_t ks = __shfl_sync(0xFFFFFFFFu, room, 0) + (list_base & 0xFFFFu);
+        uint32_t kq = __shfl_sync(0xFFFFFFFFu, room, 1) + (list_base >> 16);
+        uint32_t km = __shfl_sync(0xFFFFFFFFu, room, 2) + (list_base2 & 0xFFFFu);
+        uint32_t kl = __shfl_sync(0xFFFFFFFFu, room, 3) + (list_base2 >> 16);
 #pragma unroll
         for (uint32_t k = 0; k < 8u; ++k) {
-            if (c[k] >= 2u && c[k] <= kThreadSortMax) A.cells_small[ks++] = make_uint2(base + e[k], c[k]);
-            else if (c[k] > kThreadSortMax && c[k] <= kGroupSortMax) A.cells_mid[km++] = make_uint2(base + e[k], c[k]);
-            else if (c[k] > kGroupSortMax) A.cells_large[kl++] = make_uint2(base + e[k], c[k]);
+            const uint2 cell = make_uint2(base + e[k], c[k]);
+            if (c[k] >= 2u && c[k] <= kThreadSortMax) A.cells_small[ks++] = cell;
+            else if (c[k] > kThreadSortMax && c[k] <= kQuadSortMax) A.cells_quad[kq++] = cell;
+            else if (c[k] > kQuadSortMax && c[k] <= kGroupSortMax) A.cells_mid[km++] = cell;
+            else if (c[k] > kGroupSortMax) A.cells_large[kl++] = cell;
         }
         // append_active_fine_tile (:2207-2238): each of the page's 16 fine tiles
         // that lies on screen gets its non-empty cells, the tile's work items of
@@ -1357,13 +1363,26 @@ struct ByRecord {
         return ByRecord{__shfl_xor_sync(0xFFFFFFFFu, w, mask), __shfl_xor_sync(0xFFFFFFFFu, t, mask)};
     }
 };
+// Compare and exchange by selects: as branches the exchanges diverged and most
+// of the sort's time was branch resolution (291 M -> 105 M warp
+// instructions, 0.42 -> 0.19 ms for the 23 M references of the medium frame).
+__device__ __forceinline__ ByTask pick(bool p, ByTask a, ByTask b) { return ByTask{p ? a.w : b.w}; }
+__device__ __forceinline__ ByRecord pick(bool p, ByRecord a, ByRecord b) {
+    return ByRecord{p ? a.w : b.w, p ? a.t : b.t};
+}
+// Whether the lane that keeps the smaller (or the larger) of a pair takes the
+// other lane's. Words of ByTask differ or are both padding; keys of ByRecord
+// repeat where strands share segments, and then both lanes keep their own.
+__device__ __forceinline__ bool takes_other(ByTask o, ByTask own, bool smaller) { return (o.w < own.w) == smaller; }
+__device__ __forceinline__ bool takes_other(ByRecord o, ByRecord own, bool smaller) {
+    return smaller ? o.w < own.w : o.w > own.w;
+}
 template <class E>
 __device__ __forceinline__ void order(E& a, E& b, bool up) {
-    if (up ? (a.w > b.w) : (a.w < b.w)) {
-        const E x = a;
-        a = b;
-        b = x;
-    }
+    const bool exchange = (a.w > b.w) == up;
+    const E x = pick(exchange, b, a), y = pick(exchange, a, b);
+    a = x;
+    b = y;
 }
 
 // A group of G lanes (G-aligned inside the warp) sorts one cell of up to G x R
@@ -1393,7 +1412,7 @@ __device__ __forceinline__ void group_sort_cell(const PrepassArgs& A, uint32_t b
                     const E o = k[r].other(stride / R);
                     const bool up = (e & size) == 0;
                     const bool lower = (e & stride) == 0;
-                    if (lower == up ? (o.w < k[r].w) : (o.w > k[r].w)) k[r] = o;
+                    k[r] = pick(takes_other(o, k[r], lower == up), o, k[r]);
                 }
             } else {
 #pragma unroll
@@ -1534,14 +1553,20 @@ __device__ __forceinline__ void warp_sort_small_cells(const PrepassArgs& A, uint
 template <class E>
 __device__ __forceinline__ void sort_cells(const PrepassArgs& A, SortSpanSmem* s_span) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t n_small = *((volatile uint32_t*)&A.counters->small_cells);
-    const uint32_t n_large = *((volatile uint32_t*)&A.counters->large_cells);
+    const volatile uint32_t* n_cells = A.counters->list_cells;
+    const uint32_t n_small = n_cells[kListSmall], n_quad = n_cells[kListQuad];
+    const uint32_t n_mid = n_cells[kListMid], n_large = n_cells[kListLarge];
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; i0 < n_small; i0 += stride)
         warp_sort_small_cells(A, i0, n_small, lane, s_span, E{});
     const uint32_t warps = stride >> 5;
-    // Cells of 9..32 references: four per warp, eight lanes each.
-    const uint32_t n_mid = *((volatile uint32_t*)&A.counters->mid_cells);
+    // Cells of 9..16 references: eight per warp, four lanes each.
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 8u < n_quad; w += warps) {
+        const uint32_t ci = w * 8u + (lane >> 2);
+        const uint2 e = ci < n_quad ? A.cells_quad[ci] : make_uint2(0u, 0u);
+        group_sort_cell<E, 4, 4>(A, e.x, e.y, (int)lane);
+    }
+    // Cells of 17..32: four per warp, eight lanes each.
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 4u < n_mid; w += warps) {
         const uint32_t ci = w * 4u + (lane >> 3);
         const uint2 e = ci < n_mid ? A.cells_mid[ci] : make_uint2(0u, 0u);
@@ -1557,14 +1582,13 @@ __device__ __forceinline__ void sort_cells(const PrepassArgs& A, SortSpanSmem* s
 
 // Canonical order inside every cell, in place, after the fill, over the cell
 // lists k_prefix_pages made: a warp per 32 cells of 2..8 references (a lane per
-// cell), four cells of 9..32 references per warp (eight lanes each), then a
-// warp per larger cell; a cell longer than a warp sort is queued for
-// k_sort_big_cells. Bound by instruction issue (the networks' 64-bit compares)
-// and the L2 latency of the key gathers. Writing 4 B task indices in place
-// instead of 20 B of reference, key and task, and sorting one word instead of
-// a word and its task, took this kernel from 0.57 to 0.37 ms for the 23.5 M
-// references of the medium frame and from 11.8 to 7.6 ms for the large
-// frame's 349 M.
+// cell), eight cells of 9..16 references per warp (four lanes each), four of
+// 17..32 (eight lanes each), then a warp per larger cell; a cell longer than a warp sort is queued for
+// k_sort_big_cells. Bound by the networks' 64-bit compares and selects (ALU pipe
+// 71 % busy); the key gathers hide behind them (2 % of the time). The start
+// wrote 20 B of reference, key and task per entry and sorted a word beside its
+// task by branches: 0.57 -> 0.19 ms for the medium frame, 11.8 -> 4.9 ms for
+// the large frame's 349 M references.
 __global__ void __launch_bounds__(256, 5) k_sort_cells(PrepassArgs A) {
     if (frame_failed(A.counters)) return;
     __shared__ SortSpanSmem s_span[8];
