@@ -28,8 +28,19 @@ constexpr float kPiHalf = kPi / 2.0f;
 __device__ __forceinline__ float dot3(F3 a, F3 b) {
     return __fadd_rn(__fadd_rn(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)), __fmul_rn(a.z, b.z));
 }
+// v / |v|. One corrected root and reciprocal serve the three quotients (see
+// Exact in fiber_device.cuh) where the squared length is of ordinary size; a
+// component below 2^-79 beside a length of at least 2^-40 may round the other
+// way, 2^-39 of the vector at most. Zero, infinite and NaN lengths take the
+// plain operators.
 __device__ __forceinline__ F3 nrm3(F3 v) {
-    const float l = __fsqrt_rn(dot3(v, v));
+    const float d = dot3(v, v);
+    if (d >= 8.2718061e-25f && d <= 1.2e24f) {  // 2^-80 .. 2^80
+        const float e = rsqrt_estimate(d), s = __fmul_rn(d, e);
+        const float l = __fmaf_rn(__fmaf_rn(-s, s, d), __fmul_rn(0.5f, e), s), y = rcp_exact(l);
+        return f3(div_by_rcp(v.x, l, y), div_by_rcp(v.y, l, y), div_by_rcp(v.z, l, y));
+    }
+    const float l = __fsqrt_rn(d);
     return f3(__fdiv_rn(v.x, l), __fdiv_rn(v.y, l), __fdiv_rn(v.z, l));
 }
 __device__ __forceinline__ F3 cross3(F3 a, F3 b) {
@@ -82,7 +93,7 @@ __device__ __forceinline__ float fresnel_reflectance(float eta_t, float ratio, f
 struct Detector {
     float var, norm, neg_inv_two_var, reach;
     bool near3;  // var < 2: the three wrapped terms nearest to phi carry the sum
-    bool near1;  // var < 0.26: the nearest term alone does
+    bool near1;  // 1e-6 <= var < 0.26: the nearest term alone does
 };
 
 __device__ __forceinline__ Detector make_detector(float beta) {
@@ -93,8 +104,20 @@ __device__ __forceinline__ Detector make_detector(float beta) {
     g.neg_inv_two_var = -1.0f / two_var;
     g.reach = sqrtf(110.0f * two_var) * 1.001f + 1e-3f;
     g.near3 = g.var < 2.0f;
-    g.near1 = g.var < 0.26f;
+    g.near1 = g.var >= 1e-6f && g.var < 0.26f;
     return g;
+}
+
+// The nearest wrapped term alone, for var < 0.26: with k_c the wrap nearest to
+// phi (|phi - 2 pi k_c| <= pi; |phi| stays below 19, so k_c is inside -10..10)
+// every other term is below exp(-pi^2 / (2 var)) < 5.8e-9 (|phi - 2 pi k| >=
+// pi), and the 20 of them change the detector by less than 1.2e-8 norm. Adding
+// and taking away 1.5 2^23 rounds to the nearest integer. NaN stays NaN.
+__device__ __forceinline__ float nearest_detector(const Detector& g, float phi_delta) {
+    const float magic = 12582912.0f;
+    const float kc = __fsub_rn(__fmaf_rn(phi_delta, 1.0f / (2.0f * kPi), magic), magic);
+    const float a = phi_delta - (2.0f * kPi) * kc;
+    return g.norm * __expf((a * a) * g.neg_inv_two_var);
 }
 
 // Sum of the 21 wrapped Gaussians (k = -10..10). Terms whose exponent is below
@@ -105,25 +128,19 @@ __device__ __forceinline__ Detector make_detector(float beta) {
 // widened by 1e-3 relative + 1e-3 absolute), in the same increasing k order; a
 // NaN phi takes the full range. The exponent is a product with -1 / (2 var)
 // and exp is the hardware exp2 path (__expf), within the shading tolerance.
-__device__ __forceinline__ float gaussian_detector(const Detector& g, float phi_delta) {
+// Not inlined: six copies of it overflowed the instruction cache.
+__device__ __noinline__ float wide_detector(const Detector& g, float phi_delta) {
     if (g.var < 1e-6f) {
         float two_pi = 2.0f * kPi;
         float m = phi_delta - two_pi * truncf(phi_delta / two_pi);
         return fabsf(m) < 1e-3f ? 0.0f : 1e6f;
     }
-    // Let k_c be the wrap nearest to phi (|phi - 2 pi k_c| <= pi; |phi| < 56
-    // keeps k_c +- 1 inside k = -10..10). Nearest term alone: with var < 0.26
-    // every other term is below exp(-pi^2 / (2 var)) < 5.8e-9 (|phi - 2 pi k|
-    // >= pi), and the 20 of them change the detector by less than 1.2e-8 norm.
-    if (g.near1 && fabsf(phi_delta) < 56.0f) {
-        const float a = phi_delta - (2.0f * kPi) * rintf(phi_delta * (1.0f / (2.0f * kPi)));
-        return g.norm * __expf((a * a) * g.neg_inv_two_var);
-    }
     // Three nearest terms: every k other than k_c and k_c +- 1 has
     // |phi - 2 pi k| >= 3 pi, so its term is below exp(-9 pi^2 / (2 var)) <
     // 2.3e-10 for var < 2; the at most 18 such terms change the detector by
     // less than 4.2e-9 norm, far inside the shading tolerance. Summed in
-    // increasing k, as the full loop does.
+    // increasing k, as the full loop does. |phi| < 56 keeps k_c +- 1 inside
+    // k = -10..10.
     if (g.near3 && fabsf(phi_delta) < 56.0f) {
         const float two_pi = 2.0f * kPi;
         const float kc = rintf(phi_delta * (1.0f / two_pi));
@@ -166,6 +183,53 @@ __device__ __forceinline__ void fill_quad_table(QuadTable& t) {
     }
 }
 
+// The quadrature point's Fresnel and absorption terms depend on the segment
+// only, not on the path p, and on the root's magnitude only: the roots are
+// +-h pairs with equal weights, asin is odd and the terms take its cosine.
+// So they are evaluated once per pair (five times instead of ten, of which
+// they were most of the shading's instructions), and a pair adds its two
+// detector values, at azimuth shifts of opposite odd part. asin(h) serves
+// gamma_i and the azimuth shift alike, and asin(clamp(x)) equals asin(x)
+// whenever |x| <= 1. The path powers are exact products: pow(x, 0) = 1,
+// pow(x, 1) = x and pow(x, 2) = x * x correctly rounded.
+template <bool kNear1>
+__device__ __forceinline__ void quadrature(const QuadTable& qt, float eta, float inv_eta, float inv_eta_prime, float cos_td,
+                                           const float* mup, float phi, const Detector& det_azim, float (&acc)[3][3]) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < 5u; ++i) {
+        const float h = qt.h[i];
+        // A (:383-413)
+        const float x_t = h * inv_eta_prime;
+        float gamma_t = asinf(x_t);
+        float gamma_i = qt.gi[i];
+        float fr = fresnel_reflectance(eta, inv_eta, acosf(cos_td * qt.cgi[i]));
+        float c2 = 1.0f + __cosf(2.0f * gamma_t);
+        float T[3] = {__expf(-2.0f * mup[0] * c2), __expf(-2.0f * mup[1] * c2), __expf(-2.0f * mup[2] * c2)};
+        float f_ = 1.0f - fr;
+        // Phi (:464-468)
+        float gt2 = fabsf(x_t) <= 1.0f ? gamma_t : asinf(wclamp(x_t, -1.0f, 1.0f));
+        const float w = c_leg_weights[i];
+#pragma unroll
+        for (uint32_t p = 0; p < 3u; ++p) {
+            float A[3];
+            if (p == 0u) {
+                for (int q = 0; q < 3; ++q) A[q] = fr * T[q] * T[q];
+            } else if (p == 1u) {
+                float k = (f_ * f_) * 1.0f;
+                for (int q = 0; q < 3; ++q) A[q] = k * T[q];
+            } else {
+                float k = (f_ * f_) * fr;
+                for (int q = 0; q < 3; ++q) A[q] = k * (T[q] * T[q]);
+            }
+            const float odd = 2.0f * u2f(p) * gt2 - 2.0f * gamma_i, even = u2f(p) * kPi;
+            const float d0 = phi - (even + odd), d1 = phi - (even - odd);
+            const float det = kNear1 ? nearest_detector(det_azim, d0) + nearest_detector(det_azim, d1)
+                                     : wide_detector(det_azim, d0) + wide_detector(det_azim, d1);
+            for (int q = 0; q < 3; ++q) acc[p][q] = acc[p][q] + A[q] * det * w;
+        }
+    }
+}
+
 __device__ F3 marschner(F3 L, F3 V, F3 U, const fiber_strand_material& m, float occlusion, const QuadTable& qt,
                         const Detector& det_azim) {
     float theta_i = acosf(dot3(L, U));
@@ -186,7 +250,9 @@ __device__ F3 marschner(F3 L, F3 V, F3 U, const fiber_strand_material& m, float 
         float trs = theta_r + m.shift;
         float ti = wclamp(-kPiHalf + 1e-6f, kPiHalf - 1e-6f, theta_i);
         trs = wclamp(-kPiHalf + 1e-6f, kPiHalf - 1e-6f, trs);
-        float cti = cosf(-ti), ctr = cosf(trs), sti = sinf(-ti), strs = sinf(trs);
+        float cti, ctr, sti, strs;
+        sincosf(-ti, &sti, &cti);
+        sincosf(trs, &strs, &ctr);
         if (v_long < 1e-6f) {
             float tol = 0.1f * (kPi / 180.0f);
             mp = fabsf(trs + ti) < tol ? 0.0f : 1e6f / tol;
@@ -215,42 +281,9 @@ __device__ F3 marschner(F3 L, F3 V, F3 U, const fiber_strand_material& m, float 
     const float inv_eta = 1.0f / m.eta;
     float mup[3] = {sig[0] / ctd, sig[1] / ctd, sig[2] / ctd};
     const float cos_td = ctd;  // cos(theta_d), the same evaluation
-    // The quadrature point's Fresnel, absorption and azimuth terms depend on
-    // the segment only, not on the path p, so they are evaluated once per point
-    // and reused by the three paths; each path's sum keeps its order (i = 0..9).
-    // asin(h) serves gamma_i and the azimuth shift alike, and asin(clamp(x))
-    // equals asin(x) whenever |x| <= 1. The path powers are exact products:
-    // pow(x, 0) = 1, pow(x, 1) = x and pow(x, 2) = x * x correctly rounded.
     float acc[3][3] = {{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}};
-    for (uint32_t i = 0; i < 10u; ++i) {
-        const float h = qt.h[i];
-        // A (:383-413)
-        const float x_t = h * inv_eta_prime;
-        float gamma_t = asinf(x_t);
-        float gamma_i = qt.gi[i];
-        float fr = fresnel_reflectance(m.eta, inv_eta, acosf(cos_td * qt.cgi[i]));
-        float c2 = 1.0f + __cosf(2.0f * gamma_t);
-        float T[3] = {__expf(-2.0f * mup[0] * c2), __expf(-2.0f * mup[1] * c2), __expf(-2.0f * mup[2] * c2)};
-        float f_ = 1.0f - fr;
-        // Phi (:464-468)
-        float gt2 = fabsf(x_t) <= 1.0f ? gamma_t : asinf(wclamp(x_t, -1.0f, 1.0f));
-        float asin_h = gamma_i;
-        for (uint32_t p = 0; p < 3u; ++p) {
-            float A[3];
-            if (p == 0u) {
-                for (int q = 0; q < 3; ++q) A[q] = fr * T[q] * T[q];
-            } else if (p == 1u) {
-                float k = (f_ * f_) * 1.0f;
-                for (int q = 0; q < 3; ++q) A[q] = k * T[q];
-            } else {
-                float k = (f_ * f_) * fr;
-                for (int q = 0; q < 3; ++q) A[q] = k * (T[q] * T[q]);
-            }
-            float shift = 2.0f * u2f(p) * gt2 - 2.0f * asin_h + u2f(p) * kPi;
-            float det = gaussian_detector(det_azim, phi - shift);
-            for (int q = 0; q < 3; ++q) acc[p][q] = acc[p][q] + A[q] * det * c_leg_weights[i];
-        }
-    }
+    if (det_azim.near1) quadrature<true>(qt, m.eta, inv_eta, inv_eta_prime, cos_td, mup, phi, det_azim, acc);
+    else quadrature<false>(qt, m.eta, inv_eta, inv_eta_prime, cos_td, mup, phi, det_azim, acc);
     for (uint32_t p = 0; p < 3u; ++p) {
         float wgt = (u2f(p + 1u) * vis) / 3.0f;
         for (int q = 0; q < 3; ++q) tot[q] = tot[q] + (acc[p][q] * 0.5f) * wgt;
@@ -258,6 +291,10 @@ __device__ F3 marschner(F3 L, F3 V, F3 U, const fiber_strand_material& m, float 
     return f3(tot[0], tot[1], tot[2]);
 }
 
+// Bound by instruction issue. Medium frame (2.97 M segments): 329 M -> 220 M warp
+// instructions and 0.43 -> 0.26 ms, by evaluating quadrature pairs together and
+// by keeping the rare detectors out of line (with six inlined copies of them a
+// third of the issue slots waited for instructions: 0.375 ms).
 __global__ void __launch_bounds__(128, 8) k_shade(const FrameParams* __restrict__ Pp,
                                                const InstanceView* __restrict__ inst, RenderArgs R) {
     if (frame_failed(R.counters)) return;
