@@ -856,10 +856,18 @@ static fiber_status frame_begin_views(fiber_ctx* c, const fiber_view* views, uin
         for (uint32_t i = i0; i < i0 + ni; ++i) ns += c->views[i].strand_count;
         P.view_strands[v] = ns;
     }
-    P.fine_tile_base[0] = 0u;
-    for (uint32_t f = 0; f < n_frusta; ++f)
-        P.fine_tile_base[f + 1] =
-            P.fine_tile_base[f] + (P.view_strands[P.fview[f]] + kFineStrandsPerTile - 1u) / kFineStrandsPerTile;
+    // k_fine's tiles: as many strands per warp, up to 8, as leave a tile for
+    // every resident block (4 per SM). Eight strands share a look-back on the
+    // medium and large frames; the tiny frame's 600 take 31 us as ten tiles of
+    // 64 strands and 14 us as 76 of 8.
+    P.fine_per_warp = kFineMaxPerWarp;
+    for (;; P.fine_per_warp /= 2u) {
+        const uint32_t per_tile = P.fine_per_warp * kFineTileWarps;
+        P.fine_tile_base[0] = 0u;
+        for (uint32_t f = 0; f < n_frusta; ++f)
+            P.fine_tile_base[f + 1] = P.fine_tile_base[f] + (P.view_strands[P.fview[f]] + per_tile - 1u) / per_tile;
+        if (P.fine_per_warp == 1u || P.fine_tile_base[n_frusta] >= 4u * (uint32_t)c->sm_count) break;
+    }
     P.n_views = nv;
     std::memcpy(P.camera_pos, views[0].camera.world_position, 12);
     std::memcpy(P.ambient, st.ambient_color, 16);

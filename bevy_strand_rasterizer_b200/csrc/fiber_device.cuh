@@ -25,8 +25,8 @@ constexpr uint32_t kMarked = 0xFFFFFFFEu;  // MARKED_COUNT_PAGE (strand_prepass.
 constexpr uint32_t kMaxFrusta = 128;  // frusta of a frame (a multi-view frame: every view's camera and lights)
 constexpr uint32_t kMaxViews = 64;    // views of a multi-view frame
 constexpr uint32_t kPixelSlots = 64;       // strand_rasterizer.wgsl:309,839
-// Strands per look-back tile of the fine prepass (k_fine).
-constexpr uint32_t kFineStrandsPerTile = 64;
+// A look-back tile of the fine prepass (k_fine): 8 warps of up to 8 strands.
+constexpr uint32_t kFineTileWarps = 8, kFineMaxPerWarp = 8;
 
 // Error words written by device code (never trap).
 constexpr uint32_t kErrTimeout = 1u;
@@ -86,6 +86,7 @@ struct FrameParams {
     uint32_t flayer[kMaxFrusta];         // DOM layer of a light frustum, kInvalid otherwise
     uint32_t layer_frustum[kMaxFrusta];  // frustum of each DOM layer
     uint32_t out_base[kMaxFrusta];       // first pixel of a camera's colour / depth / fragment image
+    uint32_t fine_per_warp;              // strands per warp of k_fine's tiles
     uint32_t fine_tile_base[kMaxFrusta + 1];  // k_fine's tiles of each frustum (prefix)
     uint32_t view_strand0[kMaxViews], view_strands[kMaxViews];  // a view's strands (global strand indices)
     uint32_t view_layer0[kMaxViews], view_layers[kMaxViews];    // a view's lights (DOM layers, light indices)

@@ -291,8 +291,8 @@ __global__ void k_lut(const FrameParams* __restrict__ Pp, PrepassArgs A) {
 
 // ===========================================================================
 // K2 + K6 fine prepass: a warp per strand (a lane per segment), each warp
-// taking kFineStrandsPerWarp consecutive strands, one block per (frustum,
-// kFineStrandsPerTile-strand chunk) in frustum-major order. Pass A counts
+// taking fine_per_warp consecutive strands (at most 8), one block per (frustum,
+// 8 fine_per_warp-strand tile) in frustum-major order. Pass A counts
 // every strand's clipped segments; the block takes its output offset from a
 // decoupled look-back; pass B projects again and writes BinningTask +
 // ProjectedSegment in (frustum, inst, strand, seg) order — the binning
@@ -301,8 +301,7 @@ __global__ void k_lut(const FrameParams* __restrict__ Pp, PrepassArgs A) {
 // ===========================================================================
 constexpr int kFineThreads = 256;
 constexpr int kFineWarps = kFineThreads / 32;
-constexpr uint32_t kFineStrandsPerWarp = kFineStrandsPerTile / kFineWarps;
-static_assert(kFineStrandsPerWarp * kFineWarps == kFineStrandsPerTile, "fine tile shape");
+static_assert(kFineWarps == (int)kFineTileWarps, "fine tile shape");
 
 struct SegOut {
     uint32_t seg;
@@ -366,6 +365,17 @@ __device__ __forceinline__ bool fine_chunk(const FrameParams& P, const InstanceV
 struct FineStrand {
     uint32_t i, s, nseg, meta_offset, packed, material;
     bool ordered;  // its segments follow the previous strand's in the index slab
+    __device__ __forceinline__ FineStrand of_lane(int k) const {
+        FineStrand r;
+        r.i = __shfl_sync(0xFFFFFFFFu, i, k);
+        r.s = __shfl_sync(0xFFFFFFFFu, s, k);
+        r.nseg = __shfl_sync(0xFFFFFFFFu, nseg, k);
+        r.meta_offset = __shfl_sync(0xFFFFFFFFu, meta_offset, k);
+        r.packed = __shfl_sync(0xFFFFFFFFu, packed, k);
+        r.material = __shfl_sync(0xFFFFFFFFu, material, k);
+        r.ordered = true;
+        return r;
+    }
 };
 
 __device__ __forceinline__ FineStrand fine_strand(const FrameParams& P, const InstanceView* __restrict__ inst,
@@ -414,7 +424,7 @@ __global__ void __launch_bounds__(kFineThreads, 4) k_fine(const FrameParams* __r
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // Each frustum's tiles cover its view's strands (every strand of a
     // single-view frame): fine_tile_base is their prefix over frusta.
-    const uint32_t n_tiles = P.fine_tile_base[P.F];
+    const uint32_t n_tiles = P.fine_tile_base[P.F], per_warp = P.fine_per_warp;
     for (;;) {
         if (threadIdx.x == 0) s_tile = atomicAdd(A.tile_counter, 1u);
         __syncthreads();
@@ -428,15 +438,18 @@ __global__ void __launch_bounds__(kFineThreads, 4) k_fine(const FrameParams* __r
         const uint32_t lt = tile - P.fine_tile_base[f];
         const uint32_t v = P.fview[f];
         const uint32_t g_end = P.view_strand0[v] + P.view_strands[v];
-        const uint32_t g0 = P.view_strand0[v] + lt * kFineStrandsPerTile + (uint32_t)warp * kFineStrandsPerWarp;
+        const uint32_t g0 = P.view_strand0[v] + (lt * kFineWarps + (uint32_t)warp) * per_warp;
+        // Lane k looks up the warp's strand k, once for both passes.
+        FineStrand own{0u, 0u, 0u, 0u, 0u, 0u, true};
+        if (lane < (int)per_warp) own = fine_strand(P, inst, A, f, g0 + lane, g_end);
+        if (!own.ordered) A.counters->seg_unordered = 1u;
+        // FRUSTUM_TELEMETRY_RETAINED_STRANDS (:1085): every strand the keep
+        // tests pass.
+        if (A.tel && own.nseg > 0u) atomicAdd(tel_frustum(A.tel, f, kTelRetainedStrands), 1u);
         // Pass A: count the clipped segments of the warp's strands.
         uint32_t count = 0;
-        for (uint32_t k = 0; k < kFineStrandsPerWarp; ++k) {
-            const FineStrand fs = fine_strand(P, inst, A, f, g0 + k, g_end);
-            if (!fs.ordered) A.counters->seg_unordered = 1u;
-            // FRUSTUM_TELEMETRY_RETAINED_STRANDS (:1085): every strand the
-            // keep tests pass.
-            if (A.tel && lane == 0 && fs.nseg > 0u) atomicAdd(tel_frustum(A.tel, f, kTelRetainedStrands), 1u);
+        for (uint32_t k = 0; k < per_warp; ++k) {
+            const FineStrand fs = own.of_lane((int)k);
             for (uint32_t c = 0; c < fs.nseg; c += kFineChunk) {
                 SegOut o;
                 const bool ok = fine_chunk(P, inst[fs.i], f, fs.meta_offset, fs.nseg, c, lane, o);
@@ -463,8 +476,8 @@ __global__ void __launch_bounds__(kFineThreads, 4) k_fine(const FrameParams* __r
         uint32_t out = s_base;
         for (int w = 0; w < warp; ++w) out += s_warp_count[w];
         // Pass B: project again and write in segment order.
-        for (uint32_t k = 0; k < kFineStrandsPerWarp; ++k) {
-            const FineStrand fs = fine_strand(P, inst, A, f, g0 + k, g_end);
+        for (uint32_t k = 0; k < per_warp; ++k) {
+            const FineStrand fs = own.of_lane((int)k);
             for (uint32_t c = 0; c < fs.nseg; c += kFineChunk) {
                 SegOut o;
                 const bool ok = fine_chunk(P, inst[fs.i], f, fs.meta_offset, fs.nseg, c, lane, o);
@@ -1071,113 +1084,153 @@ __device__ __forceinline__ void page_active_tiles(const FrameParams& P, const Pr
     add_tile_work(P, A, page, A.page_meta[page].coarse_tile_id, lt, work);
 }
 
+// A page's cell counts as one warp holds them: lane l has cells 8 l .. 8 l + 7
+// (one fine depth slice, fine tiles 8 (l & 1) .. + 7), their sum, and how many
+// fall in each of the cell sort's size classes, 16 bits each.
+struct PageCells {
+    uint32_t c[8], sum, small_quad, mid_large;
+    __device__ __forceinline__ PageCells(const uint32_t* counts, uint32_t page, uint32_t lane) {
+        const size_t g0 = (size_t)page * kPageSize + lane * 8u;
+        const uint4 ca = *reinterpret_cast<const uint4*>(counts + g0);
+        const uint4 cb = *reinterpret_cast<const uint4*>(counts + g0 + 4u);
+        c[0] = ca.x; c[1] = ca.y; c[2] = ca.z; c[3] = ca.w;
+        c[4] = cb.x; c[5] = cb.y; c[6] = cb.z; c[7] = cb.w;
+        sum = small_quad = mid_large = 0u;
+#pragma unroll
+        for (uint32_t k = 0; k < 8u; ++k) {
+            sum += c[k];
+            if (c[k] >= 2u && c[k] <= kThreadSortMax) small_quad += 1u;
+            if (c[k] > kThreadSortMax && c[k] <= kQuadSortMax) small_quad += 1u << 16;
+            if (c[k] > kQuadSortMax && c[k] <= kGroupSortMax) mid_large += 1u;
+            if (c[k] > kGroupSortMax) mid_large += 1u << 16;
+        }
+    }
+};
+
 // csr: a page-CSR frame, where k_build_pages does this work unless the visit
-// records went unused. One warp per page, claimed in page order: lane l holds
-// cells 8 l .. 8 l + 7 (one fine depth slice, fine tiles 8 (l & 1) .. + 7), so
-// a warp scan gives the cell offsets and the look-back the page base, with no
-// block barrier.
+// records went unused. A warp per group of pages, claimed in page order: the
+// group's sums first (one look-back and one reservation of list room per
+// group), then page by page the cell offsets from a warp scan, with no block
+// barrier. A group is the pages' share of a resident warp, at most eight. Bound
+// by the latency of the look-back chain and of the list counters' atomics, which
+// a group pays once: with a page per warp it took 28 us on the tiny frame (184
+// pages), 53 on the small, 119 on the medium (23,195) and 566 on the large one
+// (133,640), now 16, 37, 59 and 262 (at most four pages: 16, 37, 70, 307).
+constexpr uint32_t kPageGroup = 8;
 __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restrict__ Pp, PrepassArgs A, bool csr) {
     if (frame_failed(A.counters)) return;
     if (csr && !visits_unused(A)) return;
     const FrameParams& P = *Pp;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t pages = *((volatile uint32_t*)&A.counters->pages);
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t per = min(kPageGroup, ceil_div(pages, warps));
     for (;;) {
-        uint32_t page = 0u;
-        if (lane == 0u) page = atomicAdd(A.tile_counter, 1u);
-        page = __shfl_sync(0xFFFFFFFFu, page, 0);
-        if (page >= pages) break;
-        const size_t g0 = (size_t)page * kPageSize + lane * 8u;
-        const uint4 ca = *reinterpret_cast<const uint4*>(A.counts + g0);
-        const uint4 cb = *reinterpret_cast<const uint4*>(A.counts + g0 + 4u);
-        const uint32_t c[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
-        uint32_t e[8], sum = 0u, nsmall = 0u, nquad = 0u, nmid = 0u, nlarge = 0u;
+        uint32_t group = 0u;
+        if (lane == 0u) group = atomicAdd(A.tile_counter, 1u);
+        group = __shfl_sync(0xFFFFFFFFu, group, 0);
+        if ((uint64_t)group * per >= pages) break;
+        const uint32_t first = group * per, end = min(first + per, pages);
+        uint32_t total = 0u, small_quad = 0u, mid_large = 0u;
 #pragma unroll
-        for (uint32_t k = 0; k < 8u; ++k) {
-            e[k] = sum;
-            sum += c[k];
-            nsmall += (c[k] >= 2u && c[k] <= kThreadSortMax) ? 1u : 0u;
-            nquad += (c[k] > kThreadSortMax && c[k] <= kQuadSortMax) ? 1u : 0u;
-            nmid += (c[k] > kQuadSortMax && c[k] <= kGroupSortMax) ? 1u : 0u;
-            nlarge += c[k] > kGroupSortMax ? 1u : 0u;
+        for (uint32_t u = 0; u < kPageGroup; ++u) {
+            if (first + u >= end) break;
+            const PageCells pc(A.counts, first + u, lane);
+            total += pc.sum;
+            small_quad += pc.small_quad;
+            mid_large += pc.mid_large;
         }
-        // The scans carry the reference count (exclusive per cell) and, packed
-        // 16 bits each, the cell counts of the lists' size classes.
-        const uint32_t mine = nsmall | (nquad << 16), mine2 = nmid | (nlarge << 16);
-        uint32_t x = sum, y = mine, z = mine2;
-#pragma unroll
-        for (uint32_t o = 1; o < 32u; o <<= 1) {
-            const uint32_t xa = __shfl_up_sync(0xFFFFFFFFu, x, o), ya = __shfl_up_sync(0xFFFFFFFFu, y, o);
-            const uint32_t za = __shfl_up_sync(0xFFFFFFFFu, z, o);
-            if (lane >= o) { x += xa; y += ya; z += za; }
-        }
-        const uint32_t total = __shfl_sync(0xFFFFFFFFu, x, 31), both = __shfl_sync(0xFFFFFFFFu, y, 31);
-        const uint32_t both2 = __shfl_sync(0xFFFFFFFFu, z, 31);
-        const uint32_t lane_base = x - sum, list_base = y - mine, list_base2 = z - mine2;
-#pragma unroll
-        for (uint32_t k = 0; k < 8u; ++k) e[k] += lane_base;
-        *reinterpret_cast<uint4*>(A.offsets + g0) = make_uint4(e[0], e[1], e[2], e[3]);
-        *reinterpret_cast<uint4*>(A.offsets + g0 + 4u) = make_uint4(e[4], e[5], e[6], e[7]);
-        const uint32_t base = lb_exclusive_warp(A.lb_status, page, P.epoch, total, &A.counters->error, lb_limit(P),
-                                              lb_withheld(P, kStagePrefix));
-        uint32_t flags = 0u, tile = 0u;
-        if (lane == 0u) {
-            fiber_fine_page_meta pm = A.page_meta[page];
-            if (total > 0u && (uint64_t)base + total > (uint64_t)P.ref_capacity) {
-                flags = 1u;
-                atomicOr(&A.counters->overflow, 4u);
-            }
-            pm.seg_ref_base = total > 0u ? base : 0u;
-            pm.seg_ref_count = flags ? 0u : total;
-            pm.flags = flags;
-            A.page_meta[page] = pm;
-            tile = pm.coarse_tile_id;
-            if (page == pages - 1u) A.counters->refs = base + total;
-        }
-        flags = __shfl_sync(0xFFFFFFFFu, flags, 0);
-        // Each cell's first reference, for the fill.
-        const uint32_t lost = flags ? kInvalid : 0u;
-        *reinterpret_cast<uint4*>(A.cursors + g0) =
-            make_uint4((base + e[0]) | lost, (base + e[1]) | lost, (base + e[2]) | lost, (base + e[3]) | lost);
-        *reinterpret_cast<uint4*>(A.cursors + g0 + 4u) =
-            make_uint4((base + e[4]) | lost, (base + e[5]) | lost, (base + e[6]) | lost, (base + e[7]) | lost);
-        // A page that lost its references lists no cells and no work.
-        if (flags != 0u) {
-            if (lane < 16u) A.page_items[(size_t)page * 16u + lane] = 0u;
-            continue;
-        }
-        // The page's cells for k_sort_cells, in cell order: 2..8 references in
-        // the small list, 9..16 in the quad one, 17..32 in the middle one, more in
-        // the large one (a single reference is in order). Lanes 0..3 reserve the
-        // lists' room at once.
+        total = __reduce_add_sync(0xFFFFFFFFu, total);
+        small_quad = __reduce_add_sync(0xFFFFFFFFu, small_quad);  // at most 8 x 256 per class
+        mid_large = __reduce_add_sync(0xFFFFFFFFu, mid_large);
+        uint32_t base = lb_exclusive_warp(A.lb_status, group, P.epoch, total, &A.counters->error, lb_limit(P),
+                                          lb_withheld(P, kStagePrefix));
+        if (lane == 0u && end == pages) A.counters->refs = base + total;
+        // Room in the cell sort's lists (lane = class), for the whole group
+        // unless some of its pages may lose their references.
+        const bool tight = (uint64_t)base + total > (uint64_t)P.ref_capacity;
         uint32_t room = 0u;
-        if (lane < 4u) {
-            const uint32_t w = lane < 2u ? both : both2, want = lane & 1u ? w >> 16 : w & 0xFFFFu;
-            if (want) room = atomicAdd(&A.counters->list_cells[lane], want);
-        }
-        uint32_t ks = __shfl_sync(0xFFFFFFFFu, room, 0) + (list_base & 0xFFFFu);
-        uint32_t kq = __shfl_sync(0xFFFFFFFFu, room, 1) + (list_base >> 16);
-        uint32_t km = __shfl_sync(0xFFFFFFFFu, room, 2) + (list_base2 & 0xFFFFu);
-        uint32_t kl = __shfl_sync(0xFFFFFFFFu, room, 3) + (list_base2 >> 16);
+        auto reserve = [&](uint32_t sq, uint32_t ml) {
+            const uint32_t w = lane < 2u ? sq : ml, want = lane & 1u ? w >> 16 : w & 0xFFFFu;
+            if (lane < 4u && want) room = atomicAdd(&A.counters->list_cells[lane], want);
+        };
+        if (!tight) reserve(small_quad, mid_large);
+#pragma unroll 1
+        for (uint32_t page = first; page < end; ++page) {
+            const PageCells pc(A.counts, page, lane);
+            uint32_t x = pc.sum, y = pc.small_quad, z = pc.mid_large;
 #pragma unroll
-        for (uint32_t k = 0; k < 8u; ++k) {
-            const uint2 cell = make_uint2(base + e[k], c[k]);
-            if (c[k] >= 2u && c[k] <= kThreadSortMax) A.cells_small[ks++] = cell;
-            else if (c[k] > kThreadSortMax && c[k] <= kQuadSortMax) A.cells_quad[kq++] = cell;
-            else if (c[k] > kQuadSortMax && c[k] <= kGroupSortMax) A.cells_mid[km++] = cell;
-            else if (c[k] > kGroupSortMax) A.cells_large[kl++] = cell;
-        }
-        // append_active_fine_tile (:2207-2238): each of the page's 16 fine tiles
-        // that lies on screen gets its non-empty cells, the tile's work items of
-        // this page. Fine tile 8 p + k is register k of the lanes of parity p.
-        uint32_t work = 0u;
+            for (uint32_t o = 1; o < 32u; o <<= 1) {
+                const uint32_t xa = __shfl_up_sync(0xFFFFFFFFu, x, o), ya = __shfl_up_sync(0xFFFFFFFFu, y, o);
+                const uint32_t za = __shfl_up_sync(0xFFFFFFFFu, z, o);
+                if (lane >= o) { x += xa; y += ya; z += za; }
+            }
+            const uint32_t refs = __shfl_sync(0xFFFFFFFFu, x, 31), sq = __shfl_sync(0xFFFFFFFFu, y, 31);
+            const uint32_t ml = __shfl_sync(0xFFFFFFFFu, z, 31);
+            uint32_t e[8];  // exclusive offsets inside the page
+            e[0] = x - pc.sum;
 #pragma unroll
-        for (uint32_t k = 0; k < 8u; ++k) {
-            const uint32_t nonempty = __ballot_sync(0xFFFFFFFFu, c[k] > 0u);
-            if (k == (lane & 7u)) work = (uint32_t)__popc(nonempty & ((lane & 8u) ? 0xAAAAAAAAu : 0x55555555u));
+            for (uint32_t k = 1; k < 8u; ++k) e[k] = e[k - 1] + pc.c[k - 1];
+            const size_t g0 = (size_t)page * kPageSize + lane * 8u;
+            *reinterpret_cast<uint4*>(A.offsets + g0) = make_uint4(e[0], e[1], e[2], e[3]);
+            *reinterpret_cast<uint4*>(A.offsets + g0 + 4u) = make_uint4(e[4], e[5], e[6], e[7]);
+            const uint32_t page_base = base;
+            base += refs;
+            const bool fits = refs == 0u || (uint64_t)page_base + refs <= (uint64_t)P.ref_capacity;
+            // seg_ref_base, seg_ref_count; coarse_tile_id, coarse_z, -, flags
+            uint4* meta = reinterpret_cast<uint4*>(A.page_meta + page);
+            uint4 m = meta[1];
+            __syncwarp();
+            if (lane == 0u) {
+                if (!fits) atomicOr(&A.counters->overflow, 4u);
+                meta[0] = make_uint4(refs > 0u ? page_base : 0u, fits ? refs : 0u, 0u, 0u);
+                m.w = fits ? 0u : 1u;
+                meta[1] = m;
+            }
+            // Each cell's first reference, for the fill.
+            const uint32_t lost = fits ? 0u : kInvalid;
+#pragma unroll
+            for (uint32_t k = 0; k < 8u; ++k) e[k] += page_base;
+            *reinterpret_cast<uint4*>(A.cursors + g0) = make_uint4(e[0] | lost, e[1] | lost, e[2] | lost, e[3] | lost);
+            *reinterpret_cast<uint4*>(A.cursors + g0 + 4u) = make_uint4(e[4] | lost, e[5] | lost, e[6] | lost, e[7] | lost);
+            // A page that lost its references lists no cells and no work.
+            if (!fits) {
+                if (lane < 16u) A.page_items[(size_t)page * 16u + lane] = 0u;
+                continue;
+            }
+            if (tight) reserve(sq, ml);
+            // The page's cells for k_sort_cells, in cell order: 2..8 references
+            // in the small list, 9..16 in the quad one, 17..32 in the middle one,
+            // more in the large one (a single reference is in order).
+            uint32_t ks = __shfl_sync(0xFFFFFFFFu, room, 0) + ((y - pc.small_quad) & 0xFFFFu);
+            uint32_t kq = __shfl_sync(0xFFFFFFFFu, room, 1) + ((y - pc.small_quad) >> 16);
+            uint32_t km = __shfl_sync(0xFFFFFFFFu, room, 2) + ((z - pc.mid_large) & 0xFFFFu);
+            uint32_t kl = __shfl_sync(0xFFFFFFFFu, room, 3) + ((z - pc.mid_large) >> 16);
+#pragma unroll
+            for (uint32_t k = 0; k < 8u; ++k) {
+                const uint32_t n = pc.c[k];
+                const uint2 cell = make_uint2(e[k], n);
+                if (n >= 2u && n <= kThreadSortMax) A.cells_small[ks++] = cell;
+                else if (n > kThreadSortMax && n <= kQuadSortMax) A.cells_quad[kq++] = cell;
+                else if (n > kQuadSortMax && n <= kGroupSortMax) A.cells_mid[km++] = cell;
+                else if (n > kGroupSortMax) A.cells_large[kl++] = cell;
+            }
+            if (!tight && lane < 4u) {
+                const uint32_t w = lane < 2u ? sq : ml;
+                room += lane & 1u ? w >> 16 : w & 0xFFFFu;
+            }
+            // append_active_fine_tile (:2207-2238): each of the page's 16 fine
+            // tiles that lies on screen gets its non-empty cells, the tile's work
+            // items of this page. Fine tile 8 p + k is register k of the lanes of
+            // parity p.
+            uint32_t work = 0u;
+#pragma unroll
+            for (uint32_t k = 0; k < 8u; ++k) {
+                const uint32_t nonempty = __ballot_sync(0xFFFFFFFFu, pc.c[k] > 0u);
+                if (k == (lane & 7u)) work = (uint32_t)__popc(nonempty & ((lane & 8u) ? 0xAAAAAAAAu : 0x55555555u));
+            }
+            if (lane < 16u) add_tile_work(P, A, page, m.x, lane, work);
         }
-        tile = __shfl_sync(0xFFFFFFFFu, tile, 0);
-        if (lane < 16u) add_tile_work(P, A, page, tile, lane, work);
     }
 }
 
@@ -1913,7 +1966,7 @@ void launch_count(const LaunchCtx& L, const PrepassArgs& A) {
     else k_traverse<kCount, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
 }
 void launch_prefix(const LaunchCtx& L, const PrepassArgs& A, bool csr) {
-    k_prefix_pages<<<L.sm_count * 6, 256, 0, L.stream>>>(L.P, A, csr);
+    k_prefix_pages<<<L.sm_count * 3, 256, 0, L.stream>>>(L.P, A, csr);
 }
 void launch_page_csr_count(const LaunchCtx& L, const PrepassArgs& A) {
     k_page_count<<<L.sm_count * 8, 256, 0, L.stream>>>(A);

@@ -4,12 +4,14 @@ to 32, up to 256, more), with strands that follow one another in the index slab
 (the task index alone breaks depth-key ties) and with strands whose index
 ranges are shuffled (the full instance and segment key does), on both binning
 backends. Every dump is compared exactly."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from bevy_strand_rasterizer_b200 import abi
-from common import build_scene, run_gpu
-from test_gpu_parity import _compare
+from common import build_scene, run_gpu, run_ref
+from test_gpu_parity import _compare, _exact
 
 pytestmark = pytest.mark.gpu
 
@@ -30,3 +32,23 @@ def test_cell_order_matches_oracle(strands, points, side, shuffled, backend):
         p.close()
         assert largest > 256 or side != 64
     _compare(scene)
+
+
+@pytest.mark.parametrize("name,kw", [("tiny", {}), ("small", {}), ("small", dict(strands=20_000, width=1600, height=900))])
+def test_pages_that_lose_their_references(name, kw):
+    # A reference budget that runs out inside a group of pages: the pages kept,
+    # flagged and listed are the oracle's, and the next frame with room for all
+    # of them matches it everywhere.
+    scene = build_scene(name, settings_overrides={"ref_capacity_factor": 1}, **kw)
+    plugin, ref = run_gpu(scene), run_ref(scene)
+    assert plugin.stats(allow_overflow=True).overflow_flags & 4
+    for what in (abi.DUMP_PAGE_META, abi.DUMP_COUNTS, abi.DUMP_OFFSETS, abi.DUMP_ACTIVE_TILES, abi.DUMP_RUNS,
+                 abi.DUMP_WORK):
+        _exact(plugin.dump(what), ref.get(what), what)
+    scene.settings.ref_capacity_factor = 16
+    abi.check(plugin.lib.fiber_settings_set(plugin.ctx, C.byref(scene.settings)), "fiber_settings_set")
+    run_gpu(scene, plugin=plugin)
+    full = run_ref(scene)
+    for what in (abi.DUMP_PAGE_META, abi.DUMP_REFS, abi.DUMP_WORK, abi.DUMP_DOM_OPACITY):
+        _exact(plugin.dump(what), full.get(what), what)
+    plugin.close()
