@@ -835,7 +835,7 @@ __device__ __forceinline__ bool visits_unused(const PrepassArgs& A) {
 // kOpaque: the frame has opaque fine tiles (K0 ran); the variant without them
 // carries no cull code. kTel: count page candidates for the telemetry.
 template <bool kOpaque, bool kTel>
-__global__ void __launch_bounds__(kVisitThreads, 4) k_visit(const FrameParams* __restrict__ Pp, PrepassArgs A) {
+__global__ void __launch_bounds__(kVisitThreads, 3) k_visit(const FrameParams* __restrict__ Pp, PrepassArgs A) {
     if (frame_failed(A.counters)) return;
     const FrameParams& P = *Pp;
     __shared__ uint32_t s_buf[kVisitSlots * kVisitThreads];
@@ -1945,7 +1945,7 @@ void launch_fine(const LaunchCtx& L, const PrepassArgs& A) {
     k_fine<<<L.sm_count * 6, kFineThreads, 0, L.stream>>>(L.P, L.inst, A);
 }
 void launch_visit(const LaunchCtx& L, const PrepassArgs& A) {
-    const unsigned grid = L.sm_count * 4;  // the resident blocks (4 per SM), each looping over warps of tasks
+    const unsigned grid = L.sm_count * 3;  // the resident blocks (3 per SM), each looping over warps of tasks
     if (L.telemetry) {
         if (L.opaque) k_visit<true, true><<<grid, kVisitThreads, 0, L.stream>>>(L.P, A);
         else k_visit<false, true><<<grid, kVisitThreads, 0, L.stream>>>(L.P, A);
