@@ -31,7 +31,7 @@ const char* kSpanNames[kSpanCount] = {
     "strand_prepass/binning",              // count
     "strand_prepass/prefix_fine_pages",
     "strand_prepass/fill_segment_refs",
-    "strand_prepass/compact_active_tiles",  // what compaction and emit take beyond the fill they run beside
+    "strand_prepass/compact_active_tiles",  // beside the fill, as the emit is
     "strand_prepass/emit_raster_work",      // canonical cell order
     "strand_shadow_rasterizer/rasterize",  // incl. fused stampback
     "strand_shading/shade",
@@ -121,7 +121,7 @@ struct fiber_ctx {
     // beside the frame; ev_in = uploaded, ev_out = the last download queued.
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
-    // The prepass's active-tile compaction and emit run on this stream beside the fill.
+    // Stages beside the prepass's main chain (run_prepass).
     cudaStream_t side_stream = nullptr;
     cudaStream_t side_override = nullptr;  // fiber_ctx_set_side_stream (request server priorities)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -147,8 +147,7 @@ struct fiber_ctx {
     DevBuf d_color, d_depth, d_fragments, d_validate, d_host_scene, d_host_depth;
     int hist_cur = 0;
     // timing
-    cudaEvent_t ev[kSpanCount + 1] = {};
-    bool events_ok = false;
+    DevBuf d_stamps;  // [kStampCount_] device clock at the stages' starts and the frame's end
     cudaStream_t last_stream = nullptr;
     // graph replay of fiber_frame_fused
     cudaGraphExec_t graph = nullptr;
@@ -220,6 +219,7 @@ LaunchCtx launch_ctx(fiber_ctx* c, cudaStream_t s) {
 PrepassArgs prepass_args(fiber_ctx* c) {
     PrepassArgs A{};
     A.counters = dp<FrameCounters>(c->d_counters);
+    A.stamps = dp<unsigned long long>(c->d_stamps);
     A.range_valid = dp<uint32_t>(c->d_range_valid);
     A.ranges = dp<fiber_coarse_asset_range>(c->d_ranges);
     A.keep = dp<float>(c->d_keep);
@@ -272,6 +272,7 @@ void set_stage(fiber_ctx* c, PrepassArgs& A, uint32_t stage) {
 RenderArgs render_args(fiber_ctx* c) {
     RenderArgs R{};
     R.counters = dp<FrameCounters>(c->d_counters);
+    R.stamps = dp<unsigned long long>(c->d_stamps);
     R.tasks = dp<fiber_binning_task>(c->d_tasks);
     R.work = dp<fiber_raster_work_item>(c->d_work);
     R.runs = dp<fiber_raster_tile_run>(c->d_runs);
@@ -290,23 +291,6 @@ RenderArgs render_args(fiber_ctx* c) {
     R.fragments = dp<uint32_t>(c->d_fragments);
     R.neg_zero2 = 0x8000000080000000ull;
     return R;
-}
-
-// Span events: while a stream is being captured they are recorded as external
-// event nodes, so they keep timing the frame when it is replayed from the CUDA
-// graph; otherwise they are plain records. A failed record only disables the
-// spans; it never leaves an error behind for the node that called it.
-void record(fiber_ctx* c, int span, cudaStream_t s) {
-    if (!c->events_ok) return;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (s && cudaStreamIsCapturing(s, &cs) != cudaSuccess) cs = cudaStreamCaptureStatusNone;
-    cudaError_t e = cs == cudaStreamCaptureStatusActive
-                        ? cudaEventRecordWithFlags(c->ev[span], s, cudaEventRecordExternal)
-                        : cudaEventRecord(c->ev[span], s);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        c->events_ok = false;
-    }
 }
 
 fiber_status check_launch() {
@@ -368,52 +352,56 @@ struct OpaqueSource {
 fiber_status run_prepass(fiber_ctx* c, cudaStream_t s, const OpaqueSource* opaque = nullptr) {
     LaunchCtx L = launch_ctx(c, s);
     PrepassArgs A = prepass_args(c);
-    record(c, 0, s);
     if (opaque) {
-        launch_opaque(L, A, opaque->depth, opaque->pitch, opaque->samples, c->camera_fine_tiles);
+        launch_opaque(L, A, opaque->depth, opaque->pitch, opaque->samples, c->camera_fine_tiles, true);
         L.opaque = true;
     }
-    launch_broad(L, A);
+    launch_broad(L, A, opaque == nullptr);
     launch_lut(L, A);
-    record(c, 1, s);
     set_stage(c, A, kStageFine);
     launch_fine(L, A);
-    record(c, 2, s);
     launch_visit(L, A);
-    record(c, 3, s);
     set_stage(c, A, kStageAlloc);
     launch_alloc(L, A);
     launch_zero_pages(L, A);
     // FineBinningBackend (src/pipelines/prepass.rs:1261-1295): segment-owned
     // count / prefix / fill, or the page CSR with page-owned cell building.
+    //
+    // What the frame's main chain does not wait for runs on the side stream (a
+    // branch of the frame graph when captured): the walking passes, which only
+    // frames whose visit records did not fit use, and the active-tile compaction
+    // and the emit, which need only the prefix and run beside the fill (beside
+    // the cell sort its blocks would leave them no room).
     const bool csr = c->settings.fine_binning_backend == 1u;
-    record(c, 4, s);
+    cudaStream_t side = c->side_override ? c->side_override : c->side_stream;
+    LaunchCtx Ls = L;
+    Ls.stream = side;
+    auto fork = [&]() -> cudaError_t {
+        const cudaError_t e = cudaEventRecord(c->ev_fork, s);
+        return e != cudaSuccess ? e : cudaStreamWaitEvent(side, c->ev_fork, 0);
+    };
+    auto join = [&]() -> cudaError_t {
+        const cudaError_t e = cudaEventRecord(c->ev_join, side);
+        return e != cudaSuccess ? e : cudaStreamWaitEvent(s, c->ev_join, 0);
+    };
+    FIBER_CUDA(fork());
+    launch_count_walk(Ls, A);
     if (csr) launch_page_csr_count(L, A);
     else launch_count(L, A);
-    record(c, 5, s);
+    FIBER_CUDA(join());
     set_stage(c, A, kStagePrefix);
     launch_prefix(L, A, csr);
     if (csr) launch_build_pages(L, A);
-    // The active-tile compaction and the emit need only the counts, the fill
-    // and the cell sort only the offsets: the first two run on the side stream
-    // beside the fill (a branch of the frame graph when captured) and join
-    // before the sort, whose blocks would leave them no room.
-    cudaStream_t side = c->side_override ? c->side_override : c->side_stream;
-    FIBER_CUDA(cudaEventRecord(c->ev_fork, s));
-    FIBER_CUDA(cudaStreamWaitEvent(side, c->ev_fork, 0));
-    LaunchCtx Ls = L;
-    Ls.stream = side;
+    FIBER_CUDA(fork());
     PrepassArgs As = A;
     set_stage(c, As, kStageActive);
     launch_compact_active(Ls, As, dp<unsigned long long>(c->d_lb) + c->lb_offset[kStageEmit]);
     launch_emit(Ls, As, c->P.work_capacity);
-    FIBER_CUDA(cudaEventRecord(c->ev_join, side));
-    record(c, 6, s);
-    if (csr) launch_fill_walk(L, A);
-    else launch_fill(L, A);
-    record(c, 7, s);
-    FIBER_CUDA(cudaStreamWaitEvent(s, c->ev_join, 0));
-    record(c, 8, s);
+    launch_fill_walk(Ls, As);
+    if (!csr) launch_fill(L, A);
+    // The walking fill and the streaming one are one frame's alternatives: the
+    // sorts wait for both.
+    FIBER_CUDA(join());
     launch_sort_cells(L, A);
     launch_sort_big(L, A);
     if (L.telemetry) launch_telemetry(L, A);
@@ -421,7 +409,6 @@ fiber_status run_prepass(fiber_ctx* c, cudaStream_t s, const OpaqueSource* opaqu
 }
 
 fiber_status run_shadows(fiber_ctx* c, cudaStream_t s) {
-    record(c, 9, s);
     if (c->P.L) {
         const LaunchCtx L = launch_ctx(c, s);
         const RenderArgs R = render_args(c);
@@ -432,14 +419,12 @@ fiber_status run_shadows(fiber_ctx* c, cudaStream_t s) {
 }
 
 fiber_status run_shading(fiber_ctx* c, cudaStream_t s) {
-    record(c, 10, s);
     launch_shade(launch_ctx(c, s), render_args(c));
     c->hist_cur = 1 - c->hist_cur;  // shadow-history ping-pong flip (pipelines/shading.rs:564-566)
     return check_launch();
 }
 
 fiber_status run_raster(fiber_ctx* c, cudaStream_t s) {
-    record(c, 11, s);
     launch_raster(launch_ctx(c, s), render_args(c));
     return check_launch();
 }
@@ -465,7 +450,6 @@ fiber_status opaque_source(const fiber_ctx* c, const fiber_image* im, uint32_t s
 
 fiber_status run_composite(fiber_ctx* c, const fiber_image* scene_color, const fiber_image* scene_depth,
                            fiber_image* out, cudaStream_t s) {
-    record(c, 12, s);
     if (!scene_color || !out || !scene_color->ptr || !out->ptr) return FIBER_EINVAL;
     if (c->n_views != 1u) return FIBER_EINVAL;  // a multi-view frame has no single scene image
     if (scene_color->width != c->P.width || scene_color->height != c->P.height || out->width != c->P.width ||
@@ -484,6 +468,7 @@ fiber_status run_composite(fiber_ctx* c, const fiber_image* scene_color, const f
         (scene_depth && !aligned(scene_depth, 4u)))
         return FIBER_EINVAL;
     CompositeArgs C{};
+    C.stamps = dp<unsigned long long>(c->d_stamps);
     C.strand_color = dp<__half>(c->d_color);
     C.strand_depth = dp<float>(c->d_depth);
     C.scene_color = scene_color->ptr;
@@ -555,9 +540,6 @@ fiber_status fiber_ctx_create(int device, uint64_t hbm_budget, fiber_ctx** out) 
     c->budget = hbm_budget;
     cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
     fiber_settings_default(&c->settings);
-    c->events_ok = true;
-    for (int i = 0; i <= kSpanCount; ++i)
-        if (cudaEventCreate(&c->ev[i]) != cudaSuccess) c->events_ok = false;
     fiber_status st = FIBER_OK;
     if (cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
@@ -567,6 +549,7 @@ fiber_status fiber_ctx_create(int device, uint64_t hbm_budget, fiber_ctx** out) 
     }
     if (st == FIBER_OK) st = ensure(c, c->d_counters, sizeof(FrameCounters), true);
     if (st == FIBER_OK) st = ensure(c, c->d_validate, 64, true);
+    if (st == FIBER_OK) st = ensure(c, c->d_stamps, kStampCount_ * 8, true);
     if (st != FIBER_OK) {
         fiber_ctx_destroy(c);
         return st;
@@ -589,14 +572,12 @@ fiber_status fiber_ctx_destroy(fiber_ctx* c) {
                       &c->d_tile_work, &c->d_tile_slot, &c->d_page_items, &c->d_active_list, &c->d_work, &c->d_runs,
                       &c->d_big_cells, &c->d_dom_depth, &c->d_dom_opacity, &c->d_shadow_map, &c->d_atlas,
                       &c->d_history[0], &c->d_history[1], &c->d_color, &c->d_depth, &c->d_fragments,
-                      &c->d_validate, &c->d_host_scene, &c->d_host_depth, &c->d_visit_rec,
+                      &c->d_validate, &c->d_stamps, &c->d_host_scene, &c->d_host_depth, &c->d_visit_rec,
                       &c->d_visit_task, &c->d_visit_rank, &c->d_task_key,
                       &c->d_cells_small, &c->d_cells_quad, &c->d_cells_mid, &c->d_cells_large, &c->d_opaque, &c->d_page_nvis, &c->d_page_vbase,
                       &c->d_page_bucket, &c->d_tel, &c->d_tel_slots, &c->d_dom_page_table, &c->d_dom_pool,
                       &c->d_task_rec, &c->d_ref_task};
     for (DevBuf* b : bufs) release(c, *b);
-    for (int i = 0; i <= kSpanCount; ++i)
-        if (c->ev[i]) cudaEventDestroy(c->ev[i]);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     if (c->side_stream) cudaStreamDestroy(c->side_stream);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
@@ -1082,7 +1063,7 @@ fiber_status fiber_opaque_depth(fiber_ctx* c, const fiber_image* depth, uint32_t
     cudaSetDevice(c->device);
     cudaStream_t s = (cudaStream_t)stream;
     c->last_stream = s;
-    launch_opaque(launch_ctx(c, s), prepass_args(c), o.depth, o.pitch, o.samples, c->camera_fine_tiles);
+    launch_opaque(launch_ctx(c, s), prepass_args(c), o.depth, o.pitch, o.samples, c->camera_fine_tiles, false);
     c->opaque_frame = true;
     return check_launch();
 }
@@ -1126,7 +1107,6 @@ fiber_status fiber_composite(fiber_ctx* c, uint32_t view, const fiber_image* sce
     cudaSetDevice(c->device);
     c->last_stream = (cudaStream_t)stream;
     fiber_status st = run_composite(c, scene_color, scene_depth, out, (cudaStream_t)stream);
-    record(c, 13, (cudaStream_t)stream);
     return st;
 }
 
@@ -1150,8 +1130,7 @@ fiber_status fiber_frame_fused(fiber_ctx* c, const fiber_image* scene_color, con
         if (st == FIBER_OK) st = run_shading(c, s);
         if (st == FIBER_OK) st = run_raster(c, s);
         if (st == FIBER_OK && composite) st = run_composite(c, scene_color, scene_depth, out, s);
-        record(c, 13, s);
-        return st;
+            return st;
     }
     // Every kernel argument is stable across frames (per-frame values live in
     // the device FrameParams), so one captured graph serves every frame of the
@@ -1189,8 +1168,7 @@ fiber_status fiber_frame_fused(fiber_ctx* c, const fiber_image* scene_color, con
         if (st == FIBER_OK) st = run_shading(c, s);
         if (st == FIBER_OK) st = run_raster(c, s);
         if (st == FIBER_OK && composite) st = run_composite(c, scene_color, scene_depth, out, s);
-        record(c, 13, s);
-        cudaError_t ce = cudaStreamEndCapture(s, &g);
+            cudaError_t ce = cudaStreamEndCapture(s, &g);
         if (st != FIBER_OK || ce != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
             c->hist_cur = hist_before;
@@ -1334,7 +1312,6 @@ fiber_status fiber_ctx_enqueue_frame(fiber_ctx* c, cudaStream_t s) {
     if (st == FIBER_OK) st = run_shadows(c, s);
     if (st == FIBER_OK) st = run_shading(c, s);
     if (st == FIBER_OK) st = run_raster(c, s);
-    record(c, 13, s);
     c->hist_cur = hist_before;  // the device flips the history in k_frame_advance
     return st;
 }
@@ -1380,7 +1357,6 @@ fiber_status fiber_ctx_render_host_nodes(fiber_ctx* c, const void* scene_host, v
     if (st == FIBER_OK) st = run_shading(c, s);
     if (st == FIBER_OK) st = run_raster(c, s);
     if (st == FIBER_OK) st = run_composite(c, &scene, nullptr, &scene, s);
-    record(c, 13, s);
     if (st != FIBER_OK) return st;
     FIBER_CUDA(cudaMemcpyAsync(out_host, c->d_host_scene.p, W * H * 8, cudaMemcpyDeviceToHost, s));
     return FIBER_OK;
@@ -1633,17 +1609,24 @@ const char* fiber_span_name(uint32_t i) { return i < (uint32_t)kSpanCount ? kSpa
 
 fiber_status fiber_span_times(fiber_ctx* c, float* ms, uint32_t n) {
     if (!c || !ms) return FIBER_EINVAL;
-    if (!c->events_ok) return FIBER_ENOTREADY;
     cudaSetDevice(c->device);
     FIBER_CUDA(cudaStreamSynchronize(c->last_stream));
+    unsigned long long t[kStampCount_];
+    FIBER_CUDA(cudaMemcpy(t, c->d_stamps.p, sizeof(t), cudaMemcpyDeviceToHost));
+    // A stage that launched nothing begins (and ends) where the next one does;
+    // without a composite after it the raster ends the frame.
+    if (c->P.L == 0u) t[kStampShadow] = t[kStampShade];
+    const bool composite = t[kStampComposite] > t[kStampRaster];
+    const uint32_t begin[kSpanCount] = {kStampBroad, kStampFine,    kStampVisit, kStampAlloc, kStampCount,
+                                        kStampPrefix, kStampFill,   kStampCompact, kStampSort, kStampShadow,
+                                        kStampShade,  kStampRaster, kStampComposite, kStampBroad};
+    const uint32_t end[kSpanCount] = {kStampFine,   kStampVisit, kStampAlloc, kStampCount,  kStampPrefix,
+                                      kStampFill,   kStampSort,  kStampEmit,  kStampShadow, kStampShade,
+                                      kStampRaster, composite ? kStampComposite : kStampEnd, kStampEnd, kStampEnd};
     for (uint32_t i = 0; i < n && i < (uint32_t)kSpanCount; ++i) {
-        float t = 0.0f;
-        if (i + 1 < (uint32_t)kSpanCount) {
-            if (cudaEventElapsedTime(&t, c->ev[i], c->ev[i + 1]) != cudaSuccess) { cudaGetLastError(); t = -1.0f; }
-        } else {
-            if (cudaEventElapsedTime(&t, c->ev[0], c->ev[13]) != cudaSuccess) { cudaGetLastError(); t = -1.0f; }
-        }
-        ms[i] = t;
+        const unsigned long long b = t[begin[i]], e = t[end[i]];
+        const bool ran = b != 0u && e >= b && (i != 12u || composite);
+        ms[i] = ran ? (float)((double)(e - b) * 1e-6) : -1.0f;
     }
     return FIBER_OK;
 }

@@ -53,6 +53,7 @@ struct PrepassArgs {
     uint32_t* tile_counter;          // virtual block ids of the current look-back stage
     unsigned long long* lb_status;   // look-back status words of the current stage
     FrameCounters* counters;
+    unsigned long long* stamps;      // [kStampCount_]
     uint32_t* range_valid;           // [I * F]
     fiber_coarse_asset_range* ranges;
     float* keep;                     // [I * F]
@@ -112,6 +113,7 @@ __device__ __forceinline__ uint32_t* tel_frustum(uint32_t* tel, uint32_t f, uint
 // Device buffers of the shadow, shading, raster and composite stages.
 struct RenderArgs {
     FrameCounters* counters;
+    unsigned long long* stamps;  // [kStampCount_]
     const fiber_binning_task* tasks;
     const fiber_raster_work_item* work;
     const fiber_raster_tile_run* runs;
@@ -160,6 +162,7 @@ __device__ __forceinline__ bool dom_texel(const FrameParams& P, const RenderArgs
 }
 
 struct CompositeArgs {
+    unsigned long long* stamps;
     const __half* strand_color;
     const float* strand_depth;
     const void* scene_color;
@@ -181,15 +184,19 @@ struct LaunchCtx {
     bool telemetry;               // the prepass gathers telemetry
 };
 
+// stamp: the launch starts the prepass (and its first span).
 void launch_opaque(const LaunchCtx& L, const PrepassArgs& A, const float* depth, uint32_t pitch, uint32_t samples,
-                   uint32_t tiles);
-void launch_broad(const LaunchCtx& L, const PrepassArgs& A);
+                   uint32_t tiles, bool stamp);
+void launch_broad(const LaunchCtx& L, const PrepassArgs& A, bool stamp);
 void launch_lut(const LaunchCtx& L, const PrepassArgs& A);
 void launch_fine(const LaunchCtx& L, const PrepassArgs& A);
 void launch_visit(const LaunchCtx& L, const PrepassArgs& A);
 void launch_alloc(const LaunchCtx& L, const PrepassArgs& A);
 void launch_zero_pages(const LaunchCtx& L, const PrepassArgs& A);
+// The visit-record pass, and the walking pass of frames whose records did not
+// fit (one of the two returns at once).
 void launch_count(const LaunchCtx& L, const PrepassArgs& A);
+void launch_count_walk(const LaunchCtx& L, const PrepassArgs& A);
 void launch_prefix(const LaunchCtx& L, const PrepassArgs& A, bool csr = false);
 void launch_page_csr_count(const LaunchCtx& L, const PrepassArgs& A);
 void launch_build_pages(const LaunchCtx& L, const PrepassArgs& A);

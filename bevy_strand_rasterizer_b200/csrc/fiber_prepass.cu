@@ -32,7 +32,8 @@ namespace fiber {
 // ===========================================================================
 __global__ void __launch_bounds__(256) k_opaque_reduce(const FrameParams* __restrict__ Pp, PrepassArgs A,
                                                        const float* __restrict__ depth, uint32_t pitch,
-                                                       uint32_t samples) {
+                                                       uint32_t samples, bool stamp) {
+    if (stamp) stamp_start(A.stamps, kStampBroad);
     const fiber_frustum_desc& d = Pp->frusta[0];
     const uint32_t tx = (d.screen_width + d.froxel_size_x - 1u) / d.froxel_size_x;
     const uint32_t ty = (d.screen_height + d.froxel_size_y - 1u) / d.froxel_size_y;
@@ -92,7 +93,9 @@ __device__ CornerScan scan_corners(const float4* corners, const float* clip, flo
     return s;
 }
 
-__global__ void k_broad(const FrameParams* __restrict__ Pp, const InstanceView* __restrict__ inst, PrepassArgs A) {
+__global__ void k_broad(const FrameParams* __restrict__ Pp, const InstanceView* __restrict__ inst, PrepassArgs A,
+                        bool stamp) {
+    if (stamp) stamp_start(A.stamps, kStampBroad);
     const FrameParams& P = *Pp;
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.I) return;
@@ -417,6 +420,7 @@ __device__ __forceinline__ FineStrand fine_strand(const FrameParams& P, const In
 
 __global__ void __launch_bounds__(kFineThreads, 4) k_fine(const FrameParams* __restrict__ Pp,
                                                        const InstanceView* __restrict__ inst, PrepassArgs A) {
+    stamp_start(A.stamps, kStampFine);
     const FrameParams& P = *Pp;
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp_count[kFineWarps];
@@ -836,6 +840,7 @@ __device__ __forceinline__ bool visits_unused(const PrepassArgs& A) {
 // carries no cull code. kTel: count page candidates for the telemetry.
 template <bool kOpaque, bool kTel>
 __global__ void __launch_bounds__(kVisitThreads, 3) k_visit(const FrameParams* __restrict__ Pp, PrepassArgs A) {
+    stamp_start(A.stamps, kStampVisit);
     if (frame_failed(A.counters)) return;
     const FrameParams& P = *Pp;
     __shared__ uint32_t s_buf[kVisitSlots * kVisitThreads];
@@ -893,6 +898,7 @@ __global__ void __launch_bounds__(kVisitThreads, 3) k_visit(const FrameParams* _
 // per visit keeps the neighbouring cells of one task in one instruction (four
 // consecutive visits per lane took 0.24 ms against 0.18 on the medium frame).
 __global__ void __launch_bounds__(256) k_count_visits(PrepassArgs A) {
+    stamp_start(A.stamps, kStampCount);
     if (frame_failed(A.counters)) return;
     if (visits_unused(A)) return;
     const uint32_t n = (uint32_t)*((volatile unsigned long long*)&A.counters->visits);
@@ -916,6 +922,7 @@ __global__ void __launch_bounds__(256) k_count_visits(PrepassArgs A) {
 // fill 0.43 ms on the medium frame against 0.25); k_sort_cells puts each cell's
 // into canonical order.
 __global__ void __launch_bounds__(256) k_fill_visits(PrepassArgs A) {
+    stamp_start(A.stamps, kStampFill);
     if (frame_failed(A.counters)) return;
     if (visits_unused(A)) return;
     const uint32_t n = (uint32_t)*((volatile unsigned long long*)&A.counters->visits);
@@ -959,6 +966,7 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 4;
 
 __global__ void __launch_bounds__(kScanThreads) k_alloc_pages(const FrameParams* __restrict__ Pp, PrepassArgs A) {
+    stamp_start(A.stamps, kStampAlloc);
     if (frame_failed(A.counters)) return;
     const FrameParams& P = *Pp;
     __shared__ uint32_t s_tile, s_base;
@@ -1007,6 +1015,8 @@ __global__ void __launch_bounds__(kScanThreads) k_alloc_pages(const FrameParams*
     }
 }
 
+// The new pages' counts, over the whole grid (zeroed by the allocating blocks
+// they took 13 us more on the small frame than this kernel's launch).
 __global__ void k_zero_pages(PrepassArgs A) {
     const uint32_t pages = *((volatile uint32_t*)&A.counters->pages);
     const uint32_t n = pages * (kPageSize / 4u);
@@ -1102,7 +1112,7 @@ struct PageCells {
             if (c[k] >= 2u && c[k] <= kThreadSortMax) small_quad += 1u;
             if (c[k] > kThreadSortMax && c[k] <= kQuadSortMax) small_quad += 1u << 16;
             if (c[k] > kQuadSortMax && c[k] <= kGroupSortMax) mid_large += 1u;
-            if (c[k] > kGroupSortMax) mid_large += 1u << 16;
+            if (c[k] > kGroupSortMax && c[k] <= kWarpSortMax) mid_large += 1u << 16;
         }
     }
 };
@@ -1118,6 +1128,7 @@ struct PageCells {
 // (133,640), now 16, 37, 59 and 262 (at most four pages: 16, 37, 70, 307).
 constexpr uint32_t kPageGroup = 8;
 __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restrict__ Pp, PrepassArgs A, bool csr) {
+    stamp_start(A.stamps, kStampPrefix);
     if (frame_failed(A.counters)) return;
     if (csr && !visits_unused(A)) return;
     const FrameParams& P = *Pp;
@@ -1201,7 +1212,8 @@ __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restr
             if (tight) reserve(sq, ml);
             // The page's cells for k_sort_cells, in cell order: 2..8 references
             // in the small list, 9..16 in the quad one, 17..32 in the middle one,
-            // more in the large one (a single reference is in order).
+            // up to 256 in the large one (a single reference is in order); longer
+            // ones, few if any, are queued for k_sort_big_cells one by one.
             uint32_t ks = __shfl_sync(0xFFFFFFFFu, room, 0) + ((y - pc.small_quad) & 0xFFFFu);
             uint32_t kq = __shfl_sync(0xFFFFFFFFu, room, 1) + ((y - pc.small_quad) >> 16);
             uint32_t km = __shfl_sync(0xFFFFFFFFu, room, 2) + ((z - pc.mid_large) & 0xFFFFu);
@@ -1213,6 +1225,7 @@ __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restr
                 if (n >= 2u && n <= kThreadSortMax) A.cells_small[ks++] = cell;
                 else if (n > kThreadSortMax && n <= kQuadSortMax) A.cells_quad[kq++] = cell;
                 else if (n > kQuadSortMax && n <= kGroupSortMax) A.cells_mid[km++] = cell;
+                else if (n > kWarpSortMax) A.big_cells[atomicAdd(&A.counters->big_cells, 1u)] = cell;
                 else if (n > kGroupSortMax) A.cells_large[kl++] = cell;
             }
             if (!tight && lane < 4u) {
@@ -1241,6 +1254,7 @@ __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restr
 // ===========================================================================
 __global__ void __launch_bounds__(kScanThreads) k_compact_active(const FrameParams* __restrict__ Pp, PrepassArgs A,
                                                                 unsigned long long* lb_work) {
+    stamp_start(A.stamps, kStampCompact);
     if (frame_failed(A.counters)) return;
     const FrameParams& P = *Pp;
     __shared__ uint32_t s_tile, s_base, s_work;
@@ -1327,6 +1341,7 @@ __global__ void __launch_bounds__(kScanThreads) k_compact_active(const FramePara
 // (22.5 M); sixteen lanes per coarse tile left the dense tiles' warps behind.
 // ===========================================================================
 __global__ void __launch_bounds__(256) k_emit(PrepassArgs A, uint32_t work_capacity) {
+    stamp_start(A.stamps, kStampEmit);
     if (frame_failed(A.counters)) return;
     const uint32_t lt = threadIdx.x & 15u, half = threadIdx.x & 16u;
     const uint32_t pages = *((volatile uint32_t*)&A.counters->pages);
@@ -1517,7 +1532,7 @@ __device__ __forceinline__ void thread_sort_cell(const PrepassArgs& A, uint32_t 
         if ((uint32_t)e < n) A.ref_task[base + e] = k[e].task();
 }
 
-// A cell longer than a warp sort is queued for k_sort_big_cells.
+// A cell longer than a warp sort is queued for k_sort_big_cells (page CSR).
 __device__ __forceinline__ void queue_big_cell(const PrepassArgs& A, uint32_t b, uint32_t n, uint32_t lane) {
     if (lane == 0u) {
         const uint32_t slot = atomicAdd(&A.counters->big_cells, 1u);
@@ -1628,21 +1643,20 @@ __device__ __forceinline__ void sort_cells(const PrepassArgs& A, SortSpanSmem* s
     // Cells of more than 32: a warp per cell.
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n_large; w += warps) {
         const uint2 e = A.cells_large[w];
-        if (e.y <= kWarpSortMax) warp_sort_any<E>(A, e.x, e.y, (int)lane);
-        else queue_big_cell(A, e.x, e.y, lane);
+        warp_sort_any<E>(A, e.x, e.y, (int)lane);
     }
 }
 
 // Canonical order inside every cell, in place, after the fill, over the cell
 // lists k_prefix_pages made: a warp per 32 cells of 2..8 references (a lane per
 // cell), eight cells of 9..16 references per warp (four lanes each), four of
-// 17..32 (eight lanes each), then a warp per larger cell; a cell longer than a warp sort is queued for
-// k_sort_big_cells. Bound by the networks' 64-bit compares and selects (ALU pipe
+// 17..32 (eight lanes each), then a warp per larger cell of up to 256. Bound by the networks' 64-bit compares and selects (ALU pipe
 // 71 % busy); the key gathers hide behind them (2 % of the time). The start
 // wrote 20 B of reference, key and task per entry and sorted a word beside its
 // task by branches: 0.57 -> 0.19 ms for the medium frame, 11.8 -> 4.9 ms for
 // the large frame's 349 M references.
 __global__ void __launch_bounds__(256, 5) k_sort_cells(PrepassArgs A) {
+    stamp_start(A.stamps, kStampSort);
     if (frame_failed(A.counters)) return;
     __shared__ SortSpanSmem s_span[8];
     if (*((volatile uint32_t*)&A.counters->seg_unordered) == 0u) sort_cells<ByTask>(A, s_span + (threadIdx.x >> 5));
@@ -1664,6 +1678,7 @@ __global__ void __launch_bounds__(256, 5) k_sort_cells(PrepassArgs A) {
 // Visits per page; each visit keeps its rank inside its page. Lanes of a warp
 // that hit the same page share one atomic.
 __global__ void __launch_bounds__(256) k_page_count(PrepassArgs A) {
+    stamp_start(A.stamps, kStampCount);
     if (frame_failed(A.counters)) return;
     if (visits_unused(A)) return;
     const uint32_t n = (uint32_t)*((volatile unsigned long long*)&A.counters->visits);
@@ -1726,6 +1741,7 @@ __global__ void __launch_bounds__(256) k_page_scatter(PrepassArgs A) {
 
 // One block per page, in page order (the look-back of the page bases).
 __global__ void __launch_bounds__(256, 3) k_build_pages(const FrameParams* __restrict__ Pp, PrepassArgs A) {
+    stamp_start(A.stamps, kStampFill);
     if (frame_failed(A.counters)) return;
     if (visits_unused(A)) return;
     const FrameParams& P = *Pp;
@@ -1929,14 +1945,14 @@ __global__ void __launch_bounds__(256) k_expand_refs(const uint32_t* __restrict_
 // Launch wrappers
 // ---------------------------------------------------------------------------
 void launch_opaque(const LaunchCtx& L, const PrepassArgs& A, const float* depth, uint32_t pitch, uint32_t samples,
-                   uint32_t tiles) {
+                   uint32_t tiles, bool stamp) {
     unsigned blocks = ceil_div_host(tiles, 8);
     if (blocks > (unsigned)L.sm_count * 16u) blocks = (unsigned)L.sm_count * 16u;
     if (blocks == 0u) blocks = 1u;
-    k_opaque_reduce<<<blocks, 256, 0, L.stream>>>(L.P, A, depth, pitch, samples);
+    k_opaque_reduce<<<blocks, 256, 0, L.stream>>>(L.P, A, depth, pitch, samples, stamp);
 }
-void launch_broad(const LaunchCtx& L, const PrepassArgs& A) {
-    k_broad<<<ceil_div_host(L.I, 64), 64, 0, L.stream>>>(L.P, L.inst, A);
+void launch_broad(const LaunchCtx& L, const PrepassArgs& A, bool stamp) {
+    k_broad<<<ceil_div_host(L.I, 64), 64, 0, L.stream>>>(L.P, L.inst, A, stamp);
 }
 void launch_lut(const LaunchCtx& L, const PrepassArgs& A) {
     if (L.total_coarse_tiles) k_lut<<<ceil_div_host(L.total_coarse_tiles, 128), 128, 0, L.stream>>>(L.P, A);
@@ -1962,6 +1978,8 @@ void launch_zero_pages(const LaunchCtx& L, const PrepassArgs& A) {
 }
 void launch_count(const LaunchCtx& L, const PrepassArgs& A) {
     k_count_visits<<<L.sm_count * 8, 256, 0, L.stream>>>(A);
+}
+void launch_count_walk(const LaunchCtx& L, const PrepassArgs& A) {
     if (L.opaque) k_traverse<kCount, true><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
     else k_traverse<kCount, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
 }
@@ -1970,8 +1988,6 @@ void launch_prefix(const LaunchCtx& L, const PrepassArgs& A, bool csr) {
 }
 void launch_page_csr_count(const LaunchCtx& L, const PrepassArgs& A) {
     k_page_count<<<L.sm_count * 8, 256, 0, L.stream>>>(A);
-    if (L.opaque) k_traverse<kCount, true><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
-    else k_traverse<kCount, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
     k_page_scan<<<1, 1024, 0, L.stream>>>(A);
     k_page_scatter<<<L.sm_count * 8, 256, 0, L.stream>>>(A);
 }
@@ -1984,8 +2000,6 @@ void launch_fill_walk(const LaunchCtx& L, const PrepassArgs& A) {
 }
 void launch_fill(const LaunchCtx& L, const PrepassArgs& A) {
     k_fill_visits<<<L.sm_count * 8, 256, 0, L.stream>>>(A);
-    if (L.opaque) k_traverse<kFill, true><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
-    else k_traverse<kFill, false><<<L.sm_count * 8, 256, 0, L.stream>>>(L.P, A);
 }
 void launch_compact_active(const LaunchCtx& L, const PrepassArgs& A, unsigned long long* lb_work) {
     k_compact_active<<<L.sm_count * 4, kScanThreads, 0, L.stream>>>(L.P, A, lb_work);

@@ -393,6 +393,7 @@ __device__ __forceinline__ void shadow_coverage2(Mul2 mul2, const float4* e0, co
 
 __global__ void __launch_bounds__(kTileThreads, 12) k_shadow(const FrameParams* __restrict__ Pp,
                                                             const InstanceView* __restrict__ inst, RenderArgs R) {
+    stamp_start(R.stamps, kStampShadow);
     if (frame_failed(R.counters)) return;
     const FrameParams& P = *Pp;
     // Per staged entry: (ax, ay, bx, by), (z0, z1, |ab|^2, its reciprocal),
@@ -797,6 +798,7 @@ __device__ __forceinline__ bool cam_covered(const CamPoint& p) {
 
 __global__ void __launch_bounds__(kTileThreads, 12) k_raster(const FrameParams* __restrict__ Pp,
                                                             const InstanceView* __restrict__ inst, RenderArgs R) {
+    stamp_start(R.stamps, kStampRaster);
     if (frame_failed(R.counters)) return;
     const FrameParams& P = *Pp;
     // Per staged entry: (ax, ay, bx, by), (depths, then |w| of both end points,
@@ -1011,6 +1013,7 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_raster(const FrameParams* 
             if (P.fragment_counts) R.fragments[pi] = frags;
         }
     }
+    if (threadIdx.x == 0) stamp_end(R.stamps);
 }
 
 void launch_shadow(const LaunchCtx& L, const RenderArgs& R, uint32_t K) {

@@ -297,6 +297,7 @@ __device__ F3 marschner(F3 L, F3 V, F3 U, const fiber_strand_material& m, float 
 // third of the issue slots waited for instructions: 0.375 ms).
 __global__ void __launch_bounds__(128, 8) k_shade(const FrameParams* __restrict__ Pp,
                                                const InstanceView* __restrict__ inst, RenderArgs R) {
+    stamp_start(R.stamps, kStampShade);
     if (frame_failed(R.counters)) return;
     const FrameParams& P = *Pp;
     __shared__ QuadTable s_quad;
@@ -388,6 +389,7 @@ __device__ __forceinline__ void store_px(void* base, uint32_t pitch, uint32_t fm
 }
 
 __global__ void k_composite(CompositeArgs C) {
+    stamp_start(C.stamps, kStampComposite);
     const uint32_t n = C.width * C.height;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t x = i % C.width, y = i / C.width;
@@ -404,6 +406,7 @@ __global__ void k_composite(CompositeArgs C) {
                                frag.z * frag.w + dst.z * oma, frag.w * 1.0f + dst.w * oma);
         store_px(C.out, C.out_pitch, C.out_format, x, y, o);
     }
+    if (threadIdx.x == 0) stamp_end(C.stamps);
 }
 
 void launch_shade(const LaunchCtx& L, const RenderArgs& R) {
