@@ -110,7 +110,7 @@ struct fiber_ctx {
     DevBuf d_params, d_inst, d_counters, d_lb, d_range_valid, d_ranges, d_keep, d_inst_visible, d_inst_keep;
     DevBuf d_lut_tree;  // per coarse tile: the slice lookup's search tree (kLutTreeWords)
     DevBuf d_lut, d_tasks, d_projected, d_page_table, d_page_meta, d_counts, d_offsets, d_cursors;
-    DevBuf d_tile_work, d_tile_slot, d_page_items, d_active_list, d_work, d_runs, d_big_cells;
+    DevBuf d_tile_work, d_tile_slot, d_page_items, d_heavy_list, d_active_list, d_work, d_runs, d_big_cells;
     DevBuf d_visit_rec, d_visit_task, d_visit_rank, d_task_key, d_cells_small, d_cells_quad, d_cells_mid, d_cells_large;
     DevBuf d_opaque;  // (covered, farthest depth q) per camera fine tile
     DevBuf d_task_rec, d_ref_task;  // the rasters' record of each task; each reference's task
@@ -238,6 +238,8 @@ PrepassArgs prepass_args(fiber_ctx* c) {
     A.tile_slot = dp<uint2>(c->d_tile_slot);
     A.page_items = dp<uint8_t>(c->d_page_items);
     A.active_list = dp<uint32_t>(c->d_active_list);
+    A.heavy_list = dp<uint32_t>(c->d_heavy_list);
+    A.shadow_blocks = (uint32_t)c->sm_count * 12u;
     A.work = dp<fiber_raster_work_item>(c->d_work);
     A.runs = dp<fiber_raster_tile_run>(c->d_runs);
     A.big_cells = dp<uint2>(c->d_big_cells);
@@ -276,6 +278,8 @@ RenderArgs render_args(fiber_ctx* c) {
     R.tasks = dp<fiber_binning_task>(c->d_tasks);
     R.work = dp<fiber_raster_work_item>(c->d_work);
     R.runs = dp<fiber_raster_tile_run>(c->d_runs);
+    R.heavy_list = dp<uint32_t>(c->d_heavy_list);
+    R.shadow_blocks = (uint32_t)c->sm_count * 12u;
     R.ref_task = dp<uint32_t>(c->d_ref_task);
     R.task_rec = dp<float4>(c->d_task_rec);
     R.dom_depth = dp<float>(c->d_dom_depth);
@@ -413,7 +417,16 @@ fiber_status run_shadows(fiber_ctx* c, cudaStream_t s) {
         const LaunchCtx L = launch_ctx(c, s);
         const RenderArgs R = render_args(c);
         if (c->P.dom_pool_pages) launch_dom_paging(L, R, c->P.L * c->P.dom_pages_x * c->P.dom_pages_x);
+        // The heavy runs on the side stream, beside the light ones.
+        cudaStream_t side = c->side_override ? c->side_override : c->side_stream;
+        LaunchCtx Ls = L;
+        Ls.stream = side;
+        FIBER_CUDA(cudaEventRecord(c->ev_fork, s));
+        FIBER_CUDA(cudaStreamWaitEvent(side, c->ev_fork, 0));
+        launch_shadow_heavy(Ls, R, c->P.K);
+        FIBER_CUDA(cudaEventRecord(c->ev_join, side));
         launch_shadow(L, R, c->P.K);
+        FIBER_CUDA(cudaStreamWaitEvent(s, c->ev_join, 0));
     }
     return check_launch();
 }
@@ -569,7 +582,7 @@ fiber_status fiber_ctx_destroy(fiber_ctx* c) {
     DevBuf* bufs[] = {&c->d_params, &c->d_inst, &c->d_counters, &c->d_lb, &c->d_range_valid, &c->d_ranges,
                       &c->d_keep, &c->d_inst_visible, &c->d_inst_keep, &c->d_lut, &c->d_lut_tree, &c->d_tasks, &c->d_projected,
                       &c->d_page_table, &c->d_page_meta, &c->d_counts, &c->d_offsets, &c->d_cursors,
-                      &c->d_tile_work, &c->d_tile_slot, &c->d_page_items, &c->d_active_list, &c->d_work, &c->d_runs,
+                      &c->d_tile_work, &c->d_tile_slot, &c->d_page_items, &c->d_heavy_list, &c->d_active_list, &c->d_work, &c->d_runs,
                       &c->d_big_cells, &c->d_dom_depth, &c->d_dom_opacity, &c->d_shadow_map, &c->d_atlas,
                       &c->d_history[0], &c->d_history[1], &c->d_color, &c->d_depth, &c->d_fragments,
                       &c->d_validate, &c->d_stamps, &c->d_host_scene, &c->d_host_depth, &c->d_visit_rec,
@@ -955,6 +968,7 @@ static fiber_status frame_begin_views(fiber_ctx* c, const fiber_view* views, uin
     ENSURE(c->d_tile_slot, fine_tiles * sizeof(uint2), false);
     ENSURE(c->d_page_items, page_cap * 16, false);
     ENSURE(c->d_active_list, fine_tiles * 4, false);
+    ENSURE(c->d_heavy_list, fine_tiles * 4, false);
     ENSURE(c->d_work, work_cap * sizeof(fiber_raster_work_item), false);
     ENSURE(c->d_runs, fine_tiles * sizeof(fiber_raster_tile_run), false);
     ENSURE(c->d_big_cells, (ref_cap / 33 + 1) * sizeof(uint2), false);

@@ -110,12 +110,31 @@ struct FrameCounters {
     uint32_t tile_counter[8];     // virtual block ids of the look-back stages
     uint32_t visit_overflow;      // visit records unused this frame (did not fit, or disabled)
     unsigned long long visits;    // visit records appended by k_visit
+    unsigned long long shadow_refs;  // references of the lights' pages
+    uint32_t heavy_runs;          // heavy shadow runs listed
+    uint32_t pad_counters;
     uint32_t list_cells[4];       // cells listed for the cell sort, by size class (CellList)
     uint32_t opaque_bound;        // the opaque fine-tile depths of this frame are written
     uint32_t dom_pages;           // DOM pages requested this frame (sparse residency)
     uint32_t seg_unordered;       // some instance's strands do not follow one another in its index slab
 };
-static_assert(sizeof(FrameCounters) == 184 + 4 * (kMaxFrusta - 16), "FrameCounters layout");
+static_assert(sizeof(FrameCounters) == 200 + 4 * (kMaxFrusta - 16), "FrameCounters layout");
+
+// A block of the shadow raster takes a run of n references in time n, so a run
+// that is large beside the references per resident block (12 per SM) is still
+// running when the other blocks have finished. Runs of kHeavyShare of that share
+// or more are heavy: blocks of four threads per pixel render them.
+// Frames on both sides, one kernel against two: 177 runs of 10,145 references
+// 3.95 -> 2.55 ms a frame, 6,076 of 680 1.86 -> 1.45, 254 of 1,505 1.31 -> 0.95,
+// tiny (124 of 100) 0.47 -> 0.45; frames whose runs are even keep their times
+// (medium 3.86 / 3.87, large 52.5 / 52.7). At shares of 0.06, 0.125 and 0.25 the
+// medium frame took 4.15, 4.05 and 3.91 ms (four threads a pixel do the walk's
+// work at half its rate), at 1.5 the close-up 2.07 against 1.95.
+constexpr float kHeavyShare = 0.5f;
+__device__ __forceinline__ uint32_t heavy_limit(const FrameCounters* c, uint32_t shadow_blocks) {
+    const float share = (float)*((const volatile unsigned long long*)&c->shadow_refs) / (float)shadow_blocks;
+    return __float2uint_rz(fmaxf(kHeavyShare * share, 1.0f));
+}
 
 // Size classes of the cell sort's lists: 2..8, 9..16, 17..32 and more references.
 enum CellList : uint32_t { kListSmall = 0, kListQuad = 1, kListMid = 2, kListLarge = 3 };
@@ -123,7 +142,7 @@ enum CellList : uint32_t { kListSmall = 0, kListQuad = 1, kListMid = 2, kListLar
 // Look-back stages (index into FrameCounters::tile_counter and the status regions).
 enum LookbackStage : uint32_t { kStageFine = 0, kStageAlloc = 1, kStagePrefix = 2, kStageActive = 3, kStageEmit = 4, kStageCount = 5 };
 // Run counters of the rasters (blocks claim tile runs dynamically).
-constexpr uint32_t kShadowRunCounter = 5, kCameraRunCounter = 6;
+constexpr uint32_t kShadowRunCounter = 5, kCameraRunCounter = 6, kHeavyRunCounter = 7;
 
 // ---------------------------------------------------------------------------
 // Span stamps: each stage's first kernel writes the device clock (ns) when its

@@ -78,6 +78,8 @@ struct PrepassArgs {
     uint32_t* active_list;
     fiber_raster_work_item* work;
     fiber_raster_tile_run* runs;
+    uint32_t* heavy_list;            // [fine tiles] the heavy shadow runs, in no order
+    uint32_t shadow_blocks;          // resident blocks of the shadow raster
     uint2* big_cells;
     uint32_t* visit_rec;    // [ref_capacity] page-table slot << 8 | cell; the count pass rewrites it to the cell index
     uint32_t* visit_task;   // [ref_capacity] binning task of the visit
@@ -117,6 +119,8 @@ struct RenderArgs {
     const fiber_binning_task* tasks;
     const fiber_raster_work_item* work;
     const fiber_raster_tile_run* runs;
+    uint32_t* heavy_list;        // [fine tiles] the heavy shadow runs
+    uint32_t shadow_blocks;      // resident blocks of the shadow raster
     const uint32_t* ref_task;    // [refs] binning task of each reference
     const float4* task_rec;      // [tasks][kTaskRec] end points as k_fine projected them; instance, segment, material
     float* dom_depth;        // [L][D][D] (dense layers)
@@ -213,7 +217,9 @@ void launch_telemetry(const LaunchCtx& L, const PrepassArgs& A);
 void launch_expand_refs(cudaStream_t s, const uint32_t* ref_task, const float4* task_rec, uint32_t n_tasks, uint64_t n,
                         fiber_fine_seg_ref* out);
 
+// The shadow rasters of the light and of the heavy runs.
 void launch_shadow(const LaunchCtx& L, const RenderArgs& R, uint32_t K);
+void launch_shadow_heavy(const LaunchCtx& L, const RenderArgs& R, uint32_t K);
 void launch_dom_paging(const LaunchCtx& L, const RenderArgs& R, uint32_t table_entries);
 void launch_shade(const LaunchCtx& L, const RenderArgs& R);
 void launch_raster(const LaunchCtx& L, const RenderArgs& R);

@@ -1166,6 +1166,7 @@ __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restr
             if (lane < 4u && want) room = atomicAdd(&A.counters->list_cells[lane], want);
         };
         if (!tight) reserve(small_quad, mid_large);
+        uint32_t shadow = 0u;
 #pragma unroll 1
         for (uint32_t page = first; page < end; ++page) {
             const PageCells pc(A.counts, page, lane);
@@ -1243,7 +1244,9 @@ __global__ void __launch_bounds__(256) k_prefix_pages(const FrameParams* __restr
                 if (k == (lane & 7u)) work = (uint32_t)__popc(nonempty & ((lane & 8u) ? 0xAAAAAAAAu : 0x55555555u));
             }
             if (lane < 16u) add_tile_work(P, A, page, m.x, lane, work);
+            if (m.x >= P.camera_tile_end) shadow += refs;
         }
+        if (lane == 0u && shadow) atomicAdd(&A.counters->shadow_refs, (unsigned long long)shadow);
     }
 }
 
@@ -1346,6 +1349,8 @@ __global__ void __launch_bounds__(256) k_emit(PrepassArgs A, uint32_t work_capac
     const uint32_t lt = threadIdx.x & 15u, half = threadIdx.x & 16u;
     const uint32_t pages = *((volatile uint32_t*)&A.counters->pages);
     const uint32_t halves = gridDim.x * (blockDim.x >> 4);
+    const uint32_t first_shadow = *((volatile uint32_t*)&A.counters->camera_active);
+    const uint32_t limit = heavy_limit(A.counters, A.shadow_blocks);
     // Every lane of a warp takes every round.
     for (uint32_t p0 = 0; p0 < pages; p0 += halves) {
         const uint32_t page = p0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 4);
@@ -1394,7 +1399,11 @@ __global__ void __launch_bounds__(256) k_emit(PrepassArgs A, uint32_t work_capac
                 load += c[j];
             }
         }
-        if (load) atomicAdd(&A.runs[slot.x].load_score, load);
+        if (load == 0u) continue;
+        const uint32_t before = atomicAdd(&A.runs[slot.x].load_score, load);
+        // The page that takes a shadow run over the limit lists it.
+        if (slot.x >= first_shadow && before < limit && before + load >= limit)
+            A.heavy_list[atomicAdd(&A.counters->heavy_runs, 1u)] = slot.x;
     }
 }
 
@@ -1793,6 +1802,8 @@ __global__ void __launch_bounds__(256, 3) k_build_pages(const FrameParams* __res
                 else warp_sort_any<ByRecord>(A, cb, cn, (int)lane);
             }
             page_active_tiles(P, A, page, s_counts);
+            if (threadIdx.x == 0 && A.page_meta[page].coarse_tile_id >= P.camera_tile_end)
+                atomicAdd(&A.counters->shadow_refs, (unsigned long long)A.page_meta[page].seg_ref_count);
         } else if (threadIdx.x < 16u) {
             A.page_items[(size_t)page * 16u + threadIdx.x] = 0u;
         }

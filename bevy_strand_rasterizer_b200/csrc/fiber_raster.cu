@@ -7,13 +7,15 @@
 // 64 slots; its 4 depth workers per pixel become the order in which one
 // thread applies the same operations). Blocks claim runs from a counter. The
 // run's references, its work items laid end to end, are taken in rounds of
-// kRound: each warp reads 32 references' task records at a time, keeps their
+// 128: each warp reads 32 references' task records at a time, keeps their
 // end points, radii and shading in shared memory and turns them into one
 // coverage-candidate bit per (pixel, entry) by a conservative band test; then
 // each pixel walks its candidates, two at a time. Block barriers happen only
-// between rounds. The blend order is the reference's: work items near to far,
-// references in groups of 4 from each item's start, (w0 over w1) over (w2 over
-// w3), early out after each item once alpha > 0.98.
+// between rounds. Shadow runs that would outlast the rest of the frame
+// (heavy_limit) take 256-thread blocks, a thread per pixel and depth worker. The
+// blend order is the reference's: work items near to far, references in groups of
+// 4 from each item's start, (w0 over w1) over (w2 over w3), early out after each
+// item once alpha > 0.98.
 //
 // Both rasters are bound by instruction issue, so the walk is written for few
 // instructions with the results of the plain binary32 formulas, bit for bit:
@@ -25,11 +27,15 @@
 namespace fiber {
 
 constexpr uint32_t kMaxRunItems = 256;  // 16 coarse z x 16 fine z cells per fine tile
-constexpr uint32_t kTileThreads = 64;   // = kPixelSlots
-constexpr uint32_t kRound = 128;        // staged references
-constexpr uint32_t kRoundWords = kRound / 32;
-constexpr uint32_t kGroupsPerWarp = kRoundWords / (kTileThreads / 32);
-static_assert(kGroupsPerWarp * (kTileThreads / 32) * 32 == kRound, "a round is whole groups of 32 per warp");
+
+// A block of kSplit threads per pixel slot, and its round of staged references.
+template <uint32_t kSplit>
+struct Tile {
+    static constexpr uint32_t threads = kPixelSlots * kSplit, warps = threads / 32;
+    static constexpr uint32_t round = kSplit == 1 ? 128 : 256, words = round / 32;
+    static constexpr uint32_t groups = words / warps;  // of 32 references, per warp
+    static_assert(groups * warps == words, "a round is whole groups of 32 per warp");
+};
 
 // ---------------------------------------------------------------------------
 // Packed binary32 pairs. The assembler contracts a packed product and a packed
@@ -88,19 +94,19 @@ __device__ __forceinline__ F2 div2_exact(Mul2 mul2, F2 a, float b0, float b1) {
 struct RunItems {
     uint32_t base[kMaxRunItems];
     uint32_t start[kMaxRunItems + 1];
-    uint32_t warp_refs[2], warp_items[2];
+    uint32_t warp_refs[8], warp_items[8];
 };
 
 // Loads the run's work items (kChecked: those of the run's frustum and tile);
 // items without references are left out. Returns their count; `total` the
 // references. All threads; ends with a block barrier.
-template <bool kChecked>
+template <bool kChecked, uint32_t kWarps>
 __device__ __forceinline__ uint32_t load_run_items(RunItems& s, const fiber_raster_work_item* __restrict__ work,
                                                    const fiber_raster_tile_run& run, uint32_t& total) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t n = min(run.work_count, kMaxRunItems);
     uint32_t items = 0u, refs = 0u;
-    for (uint32_t c = 0; c < n; c += kTileThreads) {
+    for (uint32_t c = 0; c < n; c += kWarps * 32u) {
         const uint32_t i = c + threadIdx.x;
         uint4 w = make_uint4(0u, 0u, 0u, 0u);  // seg_ref_base, seg_ref_count, frustum_id, screen_tile_id
         if (i < n) w = __ldg(reinterpret_cast<const uint4*>(work + run.work_base + i));
@@ -117,13 +123,21 @@ __device__ __forceinline__ uint32_t load_run_items(RunItems& s, const fiber_rast
             s.warp_items[warp] = (uint32_t)__popc(kept);
         }
         __syncthreads();
-        const uint32_t at = items + (warp ? s.warp_items[0] : 0u) + (uint32_t)__popc(kept & ((1u << lane) - 1u));
+        uint32_t items_before = items, refs_before = refs;
+#pragma unroll
+        for (uint32_t v = 0; v < kWarps; ++v) {
+            if (v < warp) {
+                items_before += s.warp_items[v];
+                refs_before += s.warp_refs[v];
+            }
+            items += s.warp_items[v];
+            refs += s.warp_refs[v];
+        }
+        const uint32_t at = items_before + (uint32_t)__popc(kept & ((1u << lane) - 1u));
         if (w.y != 0u) {
             s.base[at] = w.x;
-            s.start[at] = refs + (warp ? s.warp_refs[0] : 0u) + x - w.y;
+            s.start[at] = refs_before + x - w.y;
         }
-        items += s.warp_items[0] + s.warp_items[1];
-        refs += s.warp_refs[0] + s.warp_refs[1];
         __syncthreads();
     }
     if (threadIdx.x == 0) s.start[items] = refs;
@@ -150,34 +164,34 @@ __device__ __forceinline__ uint32_t item_of(const RunItems& s, uint32_t n_items,
 // The tasks of a warp's references of one round, a lane per reference, and their
 // places: run item << 2 | worker. Read before the walk of the round before, so
 // that staging a round waits for its records alone.
+template <class T>
 struct RoundTasks {
-    uint32_t task[kGroupsPerWarp], place[kGroupsPerWarp];
-};
-__device__ __forceinline__ RoundTasks fetch_tasks(const RunItems& s, uint32_t n_items, const uint32_t* __restrict__ ref_task,
-                                                  uint32_t e0, uint32_t total, uint32_t lane, uint32_t warp) {
-    RoundTasks r;
+    uint32_t task[T::groups], place[T::groups];
+    __device__ __forceinline__ RoundTasks(const RunItems& s, uint32_t n_items, const uint32_t* __restrict__ ref_task,
+                                          uint32_t e0, uint32_t total, uint32_t lane, uint32_t warp) {
 #pragma unroll
-    for (uint32_t u = 0; u < kGroupsPerWarp; ++u) {
-        const uint32_t ef = e0 + (warp + u * (kTileThreads / 32u)) * 32u;
-        r.task[u] = r.place[u] = 0u;
-        if (ef < total) {
-            const uint32_t item = item_of(s, n_items, ef, lane);
-            if (ef + lane < total) {
-                const uint32_t j = ef + lane - s.start[item];
-                r.task[u] = __ldg(ref_task + s.base[item] + j);
-                r.place[u] = (item << 2) | (j & 3u);
+        for (uint32_t u = 0; u < T::groups; ++u) {
+            const uint32_t ef = e0 + (warp + u * T::warps) * 32u;
+            task[u] = place[u] = 0u;
+            if (ef < total) {
+                const uint32_t item = item_of(s, n_items, ef, lane);
+                if (ef + lane < total) {
+                    const uint32_t j = ef + lane - s.start[item];
+                    task[u] = __ldg(ref_task + s.base[item] + j);
+                    place[u] = (item << 2) | (j & 3u);
+                }
             }
         }
     }
-    return r;
-}
+};
 // The records of those tasks (lanes without one read task 0's).
+template <class T>
 struct RoundRecords {
-    float4 a[kGroupsPerWarp], b[kGroupsPerWarp];
-    uint4 w[kGroupsPerWarp];  // instance, segment, material
-    __device__ __forceinline__ RoundRecords(const float4* __restrict__ task_rec, const RoundTasks& t) {
+    float4 a[T::groups], b[T::groups];
+    uint4 w[T::groups];  // instance, segment, material
+    __device__ __forceinline__ RoundRecords(const float4* __restrict__ task_rec, const RoundTasks<T>& t) {
 #pragma unroll
-        for (uint32_t u = 0; u < kGroupsPerWarp; ++u) {
+        for (uint32_t u = 0; u < T::groups; ++u) {
             const float4* rec = task_rec + (size_t)kTaskRec * t.task[u];
             a[u] = __ldg(rec);
             b[u] = __ldg(rec + 1);
@@ -306,15 +320,19 @@ __device__ __forceinline__ void store_candidates(uint32_t* s_pmask, uint32_t wor
     s_pmask[word * kPixelSlots + 32u + lane] = warp_transpose32((uint32_t)(bits >> 32), lane);
 }
 
-// A pixel's walk over its candidates of a round, in entry order.
+// A pixel's walk over its candidates of a round, in entry order; with kMasked
+// over those of one worker (`own`: the worker's entries of each word).
+template <bool kMasked>
 struct Walk {
     const uint32_t* mask;  // this pixel's column of the candidate words
+    const uint32_t* own;
     uint32_t words, q, m;
-    __device__ __forceinline__ Walk(const uint32_t* s_pmask, uint32_t slot, uint32_t n)
-        : mask(s_pmask + slot), words((n + 31u) >> 5), q(0u), m(0u) {}
+    __device__ __forceinline__ Walk(const uint32_t* s_pmask, uint32_t slot, uint32_t n, const uint32_t* own_ = nullptr)
+        : mask(s_pmask + slot), own(own_), words((n + 31u) >> 5), q(0u), m(0u) {}
     __device__ __forceinline__ uint32_t next() {
         while (m == 0u && q < words) {
             m = mask[q * kPixelSlots];
+            if (kMasked) m &= own[q];
             ++q;
         }
         if (m == 0u) return kInvalid;
@@ -345,8 +363,9 @@ struct Walk {
 constexpr int kMaxDomSlices = 16;
 constexpr uint32_t kShadowEntry = 3;  // float4 words of a staged entry
 
+template <uint32_t kSplit>
 size_t shadow_smem_bytes(uint32_t K) {
-    return (size_t)kRound * kShadowEntry * sizeof(float4) + (size_t)kTileThreads * 4u * K * sizeof(float);
+    return (size_t)Tile<kSplit>::round * kShadowEntry * sizeof(float4) + (size_t)kPixelSlots * 4u * K * sizeof(float);
 }
 
 // Coverage of one staged entry at pixel centre (x, y) by the plain operators (0
@@ -391,41 +410,56 @@ __device__ __forceinline__ void shadow_coverage2(Mul2 mul2, const float4* e0, co
     cov1 = (t1 < 0.0f || t1 > 1.0f) ? 0.0f : __saturatef(__fsub_rn(1.0f, c1));
 }
 
-__global__ void __launch_bounds__(kTileThreads, 12) k_shadow(const FrameParams* __restrict__ Pp,
-                                                            const InstanceView* __restrict__ inst, RenderArgs R) {
-    stamp_start(R.stamps, kStampShadow);
+// kSplit: threads per pixel. With 1 a pixel's thread takes the four workers'
+// entries in turn; with 4 each thread takes one worker's entries (its partials
+// are its own), and the pixel's nearest item is the least of its four. The
+// first renders the light runs, the second the heavy ones (k_emit lists them), side
+// by side.
+template <uint32_t kSplit>
+__global__ void __launch_bounds__(Tile<kSplit>::threads, kSplit == 1 ? 12 : 3)
+    k_shadow(const FrameParams* __restrict__ Pp, const InstanceView* __restrict__ inst, RenderArgs R) {
+    using T = Tile<kSplit>;
+    if (kSplit == 1u) stamp_start(R.stamps, kStampShadow);
     if (frame_failed(R.counters)) return;
     const FrameParams& P = *Pp;
     // Per staged entry: (ax, ay, bx, by), (z0, z1, |ab|^2, its reciprocal),
     // (rmin, rmax, opacity, run item << 16 | worker's partial offset).
     extern __shared__ float4 s_entry[];
     // [worker][K][pixel]: a warp's 32 pixels hit 32 banks whatever the slice.
-    float* s_partial = reinterpret_cast<float*>(s_entry + kRound * kShadowEntry);
+    float* s_partial = reinterpret_cast<float*>(s_entry + T::round * kShadowEntry);
     __shared__ RunItems s_items;
-    __shared__ uint32_t s_pmask[kRoundWords * kPixelSlots];  // [word][pixel] candidate bits
+    __shared__ uint32_t s_pmask[T::words * kPixelSlots];  // [word][pixel] candidate bits
+    __shared__ uint32_t s_own[kSplit == 1 ? 1 : 4 * T::words];  // [worker][word] the worker's entries
+    __shared__ uint32_t s_best[kSplit == 1 ? 1 : T::threads];   // [worker][pixel] nearest item so far
+    __shared__ float s_best_z[kSplit == 1 ? 1 : T::threads];
     __shared__ uint32_t s_run;
 
-    const uint32_t first = *((volatile uint32_t*)&R.counters->camera_active);
-    const uint32_t last = *((volatile uint32_t*)&R.counters->active_tiles);
     const uint32_t K = P.K, D = P.dom_size, S = P.shadow_map_size;
-    const uint32_t slot = threadIdx.x;
+    const uint32_t slot = threadIdx.x % kPixelSlots, worker = threadIdx.x / kPixelSlots;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    float* partial = s_partial + slot;  // partial[(w K + i) kTileThreads]
+    float* partial = s_partial + slot;  // partial[(w K + i) kPixelSlots]
+    const uint32_t* own = kSplit == 1 ? nullptr : s_own + worker * T::words;
     const float Kf = u2f(K);
     const Mul2 mul2{R.neg_zero2};
 
     // Blocks claim runs from a counter, so long runs do not pile up on one
     // block; the next claim is in flight while a run is rendered.
+    const uint32_t first = *((volatile uint32_t*)&R.counters->camera_active);
+    const uint32_t n_runs = kSplit == 1 ? *((volatile uint32_t*)&R.counters->active_tiles) - first
+                                        : *((volatile uint32_t*)&R.counters->heavy_runs);
+    const uint32_t limit = heavy_limit(R.counters, R.shadow_blocks);
+    uint32_t* counter = &R.counters->tile_counter[kSplit == 1 ? kShadowRunCounter : kHeavyRunCounter];
     uint32_t claim = 0u;
-    if (threadIdx.x == 0) claim = atomicAdd(&R.counters->tile_counter[kShadowRunCounter], 1u);
+    if (threadIdx.x == 0) claim = atomicAdd(counter, 1u);
     for (;;) {
         __syncthreads();
-        if (threadIdx.x == 0) s_run = first + claim;
+        if (threadIdx.x == 0) s_run = claim;
         __syncthreads();
         const uint32_t r = s_run;
-        if (r >= last) break;
-        if (threadIdx.x == 0) claim = atomicAdd(&R.counters->tile_counter[kShadowRunCounter], 1u);
-        const fiber_raster_tile_run run = R.runs[r];
+        if (r >= n_runs) break;
+        if (threadIdx.x == 0) claim = atomicAdd(counter, 1u);
+        const fiber_raster_tile_run run = R.runs[kSplit == 1 ? first + r : R.heavy_list[r]];
+        if (kSplit == 1u && run.load_score >= limit) continue;  // the other kernel's
         const uint32_t f = run.frustum_id;
         const uint32_t layer = light_layer(P, f);
         if (run.work_count == 0u || layer == kInvalid) continue;
@@ -439,22 +473,22 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_shadow(const FrameParams* 
         const float pfx = u2f(px) + 0.5f, pfy = u2f(py) + 0.5f;
         const F2 pf = pack2(pfx, pfy);
         uint32_t total;
-        const uint32_t n_items = load_run_items<true>(s_items, R.work, run, total);
+        const uint32_t n_items = load_run_items<true, T::warps>(s_items, R.work, run, total);
 
         // Stages references [e0, e0 + n) of the run, whose tasks are in `next`,
         // and fetches the following round's tasks: each warp takes 32 at a
         // time, a lane per reference (its record as k_fine wrote it for this
         // frustum, then its material), stores the entry and its candidate bits.
         // Returns whether every entry is regular; has a block barrier.
-        RoundTasks next = fetch_tasks(s_items, n_items, R.ref_task, 0u, total, lane, warp);
+        RoundTasks<T> next(s_items, n_items, R.ref_task, 0u, total, lane, warp);
         auto stage = [&](uint32_t e0, uint32_t n) -> bool {
             const float x0 = u2f(tx * fsx) + 0.5f, y0 = u2f(ty * fsy) + 0.5f;
             const float tile_max = fmaxf(u2f((tx + 1u) * fsx), u2f((ty + 1u) * fsy)) + 1.0f;
             bool plain = false;
-            const RoundRecords rr(R.task_rec, next);
+            const RoundRecords<T> rr(R.task_rec, next);
 #pragma unroll
-            for (uint32_t u = 0; u < kGroupsPerWarp; ++u) {
-                const uint32_t q = warp + u * (kTileThreads / 32u), s = q * 32u + lane;
+            for (uint32_t u = 0; u < T::groups; ++u) {
+                const uint32_t q = warp + u * T::warps, s = q * 32u + lane;
                 if (q * 32u >= n) break;
                 unsigned long long bits = 0ull;
                 if (s < n) {
@@ -467,7 +501,7 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_shadow(const FrameParams* 
                     // l2 = 0: t = 0 as line_t gives it.
                     s_entry[s * kShadowEntry] = ab;
                     s_entry[s * kShadowEntry + 1u] = make_float4(z0, z1, l2, l2 > 0.0f ? 1.0f / l2 : 0.0f);
-                    const uint32_t tag = (next.place[u] >> 2 << 16) | ((next.place[u] & 3u) * K * kTileThreads);
+                    const uint32_t tag = (next.place[u] >> 2 << 16) | ((next.place[u] & 3u) * K * kPixelSlots);
                     s_entry[s * kShadowEntry + 2u] = make_float4(rmin, rmax, m.absorption_color[3], __uint_as_float(tag));
                     if (regular_segment(ab, rmax)) {
                         bits = candidate_bits(ab, z0, z1, rmin, rmax, tile_max, x0, y0, fsx, fsy, CellBox{0, 63, 0, 63});
@@ -478,8 +512,15 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_shadow(const FrameParams* 
                 }
                 __syncwarp();
                 store_candidates(s_pmask, q, bits, lane);
+                if (kSplit != 1u) {
+#pragma unroll
+                    for (uint32_t w = 0; w < 4u; ++w) {
+                        const uint32_t of_w = __ballot_sync(0xFFFFFFFFu, s < n && (next.place[u] & 3u) == w);
+                        if (lane == 0u) s_own[w * T::words + q] = of_w;
+                    }
+                }
             }
-            next = fetch_tasks(s_items, n_items, R.ref_task, e0 + kRound, total, lane, warp);
+            next = RoundTasks<T>(s_items, n_items, R.ref_task, e0 + T::round, total, lane, warp);
             return !__syncthreads_or(plain);
         };
 
@@ -491,12 +532,12 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_shadow(const FrameParams* 
         bool complete = !active;   // the best item is fully processed
         bool regular = true;       // of the round that is staged
         uint32_t e0 = 0u, staged = kInvalid;
-        for (; e0 < total; e0 += kRound) {
-            const uint32_t n = min(kRound, total - e0);
+        for (; e0 < total; e0 += T::round) {
+            const uint32_t n = min(T::round, total - e0);
             regular = stage(e0, n);
             staged = e0;
             if (!complete) {
-                Walk walk(s_pmask, slot, n);
+                Walk<kSplit != 1u> walk(s_pmask, slot, n, own);
                 for (;;) {
                     const uint32_t bi = walk.next();
                     if (bi == kInvalid) break;
@@ -509,21 +550,50 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_shadow(const FrameParams* 
                         z0 = wmax(z0, qz);
                     }
                 }
-                complete = best != kInvalid && s_items.start[best + 1u] <= e0 + n;
             }
+            uint32_t nearest = best;
+            if (kSplit != 1u) {
+                s_best[threadIdx.x] = best;
+                __syncthreads();
+#pragma unroll
+                for (uint32_t w = 0; w < kSplit; ++w) nearest = min(nearest, s_best[w * kPixelSlots + slot]);
+            }
+            complete = !active || (nearest != kInvalid && s_items.start[nearest + 1u] <= e0 + n);
             if (__syncthreads_and(complete)) break;
+        }
+        if (kSplit != 1u) {
+            // The pixel's: the nearest of its workers' items, and the depth of
+            // those that found it.
+            s_best[threadIdx.x] = best;
+            s_best_z[threadIdx.x] = z0;
+            __syncthreads();
+#pragma unroll
+            for (uint32_t w = 0; w < kSplit; ++w) {
+                const uint32_t b = s_best[w * kPixelSlots + slot];
+                const float z = s_best_z[w * kPixelSlots + slot];
+                if (b < best) {
+                    best = b;
+                    z0 = z;
+                } else if (b == best) {
+                    z0 = wmax(z0, z);
+                }
+            }
         }
         const bool found = active && best != kInvalid;
 
         // ---- Pass 2: opacity partials, each covered entry into its worker's.
-        for (uint32_t i = 0; i < 4u * K; ++i) partial[i * kTileThreads] = 0.0f;
+        if (kSplit == 1u) {
+            for (uint32_t i = 0; i < 4u * K; ++i) partial[i * kPixelSlots] = 0.0f;
+        } else {
+            for (uint32_t i = 0; i < K; ++i) partial[(worker * K + i) * kPixelSlots] = 0.0f;
+        }
         const float alpha_z0 = found ? z0 : 1.0f;
         const float inv_span = 1.0f / wmax(1e-6f, alpha_z0);
         if (__syncthreads_or(found)) {
             // Pass 1 that stopped after the first round left it staged.
-            if (staged != 0u) next = fetch_tasks(s_items, n_items, R.ref_task, 0u, total, lane, warp);
-            for (e0 = 0u; e0 < total; e0 += kRound) {
-                const uint32_t n = min(kRound, total - e0);
+            if (staged != 0u) next = RoundTasks<T>(s_items, n_items, R.ref_task, 0u, total, lane, warp);
+            for (e0 = 0u; e0 < total; e0 += T::round) {
+                const uint32_t n = min(T::round, total - e0);
                 if (e0 != 0u || staged != 0u) regular = stage(e0, n);
                 if (found) {
                     // The entry's slice and weight, then its deposits: the
@@ -537,15 +607,15 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_shadow(const FrameParams* 
                         const float wf = __fsub_rn(tl, __fsub_rn(fl, 8388608.0f));
                         const uint32_t si = min(__float_as_uint(fl) & 31u, K - 1u);
                         const float al = __fmul_rn(__fmul_rn(cov, c.x), 0.5f);
-                        float* pw = partial + ((__float_as_uint(c.y) & 0xFFFFu) + si * kTileThreads);
+                        float* pw = partial + ((__float_as_uint(c.y) & 0xFFFFu) + si * kPixelSlots);
                         const float a0 = pw[0];
                         pw[0] = __saturatef(a0 + (1.0f - a0) * (1.0f - wf) * al);
                         if (si + 1u < K) {
-                            const float a1 = pw[kTileThreads];
-                            pw[kTileThreads] = __saturatef(a1 + (1.0f - a1) * wf * al);
+                            const float a1 = pw[kPixelSlots];
+                            pw[kPixelSlots] = __saturatef(a1 + (1.0f - a1) * wf * al);
                         }
                     };
-                    Walk walk(s_pmask, slot, n);
+                    Walk<kSplit != 1u> walk(s_pmask, slot, n, own);
                     if (regular) {
                         // Candidates two at a time: both coverages side by side,
                         // the deposits in entry order.
@@ -576,7 +646,7 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_shadow(const FrameParams* 
             }
         }
         // ---- Combine the 4 workers per slice, write the DOM, stamp the shadow map.
-        if (active) {
+        if (active && worker == 0u) {
             // A texel of a page the sparse pool could not hold is not stored
             // (counted as a DOM pool overflow); the stampback still runs.
             // Dense layers index the texel directly; the sparse pool goes
@@ -601,7 +671,7 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_shadow(const FrameParams* 
                 float acc = 0.0f;
                 for (uint32_t i = 0; i < K; ++i) {
                     float a = 0.0f;
-                    for (uint32_t wk = 0; wk < 4u; ++wk) a = a + (1.0f - a) * partial[(wk * K + i) * kTileThreads];
+                    for (uint32_t wk = 0; wk < 4u; ++wk) a = a + (1.0f - a) * partial[(wk * K + i) * kPixelSlots];
                     acc = acc + (1.0f - acc) * a;  // opaque_terminal_slice = K without an opaque depth
                     if (dense) R.dom_opacity[((size_t)layer * K + i) * D * D + dom_px] = acc;
                     else if (stored) dop[i * ds] = acc;
@@ -796,17 +866,18 @@ __device__ __forceinline__ bool cam_covered(const CamPoint& p) {
     return p.t >= 0.0f && p.t <= 1.0f && p.d2 < __fmul_rn(p.rr, p.rr);
 }
 
-__global__ void __launch_bounds__(kTileThreads, 12) k_raster(const FrameParams* __restrict__ Pp,
+__global__ void __launch_bounds__(Tile<1>::threads, 12) k_raster(const FrameParams* __restrict__ Pp,
                                                             const InstanceView* __restrict__ inst, RenderArgs R) {
+    using T = Tile<1>;
     stamp_start(R.stamps, kStampRaster);
     if (frame_failed(R.counters)) return;
     const FrameParams& P = *Pp;
     // Per staged entry: (ax, ay, bx, by), (depths, then |w| of both end points,
     // at least 1e-6), (rmin, rmax, 1 / |ab|^2, visibility), the shading texels
     // of both end points; s_tag: run item << 2 | worker.
-    __shared__ float4 s_entry[kRound * kCamEntry];
-    __shared__ uint16_t s_tag[kRound];
-    __shared__ uint32_t s_pmask[kRoundWords * kPixelSlots];  // [word][pixel] candidate bits
+    __shared__ float4 s_entry[T::round * kCamEntry];
+    __shared__ uint16_t s_tag[T::round];
+    __shared__ uint32_t s_pmask[T::words * kPixelSlots];  // [word][pixel] candidate bits
     __shared__ RunItems s_items;
     __shared__ uint32_t s_run;
 
@@ -840,7 +911,7 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_raster(const FrameParams* 
         const float pcx = u2f(px) + 0.5f, pcy = u2f(py) + 0.5f;
         const F2 pc = pack2(pcx, pcy);
         uint32_t total;
-        const uint32_t n_items = load_run_items<false>(s_items, R.work, run, total);
+        const uint32_t n_items = load_run_items<false, T::warps>(s_items, R.work, run, total);
 
         Rgba fin{0ull, 0ull}, cur{0ull, 0ull}, half{0ull, 0ull};
         float gdepth = 0.0f;
@@ -895,9 +966,9 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_raster(const FrameParams* 
             gdepth = wmax(gdepth, pz);
             ++frags;
         };
-        RoundTasks next = fetch_tasks(s_items, n_items, R.ref_task, 0u, total, lane, warp);
-        for (uint32_t e0 = 0u; e0 < total; e0 += kRound) {
-            const uint32_t n = min(kRound, total - e0);
+        RoundTasks<T> next(s_items, n_items, R.ref_task, 0u, total, lane, warp);
+        for (uint32_t e0 = 0u; e0 < total; e0 += T::round) {
+            const uint32_t n = min(T::round, total - e0);
             // Stage the round, whose tasks are in `next`, and fetch the
             // following one's: each warp takes 32 references at a time, a lane
             // per reference (its record as k_fine wrote it for this frustum,
@@ -905,10 +976,10 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_raster(const FrameParams* 
             const float x0 = u2f(tx * fsx) + 0.5f, y0 = u2f(ty * fsy) + 0.5f;
             const float tile_max = fmaxf(u2f((tx + 1u) * fsx), u2f((ty + 1u) * fsy)) + 1.0f;
             bool plain = false;
-            const RoundRecords rr(R.task_rec, next);
+            const RoundRecords<T> rr(R.task_rec, next);
 #pragma unroll
-            for (uint32_t u = 0; u < kGroupsPerWarp; ++u) {
-                const uint32_t q = warp + u * (kTileThreads / 32u), s = q * 32u + lane;
+            for (uint32_t u = 0; u < T::groups; ++u) {
+                const uint32_t q = warp + u * T::warps, s = q * 32u + lane;
                 if (q * 32u >= n) break;
                 unsigned long long bits = 0ull;
                 if (s < n) {
@@ -953,10 +1024,10 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_raster(const FrameParams* 
                 __syncwarp();
                 store_candidates(s_pmask, q, bits, lane);
             }
-            next = fetch_tasks(s_items, n_items, R.ref_task, e0 + kRound, total, lane, warp);
+            next = RoundTasks<T>(s_items, n_items, R.ref_task, e0 + T::round, total, lane, warp);
             const bool regular = !__syncthreads_or(plain);
             if (!done) {
-                Walk walk(s_pmask, slot, n);
+                Walk<false> walk(s_pmask, slot, n);
                 if (regular) {
                     for (;;) {
                         const uint32_t b0 = walk.next();
@@ -1016,20 +1087,25 @@ __global__ void __launch_bounds__(kTileThreads, 12) k_raster(const FrameParams* 
     if (threadIdx.x == 0) stamp_end(R.stamps);
 }
 
-void launch_shadow(const LaunchCtx& L, const RenderArgs& R, uint32_t K) {
+template <uint32_t kSplit>
+static void launch_shadow_split(const LaunchCtx& L, const RenderArgs& R, uint32_t K) {
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    const size_t max_bytes = shadow_smem_bytes(kMaxDomSlices);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaFuncSetAttribute(k_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_bytes);
+        cudaFuncSetAttribute(k_shadow<kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)shadow_smem_bytes<kSplit>(kMaxDomSlices));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    k_shadow<<<L.sm_count * 16, kTileThreads, shadow_smem_bytes(K), L.stream>>>(L.P, L.inst, R);
+    k_shadow<kSplit><<<L.sm_count * (kSplit == 1 ? 16 : 3), Tile<kSplit>::threads, shadow_smem_bytes<kSplit>(K), L.stream>>>(
+        L.P, L.inst, R);
 }
 
+void launch_shadow(const LaunchCtx& L, const RenderArgs& R, uint32_t K) { launch_shadow_split<1>(L, R, K); }
+void launch_shadow_heavy(const LaunchCtx& L, const RenderArgs& R, uint32_t K) { launch_shadow_split<4>(L, R, K); }
+
 void launch_raster(const LaunchCtx& L, const RenderArgs& R) {
-    k_raster<<<L.sm_count * 16, kTileThreads, 0, L.stream>>>(L.P, L.inst, R);
+    k_raster<<<L.sm_count * 16, Tile<1>::threads, 0, L.stream>>>(L.P, L.inst, R);
 }
 
 }  // namespace fiber

@@ -84,6 +84,22 @@ def test_round_boundaries(strands):
     _compare(scene)
 
 
+@pytest.mark.parametrize("strands,light", [(255, 0), (256, 40), (513, 40), (6000, 1500)])
+def test_heavy_and_light_runs(strands, light):
+    # A clump of identical strands in a light tile (a heavy run, rounds of 256)
+    # beside single ones. With 6000 the limit, 1 / 3552 of the references on the
+    # 148 SMs of a B200, passes what the single ones leave in a tile: both rasters.
+    scene = build_scene("tiny", cull=False, settings_overrides=SETTINGS)
+    _camera(scene, eye=(0.0, 0.0, 0.6))
+    rng = np.random.default_rng(strands + light)
+    pos = np.zeros((strands + light, 2, 3))
+    pos[:strands] = 0.001 + rng.uniform(0.0, 0.002, (strands, 1, 3))
+    pos[strands:] = rng.uniform(-0.15, 0.15, (light, 1, 3))
+    pos[:, 1, 1] += 0.001
+    _strands(scene, pos)
+    _compare(scene)
+
+
 @pytest.mark.parametrize("scale", [1e-6, 1e13])
 def test_scene_scale(scale):
     # 1e13: clip coordinates beyond the range of the projection's shared
