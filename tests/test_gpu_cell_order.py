@@ -10,6 +10,8 @@ import numpy as np
 import pytest
 
 from bevy_strand_rasterizer_b200 import abi
+from bevy_strand_rasterizer_b200.plugin import pack_indexed_strands
+from bevy_strand_rasterizer_b200.scene import CameraSpec
 from common import build_scene, run_gpu, run_ref
 from test_gpu_parity import _compare, _exact
 
@@ -31,6 +33,27 @@ def test_cell_order_matches_oracle(strands, points, side, shuffled, backend):
         largest = int(p.dump(abi.DUMP_COUNTS).max())
         p.close()
         assert largest > 256 or side != 64
+    _compare(scene)
+
+
+@pytest.mark.parametrize("backend,n", [(0, 257), (0, 512), (0, 513), (0, 1024), (0, 1025), (1, 2048), (0, 2049), (0, 5000),
+                                       (1, 8192), (0, 8193)])
+def test_one_large_cell(n, backend):
+    # n one-segment strands inside one cell: the merge sort's sizes and their
+    # neighbours, up to the longest cell it takes and one more.
+    scene = build_scene("tiny", cull=False, settings_overrides={"fine_binning_backend": backend, "ref_capacity_factor": 64})
+    spec = CameraSpec(width=scene.camera_cfg.screen_width, height=scene.camera_cfg.screen_height, eye=(0.0, 0.0, 0.6))
+    scene.cam.clip_from_world[:] = [float(x) for x in spec.clip_from_world()]
+    scene.cam.world_position[:] = [float(x) for x in spec.eye]
+    pos = np.zeros((n, 2, 3))
+    pos[:] = 0.002 + np.random.default_rng(n).uniform(0.0, 2e-4, (n, 1, 3))
+    pos[:, 1, 1] += 1e-4
+    packed = pack_indexed_strands(pos.reshape(-1, 3).astype(np.float32), np.full(n, 2, np.uint32),
+                                  np.arange(n, dtype=np.uint32) * 2, np.arange(n * 2, dtype=np.uint32))
+    old = scene.assets[0][0]
+    packed.aabb_min, packed.aabb_max = np.minimum(packed.aabb_min, old.aabb_min), np.maximum(packed.aabb_max, old.aabb_max)
+    scene.assets[0] = (packed,) + scene.assets[0][1:]
+    assert int(run_ref(scene).get(abi.DUMP_COUNTS).max()) == n
     _compare(scene)
 
 
