@@ -419,7 +419,7 @@ template <uint32_t kSplit>
 __global__ void __launch_bounds__(Tile<kSplit>::threads, kSplit == 1 ? 12 : 3)
     k_shadow(const FrameParams* __restrict__ Pp, const InstanceView* __restrict__ inst, RenderArgs R) {
     using T = Tile<kSplit>;
-    if (kSplit == 1u) stamp_start(R.stamps, kStampShadow);
+    if (kSplit != 1u) stamp_start(R.stamps, kStampShadow);  // the heavy runs take the SMs first
     if (frame_failed(R.counters)) return;
     const FrameParams& P = *Pp;
     // Per staged entry: (ax, ay, bx, by), (z0, z1, |ab|^2, its reciprocal),
