@@ -636,6 +636,7 @@ struct FillSink {
     }
 };
 
+constexpr uint32_t kMaxCellSteps = kCoarseExtent + kCoarseExtent + kDepthSlices + 4u;  // cells of one slice's walk
 // opq: the opaque fine tiles of the camera (null when none are bound); pd:
 // the segment's clip direction (p1 - p0 and its reciprocals); (ccx, ccy): the
 // coarse tile's column and row in the frustum.
@@ -687,44 +688,47 @@ __device__ __forceinline__ void walk_page(const PrepassArgs& A, F3 p0, const Cli
                        wclamp(div_by_rcp(d0.z - zmin, zspan, zrcp), 0.0f, 0.999999f) * 16.0f};
         float l1[3] = {div_by(d1.x - ox, fsx), div_by(d1.y - oy, fsy),
                        wclamp(div_by_rcp(d1.z - zmin, zspan, zrcp), 0.0f, 0.999999f) * 16.0f};
-        int32_t f1[3], fc[3], step[3];
+        // The walk's place as one word: the cell index, x + 4, y + 4 and z + 16
+        // (in range: the field's top two bits are 01), and the steps taken, whose
+        // limit carries into bit 31. A step along an axis is one addition.
+        constexpr uint32_t kX = 1u << 10, kY = 1u << 14, kZ = 1u << 18, kStep = 1u << 26;
+        constexpr uint32_t kTop = 12u * kX + 12u * kY + 48u * kZ + (1u << 31), kIn = 4u * kX + 4u * kY + 16u * kZ;
+        uint32_t at = kIn + (32u - kMaxCellSteps) * kStep, end = kIn, move[3];
         float tm[3], dd[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            int32_t hi = a == 2 ? 15 : 3;
-            fc[a] = iclamp(f2i(floorf(l0[a])), 0, hi);
-            f1[a] = iclamp(f2i(floorf(l1[a])), 0, hi);
+            const int32_t hi = a == 2 ? 15 : 3;
+            const uint32_t unit = a == 0 ? 1u + kX : (a == 1 ? 4u + kY : 16u + kZ);
+            at += (uint32_t)iclamp(f2i(floorf(l0[a])), 0, hi) * unit;
+            end += (uint32_t)iclamp(f2i(floorf(l1[a])), 0, hi) * unit;
             float dir = l1[a] - l0[a];
-            step[a] = sgn_i32(dir);
+            const int32_t step = sgn_i32(dir);
+            move[a] = (uint32_t)step * unit + kStep;
             float sd = fabsf(dir) < 1e-6f ? 1e-6f : dir;
             const float y = rcp_exact(sd);
             dd[a] = fabsf(y);
             float fl = floorf(l0[a]);
-            tm[a] = div_by_rcp(step[a] > 0 ? (fl + 1.0f) - l0[a] : fl - l0[a], sd, y);
+            tm[a] = div_by_rcp(step > 0 ? (fl + 1.0f) - l0[a] : fl - l0[a], sd, y);
             if (fabsf(dir) < 1e-6f) tm[a] = 1e38f;
         }
-        uint32_t safety = 0;
         for (;;) {
-            if (safety > kCoarseExtent + kCoarseExtent + kDepthSlices + 3u) break;
             // A covered fine tile whose farthest opaque depth is in front of
             // this slice's nearest depth (reversed-Z: z_max) hides the cell.
             bool occluded = false;
             if (opq) {
-                const uint32_t fx = ccx * kCoarseExtent + (uint32_t)fc[0], fy = ccy * kCoarseExtent + (uint32_t)fc[1];
+                const uint32_t fx = ccx * kCoarseExtent + (at / kX & 3u), fy = ccy * kCoarseExtent + (at / kY & 3u);
                 if (fx < ftx && fy < fty) {
                     const uint2 o = __ldg(opq + (size_t)fy * ftx + fx);
                     occluded = o.x != 0u && zmax <= dequantize_depth01(o.y) - 1e-4f;
                 }
             }
-            if (!occluded) sink.cell((uint32_t)((fc[2] * 4 + fc[1]) * 4 + fc[0]));
-            if (fc[0] == f1[0] && fc[1] == f1[1] && fc[2] == f1[2]) break;
-            float m = wmin(wmin(tm[0], tm[1]), tm[2]);  // canonical_min_mask
-            int a = tm[0] == m ? 0 : (tm[1] == m ? 1 : 2);
-            if (a == 0) { fc[0] += step[0]; tm[0] += dd[0]; }
-            else if (a == 1) { fc[1] += step[1]; tm[1] += dd[1]; }
-            else { fc[2] += step[2]; tm[2] += dd[2]; }
-            if (fc[0] < 0 || fc[1] < 0 || fc[2] < 0 || fc[0] >= 4 || fc[1] >= 4 || fc[2] >= 16) break;
-            ++safety;
+            if (!occluded) sink.cell(at & 0xFFu);
+            if (((at ^ end) & (kStep - 1u)) == 0u) break;
+            const float m = wmin(wmin(tm[0], tm[1]), tm[2]);  // canonical_min_mask
+            if (tm[0] == m) { at += move[0]; tm[0] += dd[0]; }
+            else if (tm[1] == m) { at += move[1]; tm[1] += dd[1]; }
+            else { at += move[2]; tm[2] += dd[2]; }
+            if (((at ^ kIn) & kTop) != 0u) break;
         }
     }
 }
