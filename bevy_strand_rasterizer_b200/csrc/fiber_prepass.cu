@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(kFineThreads, 4) k_fine(const FrameParams* __r
 // ===========================================================================
 enum : int { kCount = 1, kFill = 2 };
 constexpr uint32_t kVisitThreads = 256;
-constexpr uint32_t kVisitSlots = 32;  // buffered visits per task; p99 is about 17 on the camera
+constexpr uint32_t kVisitSlots = 16;  // buffered visits per coarse tile of a task
 // Cell sort sizes: a thread sorts a cell of up to 8 references, a warp one of
 // up to 256 (32 lanes x 8 registers), a block anything longer.
 constexpr uint32_t kThreadSortMax = 8;
@@ -571,7 +571,7 @@ __device__ __forceinline__ void lut_slices(const fiber_coarse_depth_lut_entry* e
 template <bool kTel>
 struct VisitSink {
     uint32_t* page_table;
-    uint32_t* buf;  // this thread's column of the block buffer (stride kVisitThreads)
+    uint32_t* buf;  // this lane's column of the warp's buffer (stride 32)
     uint32_t cur, n;
     bool records;
     uint32_t* tel_slots;
@@ -582,7 +582,7 @@ struct VisitSink {
         return records;
     }
     __device__ __forceinline__ void cell(uint32_t c) {
-        if (n < kVisitSlots) buf[n * kVisitThreads] = cur | c;
+        if (n < kVisitSlots) buf[n * 32u] = cur | c;
         ++n;
     }
 };
@@ -767,47 +767,66 @@ __device__ __forceinline__ bool task_walk(const FrameParams& P, const PrepassArg
     return true;
 }
 
-// Coarse-tile 2-D DDA over the task's clipped range; each coarse tile is
-// walked by walk_page.
+// Coarse-tile 2-D DDA over the task's clipped range.
+struct TileWalk {
+    int32_t fx, fy, ex, ey, sx, sy;
+    float tx, ty, ddx, ddy;
+    uint32_t min_cx, max_cx, min_cy, max_cy, left;  // left: tiles the walk may still enter
+    __device__ __forceinline__ bool begin(const FrameParams& P, const TaskWalk& w, const ClipDir& pd) {
+        const fiber_frustum_desc& d = P.frusta[w.f];
+        const float sw = u2f(d.screen_width), sh = u2f(d.screen_height);
+        const uint32_t cpx = max(1u, d.froxel_size_x * kCoarseExtent);
+        const uint32_t cpy = max(1u, d.froxel_size_y * kCoarseExtent);
+        min_cx = w.min_cx, max_cx = w.max_cx, min_cy = w.min_cy, max_cy = w.max_cy;
+        F3 bmin = f3(u2f(min_cx * cpx), u2f(min_cy * cpy), 0.0f);
+        F3 bmax = f3(wmin(u2f((max_cx + 1u) * cpx), sw) - 1e-3f, wmin(u2f((max_cy + 1u) * cpy), sh) - 1e-3f, 1.0f);
+        F3 c0, c1;
+        if (!clip_segment_pre(w.p0, pd, bmin, bmax, c0, c1)) return false;
+        float x0 = div_by(c0.x, cpx), y0 = div_by(c0.y, cpy), x1 = div_by(c1.x, cpx), y1 = div_by(c1.y, cpy);
+        fx = iclamp(f2i(floorf(x0)), (int32_t)min_cx, (int32_t)max_cx);
+        fy = iclamp(f2i(floorf(y0)), (int32_t)min_cy, (int32_t)max_cy);
+        ex = iclamp(f2i(floorf(x1)), (int32_t)min_cx, (int32_t)max_cx);
+        ey = iclamp(f2i(floorf(y1)), (int32_t)min_cy, (int32_t)max_cy);
+        float dx = x1 - x0, dy = y1 - y0;
+        sx = sgn_i32(dx), sy = sgn_i32(dy);
+        float sdx = fabsf(dx) < 1e-6f ? 1e-6f : dx, sdy = fabsf(dy) < 1e-6f ? 1e-6f : dy;
+        // |sdx|, |sdy| are 1e-6 to 16384 coarse tiles.
+        const float rx = rcp_exact(sdx), ry = rcp_exact(sdy);
+        ddx = fabsf(rx), ddy = fabsf(ry);
+        float flx = floorf(x0), fly = floorf(y0);
+        tx = div_by_rcp(sx > 0 ? (flx + 1.0f) - x0 : flx - x0, sdx, rx);
+        ty = div_by_rcp(sy > 0 ? (fly + 1.0f) - y0 : fly - y0, sdy, ry);
+        if (fabsf(dx) < 1e-6f) tx = 1e38f;
+        if (fabsf(dy) < 1e-6f) ty = 1e38f;
+        left = (max_cx - min_cx + 1u) + (max_cy - min_cy + 1u) + 3u;
+        return true;
+    }
+    // Whether the walk is at a tile of its range.
+    __device__ __forceinline__ bool here() const {
+        return left != 0u && fx >= (int32_t)min_cx && fx <= (int32_t)max_cx && fy >= (int32_t)min_cy && fy <= (int32_t)max_cy;
+    }
+    // On to the next tile; false after the last.
+    __device__ __forceinline__ bool advance() {
+        if (fx == ex && fy == ey) return false;
+        if (tx <= ty) { fx += sx; tx += ddx; } else { fy += sy; ty += ddy; }
+        --left;
+        return true;
+    }
+};
+
+// Each coarse tile of the task is walked by walk_page.
 template <class Sink>
 __device__ __forceinline__ void walk_task(const FrameParams& P, const PrepassArgs& A, const TaskWalk& w,
                                           const uint2* opq, Sink& sink) {
     const fiber_frustum_desc& d = P.frusta[w.f];
-    const float sw = u2f(d.screen_width), sh = u2f(d.screen_height);
-    const uint32_t cpx = max(1u, d.froxel_size_x * kCoarseExtent);
-    const uint32_t cpy = max(1u, d.froxel_size_y * kCoarseExtent);
-    const uint32_t min_cx = w.min_cx, max_cx = w.max_cx, min_cy = w.min_cy, max_cy = w.max_cy;
-    F3 bmin = f3(u2f(min_cx * cpx), u2f(min_cy * cpy), 0.0f);
-    F3 bmax = f3(wmin(u2f((max_cx + 1u) * cpx), sw) - 1e-3f, wmin(u2f((max_cy + 1u) * cpy), sh) - 1e-3f, 1.0f);
-    F3 c0, c1;
     const ClipDir pd = clip_dir(w.p0, w.p1);  // shared by every coarse tile's clip
-    if (!clip_segment_pre(w.p0, pd, bmin, bmax, c0, c1)) return;
-    float x0 = div_by(c0.x, cpx), y0 = div_by(c0.y, cpy), x1 = div_by(c1.x, cpx), y1 = div_by(c1.y, cpy);
-    int32_t fx = iclamp(f2i(floorf(x0)), (int32_t)min_cx, (int32_t)max_cx);
-    int32_t fy = iclamp(f2i(floorf(y0)), (int32_t)min_cy, (int32_t)max_cy);
-    int32_t ex = iclamp(f2i(floorf(x1)), (int32_t)min_cx, (int32_t)max_cx);
-    int32_t ey = iclamp(f2i(floorf(y1)), (int32_t)min_cy, (int32_t)max_cy);
-    float dx = x1 - x0, dy = y1 - y0;
-    int32_t sx = sgn_i32(dx), sy = sgn_i32(dy);
-    float sdx = fabsf(dx) < 1e-6f ? 1e-6f : dx, sdy = fabsf(dy) < 1e-6f ? 1e-6f : dy;
-    // |sdx|, |sdy| are 1e-6 to 16384 coarse tiles.
-    const float rx = rcp_exact(sdx), ry = rcp_exact(sdy);
-    float ddx = fabsf(rx), ddy = fabsf(ry);
-    float flx = floorf(x0), fly = floorf(y0);
-    float tx = div_by_rcp(sx > 0 ? (flx + 1.0f) - x0 : flx - x0, sdx, rx);
-    float ty = div_by_rcp(sy > 0 ? (fly + 1.0f) - y0 : fly - y0, sdy, ry);
-    if (fabsf(dx) < 1e-6f) tx = 1e38f;
-    if (fabsf(dy) < 1e-6f) ty = 1e38f;
-    uint32_t safety = 0, max_steps = (max_cx - min_cx + 1u) + (max_cy - min_cy + 1u) + 2u;
-    for (;;) {
-        if (safety > max_steps) break;
-        if (fx < (int32_t)min_cx || fx > (int32_t)max_cx || fy < (int32_t)min_cy || fy > (int32_t)max_cy) break;
-        uint32_t local = (uint32_t)fy * d.coarse_tiles_x + (uint32_t)fx;
+    TileWalk t;
+    if (!t.begin(P, w, pd)) return;
+    while (t.here()) {
+        const uint32_t local = (uint32_t)t.fy * d.coarse_tiles_x + (uint32_t)t.fx;
         if (local < d.coarse_depth_tile_count)
-            walk_page(A, w.p0, pd, d, d.coarse_depth_tile_base + local, (uint32_t)fx, (uint32_t)fy, opq, sink);
-        if (fx == ex && fy == ey) break;
-        if (tx <= ty) { fx += sx; tx += ddx; } else { fy += sy; ty += ddy; }
-        ++safety;
+            walk_page(A, w.p0, pd, d, d.coarse_depth_tile_base + local, (uint32_t)t.fx, (uint32_t)t.fy, opq, sink);
+        if (!t.advance()) break;
     }
 }
 
@@ -822,66 +841,193 @@ __device__ __forceinline__ bool visits_unused(const PrepassArgs& A) {
     return *((volatile uint32_t*)&A.counters->visit_overflow) != 0u;
 }
 
-// K7: page marks + visit records. Warps walk 32 tasks at a time; each task's
-// first kVisitSlots visits go to shared memory, the warp reserves room for all
-// its visits with one atomic, and a task with more visits walks again to write
-// the rest. When the records do not fit (or slots exceed 24 bits) the pass
-// still marks every page and raises visit_overflow, which hands count and fill
-// to the walking kernels.
+// K7: page marks + visit records. A warp takes 32 tasks at a time, a lane per
+// task, and puts their coarse tiles into its queue; whenever 32 wait it walks
+// them, a lane per tile. A tile's visits go to shared memory and from there to
+// the warp's stage, which is written out with one reservation when it is full.
+// Batches that do not fit it, or hold a tile of more than kVisitSlots visits
+// (which is walked again to write the rest), are written directly. When the
+// records do not fit (or slots exceed 24 bits) the pass still marks every page and
+// raises visit_overflow, which hands count and fill to the walking kernels.
+// Bound by instruction issue: a task has 1.5 coarse tiles on average and 2.8 in
+// the longest of 32, so a lane that walked its own task's tiles (two clips, a
+// slice lookup and a cell walk each) idled half of the time. Medium frame 674 ->
+// 550 us, large 7.4 -> 6.5 ms, 16 views 3.3 -> 2.7, close-up 228 -> 175 us. What it
+// takes: the reservations are atomics on one address, which the device takes at
+// one per 3 ns (one per batch, without the stage: 960 us; a stage of 192 records
+// 10 ms on the large frame), and tiles queued task by task (one tile of each of
+// the 32 in turn: the fill's scattered accesses 257 -> 277 us). A queue of 128
+// tiles left less L1 and took 575 us.
 // kOpaque: the frame has opaque fine tiles (K0 ran); the variant without them
 // carries no cull code. kTel: count page candidates for the telemetry.
+constexpr uint32_t kTileQueue = 96;  // up to 31 left over and the 1.5 tiles per task of the next 32, mostly
+constexpr uint32_t kVisitStage = 256;
+struct VisitSmem {
+    uint4 p[kTileQueue], q[kTileQueue];  // (p0, p1.x), (p1.yz, tile x, y)
+    uint2 task[kTileQueue];              // (task, frustum)
+    uint32_t buf[kVisitSlots * 32u];     // [slot][lane] visits of this lane's tile
+    uint32_t stage_rec[kVisitStage], stage_task[kVisitStage];
+};
+constexpr size_t kVisitSmemBytes = sizeof(VisitSmem) * (kVisitThreads / 32u);
 template <bool kOpaque, bool kTel>
 __global__ void __launch_bounds__(kVisitThreads, 3) k_visit(const FrameParams* __restrict__ Pp, PrepassArgs A) {
     stamp_start(A.stamps, kStampVisit);
     if (frame_failed(A.counters)) return;
     const FrameParams& P = *Pp;
-    __shared__ uint32_t s_buf[kVisitSlots * kVisitThreads];
+    extern __shared__ VisitSmem s_visit[];
+    VisitSmem& sm = s_visit[threadIdx.x >> 5];
     const uint32_t n = *((volatile uint32_t*)&A.counters->tasks);
     const uint32_t n_cap = min(n, P.task_capacity);
     const bool records = P.visit_records != 0u;
     const uint2* opq = kOpaque ? A.opaque_tiles : nullptr;
     if (!records && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&A.counters->visit_overflow, 1u);
-    // Warps take 32 tasks at a time and reserve their records on their own,
-    // so a warp never waits for the slowest walk of its block.
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t warp_id = (blockIdx.x * kVisitThreads + threadIdx.x) >> 5;
-    const uint32_t warps = gridDim.x * (kVisitThreads / 32u);
-    for (uint32_t k0 = warp_id * 32u; k0 < n_cap; k0 += warps * 32u) {
-        const uint32_t k = k0 + lane;
-        TaskWalk w;
-        const bool ok = k < n_cap && task_walk(P, A, k, w);
-        VisitSink<kTel> vs{A.page_table, s_buf + threadIdx.x, 0u, 0u, records, A.tel_slots};
-        if (ok) walk_task(P, A, w, opq, vs);
-        if (!records) continue;
-        uint32_t incl = vs.n;
-#pragma unroll
-        for (uint32_t o = 1; o < 32u; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    // 16 tasks at a time if all of them still fit the warps: their tiles are one
+    // batch then, not two (tiny frame 13 us against 18).
+    const uint32_t warps = gridDim.x * (kVisitThreads / 32u), group = n_cap <= warps * 16u ? 16u : 32u;
+    const uint32_t stride = warps * group;
+    uint32_t k = (blockIdx.x * (kVisitThreads / 32u) + (threadIdx.x >> 5)) * group + lane;  // this lane's next task
+    uint32_t head = 0u, queued = 0u;                        // ring of queued tiles
+    bool more = false;                                      // the task has tiles left
+    TaskWalk w;
+    TileWalk t;
+    uint32_t staged = 0u;
+    auto ring = [](uint32_t at) { return at >= kTileQueue ? at - kTileQueue : at; };
+    auto in_frustum = [&](const TileWalk& c) {
+        const fiber_frustum_desc& d = P.frusta[w.f];
+        return (uint32_t)c.fy * d.coarse_tiles_x + (uint32_t)c.fx < d.coarse_depth_tile_count;
+    };
+    // This lane's task at its tile into the queue.
+    auto put = [&](uint32_t place) {
+        const uint32_t at = ring(place);
+        sm.p[at] = make_uint4(__float_as_uint(w.p0.x), __float_as_uint(w.p0.y), __float_as_uint(w.p0.z),
+                              __float_as_uint(w.p1.x));
+        sm.q[at] = make_uint4(__float_as_uint(w.p1.y), __float_as_uint(w.p1.z), (uint32_t)t.fx, (uint32_t)t.fy);
+        sm.task[at] = make_uint2(k - stride, w.f);
+    };
+    // Room for n visits; kInvalid if they do not fit.
+    auto reserve = [&](uint32_t n) -> uint32_t {
         uint32_t base = kInvalid;
-        if (lane == 31u && total > 0u && !visits_unused(A)) {
-            const unsigned long long b = atomicAdd(&A.counters->visits, (unsigned long long)total);
-            if (b + total <= (unsigned long long)P.ref_capacity) base = (uint32_t)b;
+        if (lane == 0u && n > 0u && !visits_unused(A)) {
+            const unsigned long long b = atomicAdd(&A.counters->visits, (unsigned long long)n);
+            if (b + n <= (unsigned long long)P.ref_capacity) base = (uint32_t)b;
             else atomicOr(&A.counters->visit_overflow, 1u);
         }
-        base = __shfl_sync(0xFFFFFFFFu, base, 31);
-        if (base != kInvalid && vs.n > 0u) {
-            // Visit records are placed in reservation order; the count and fill
-            // passes and the cell sort make the references independent of it.
-            const uint32_t at = base + incl - vs.n;
-            const uint32_t nb = min(vs.n, kVisitSlots);
-            // Streaming stores: the records are read once, by the count pass.
-            for (uint32_t j = 0; j < nb; ++j) {
-                __stcs(A.visit_rec + at + j, s_buf[j * kVisitThreads + threadIdx.x]);
-                __stcs(A.visit_task + at + j, k);
+        return __shfl_sync(0xFFFFFFFFu, base, 0);
+    };
+    // Visit records are placed in reservation order; the count and fill passes
+    // and the cell sort make the references independent of it. Streaming
+    // stores: the records are read once, by the count pass.
+    auto flush = [&] {
+        const uint32_t base = reserve(staged);
+        __syncwarp();
+        if (base != kInvalid)
+            for (uint32_t i = lane; i < staged; i += 32u) {
+                __stcs(A.visit_rec + base + i, sm.stage_rec[i]);
+                __stcs(A.visit_task + base + i, sm.stage_task[i]);
             }
-            if (vs.n > kVisitSlots) {
-                SpillSink sp{A.visit_rec, A.visit_task, at, k, vs.n, 0u, 0u};
-                walk_task(P, A, w, opq, sp);
+        __syncwarp();
+        staged = 0u;
+    };
+    for (;;) {
+        while (queued < 32u) {
+            if (!__any_sync(0xFFFFFFFFu, more)) {
+                if (k - lane >= n_cap) break;  // the warp's tasks are done
+                more = lane < group && k < n_cap && task_walk(P, A, k, w) && t.begin(P, w, clip_dir(w.p0, w.p1));
+                k += stride;
+                // Their tiles in task order, if the queue holds them all: the
+                // visits of a strand's neighbouring segments stay together, and
+                // so do the fill's accesses.
+                uint32_t tiles = 0u;
+                if (more) {
+                    TileWalk c = t;
+                    while (c.here()) {
+                        tiles += in_frustum(c) ? 1u : 0u;
+                        if (!c.advance()) break;
+                    }
+                }
+                uint32_t incl = tiles;
+#pragma unroll
+                for (uint32_t o = 1; o < 32u; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+                if (queued + total <= kTileQueue) {
+                    uint32_t at = head + queued + incl - tiles;
+                    while (tiles) {
+                        if (in_frustum(t)) {
+                            put(at++);
+                            --tiles;
+                        }
+                        t.advance();
+                    }
+                    queued += total;
+                    more = false;
+                    continue;
+                }
+            }
+            bool push = false;
+            if (more && t.here()) push = in_frustum(t);
+            else more = false;
+            const uint32_t pushed = __ballot_sync(0xFFFFFFFFu, push);
+            if (push) put(head + queued + (uint32_t)__popc(pushed & below));
+            queued += (uint32_t)__popc(pushed);
+            if (more) more = t.advance();
+        }
+        // The staged visits are written before they would overflow, and at the end.
+        if (queued == 0u) {
+            flush();
+            break;
+        }
+        __syncwarp();
+        const uint32_t batch = min(queued, 32u);
+        VisitSink<kTel> vs{A.page_table, sm.buf + lane, 0u, 0u, records, A.tel_slots};
+        uint32_t task = 0u;
+        // Walks this lane's tile of the batch.
+        auto walk = [&](auto& sink) {
+            const uint32_t at = ring(head + lane);
+            const uint4 a = sm.p[at], b = sm.q[at];
+            const uint2 c = sm.task[at];
+            task = c.x;
+            const fiber_frustum_desc& d = P.frusta[c.y];
+            const F3 p0 = f3(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z));
+            const F3 p1 = f3(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y));
+            walk_page(A, p0, clip_dir(p0, p1), d, d.coarse_depth_tile_base + b.w * d.coarse_tiles_x + b.z, b.z, b.w, opq, sink);
+        };
+        if (lane < batch) walk(vs);
+        if (records) {
+            uint32_t incl = vs.n;
+#pragma unroll
+            for (uint32_t o = 1; o < 32u; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+            const bool spilled = __any_sync(0xFFFFFFFFu, vs.n > kVisitSlots);
+            if (!spilled && total <= kVisitStage) {
+                if (staged + total > kVisitStage) flush();
+                const uint32_t at = staged + incl - vs.n;
+                for (uint32_t j = 0; j < vs.n; ++j) {
+                    sm.stage_rec[at + j] = sm.buf[j * 32u + lane];
+                    sm.stage_task[at + j] = task;
+                }
+                staged += total;
+            } else if (const uint32_t base = reserve(total); base != kInvalid && vs.n > 0u) {
+                const uint32_t at = base + incl - vs.n;
+                for (uint32_t j = 0; j < min(vs.n, kVisitSlots); ++j) {
+                    __stcs(A.visit_rec + at + j, sm.buf[j * 32u + lane]);
+                    __stcs(A.visit_task + at + j, task);
+                }
+                if (vs.n > kVisitSlots) {
+                    SpillSink sp{A.visit_rec, A.visit_task, at, task, vs.n, 0u, 0u};
+                    walk(sp);
+                }
             }
         }
+        __syncwarp();
+        head = ring(head + batch);
+        queued -= batch;
     }
 }
 
@@ -2042,14 +2188,25 @@ void launch_lut(const LaunchCtx& L, const PrepassArgs& A) {
 void launch_fine(const LaunchCtx& L, const PrepassArgs& A) {
     k_fine<<<L.sm_count * 6, kFineThreads, 0, L.stream>>>(L.P, L.inst, A);
 }
+template <bool kOpaque, bool kTel>
+static void launch_visit_as(const LaunchCtx& L, const PrepassArgs& A) {
+    static bool configured[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        cudaFuncSetAttribute(k_visit<kOpaque, kTel>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVisitSmemBytes);
+        if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    // The resident blocks (3 per SM), each looping over warps of tasks.
+    k_visit<kOpaque, kTel><<<L.sm_count * 3, kVisitThreads, kVisitSmemBytes, L.stream>>>(L.P, A);
+}
 void launch_visit(const LaunchCtx& L, const PrepassArgs& A) {
-    const unsigned grid = L.sm_count * 3;  // the resident blocks (3 per SM), each looping over warps of tasks
     if (L.telemetry) {
-        if (L.opaque) k_visit<true, true><<<grid, kVisitThreads, 0, L.stream>>>(L.P, A);
-        else k_visit<false, true><<<grid, kVisitThreads, 0, L.stream>>>(L.P, A);
+        if (L.opaque) launch_visit_as<true, true>(L, A);
+        else launch_visit_as<false, true>(L, A);
     } else {
-        if (L.opaque) k_visit<true, false><<<grid, kVisitThreads, 0, L.stream>>>(L.P, A);
-        else k_visit<false, false><<<grid, kVisitThreads, 0, L.stream>>>(L.P, A);
+        if (L.opaque) launch_visit_as<true, false>(L, A);
+        else launch_visit_as<false, false>(L, A);
     }
 }
 void launch_alloc(const LaunchCtx& L, const PrepassArgs& A) {

@@ -100,6 +100,18 @@ def test_heavy_and_light_runs(strands, light):
     _compare(scene)
 
 
+@pytest.mark.parametrize("strands,width,backend", [(1, 640, 0), (16, 640, 1), (33, 640, 0), (40, 96, 0), (700, 1280, 0)])
+def test_segments_across_many_tiles(strands, width, backend):
+    # Segments through the whole scene: more coarse tiles than a warp's queue
+    # holds, tiles with more visits than its buffer, batches longer than its
+    # stage; on a narrow screen, few tiles of many depth slices.
+    scene = build_scene("tiny", cull=False, width=width, height=width // 2, settings_overrides=dict(SETTINGS, fine_binning_backend=backend))
+    old = scene.assets[0][0]
+    lo, hi = np.asarray(old.aabb_min, np.float64), np.asarray(old.aabb_max, np.float64)
+    _strands(scene, np.random.default_rng(strands).uniform(lo, hi, (strands, 2, 3)))
+    _compare(scene)
+
+
 @pytest.mark.parametrize("scale", [1e-6, 1e13])
 def test_scene_scale(scale):
     # 1e13: clip coordinates beyond the range of the projection's shared
