@@ -150,14 +150,13 @@ def algorithmic_bytes(st, w, n_lights: int, K: int, D: int) -> dict:
 
     Per unit: 20 B / point + 16 B / strand (vertex float4 + index, meta), 28 B per
     binning task written and read (BinningTask 16 + ProjectedSegment 12), 8 B per
-    allocated cell (count + offset), 24 B per fine ref (written + read), 12 B per
-    binning task of cell-order key + material (written by k_visit), per visit
+    allocated cell (count + offset), 24 B per fine ref (written + read), 52 B per
+    binning task of depth key and raster record (written by k_fine), per visit
     (counted as fine refs): 8 B record written by k_visit, 16 B read/written by
     k_count_visits (record, rank, count), 20 B by k_fill_visits (record, rank,
-    task, offset read; task index written), 32 B by k_sort_cells (task index,
-    12 B key + material gathered, 16 B reference + key written); 64 B per work
-    item / tile run (written + read), 40 B per ref of endpoint gather in the
-    rasters, 40 + 8 L B per camera segment in shading, 12 B per camera pixel
+    task, offset read; task index written), 12 B by k_sort_cells (task index
+    read and written, 4 B key gathered); 64 B per work item / tile run (written +
+    read), 40 B per ref of endpoint gather in the rasters, 40 + 8 L B per camera segment in shading, 12 B per camera pixel
     (RGBA16F + R32F), 4 (K + 1) B per deep-opacity texel.
     """
     F = st.frustum_count
@@ -170,17 +169,16 @@ def algorithmic_bytes(st, w, n_lights: int, K: int, D: int) -> dict:
     WH = w.width * w.height
     dom = n_lights * 4 * (K + 1) * D * D
     per = {
-        "k_fine": 20 * P + 16 * S + sum(60 * n for n in tasks),  # + 32 B projected end points per task
-        "k_visit": sum(40 * n for n in tasks) + sum(8 * r for r in refs),
+        "k_fine": 20 * P + 16 * S + sum(80 * n for n in tasks),  # 28 B of task and projection, 52 B of key and record
+        "k_visit": sum(28 * n for n in tasks) + sum(8 * r for r in refs),
         "k_count_visits": sum(16 * r for r in refs),
         "k_fill_visits": sum(20 * r for r in refs),
         "k_prefix_pages": sum(8 * 256 * p for p in pages),
-        "k_emit+k_sort_cells": sum(32 * (wk + t) + 36 * r for wk, t, r in zip(work, runs, refs)),
-        # the rasters stage a reference from its 12 B record, its task index
-        # and the task's 32 B of projected end points
-        "k_shadow": sum(48 * refs[f] + 32 * (work[f] + runs[f]) for f in range(1, F)) + dom,
+        "k_emit+k_sort_cells": sum(32 * (wk + t) + 12 * r for wk, t, r in zip(work, runs, refs)),
+        # the rasters stage a reference from its task index and the task's 48 B record
+        "k_shadow": sum(52 * refs[f] + 32 * (work[f] + runs[f]) for f in range(1, F)) + dom,
         "k_shade": st.camera_tasks * (40 + 8 * n_lights),
-        "k_raster": 48 * refs[0] + 32 * (work[0] + runs[0]) + 12 * WH,
+        "k_raster": 52 * refs[0] + 32 * (work[0] + runs[0]) + 12 * WH,
     }
     # The frame's B_alg is the path's own formula (fixed before any kernel was
     # written); the per-kernel figures above add this implementation's records.
@@ -194,9 +192,9 @@ def algorithmic_bytes(st, w, n_lights: int, K: int, D: int) -> dict:
 # Kernels one fused frame launches: broad, lut, fine, visit, alloc, zero_pages,
 # count_visits, traverse<count> (returns at once unless the visit records did
 # not fit), prefix_pages, fill_visits, traverse<fill> (likewise),
-# compact_active, emit, sort_cells, sort_big_cells, shadow, shade, raster,
-# composite.
-KERNELS_PER_FRAME = 19
+# compact_active, emit, sort_cells, sort_big_cells, shadow (heavy and light
+# runs), shade, raster, composite.
+KERNELS_PER_FRAME = 20
 
 SPAN_TO_KERNEL = {
     "strand_prepass/fine": "k_fine",
