@@ -928,14 +928,19 @@ static fiber_status frame_begin_views(fiber_ctx* c, const fiber_view* views, uin
     P.fragment_counts = st.fragment_counts_enabled;
     P.width = views[0].camera_cfg.screen_width;
     P.height = views[0].camera_cfg.screen_height;
-    // Look-back status regions.
+    // Look-back status regions. A captured frame graph keeps their offsets, so
+    // they may follow only what its key holds: the tile table and the settings
+    // (page capacity). The fine prepass's region, whose size follows the strands
+    // (and not monotonely: 19,200 strands of two frusta take 600 tiles of 64,
+    // 18,000 take 1,126 of 32), therefore comes last.
     uint64_t fine_tiles_lb = P.fine_tile_base[P.F];
     uint64_t lb_sizes[kStageCount] = {fine_tiles_lb + 1, table / 1024 + 2, page_cap + 1, table / 1024 + 2,
                                       table / 1024 + 2};
+    constexpr uint32_t lb_order[kStageCount] = {kStageAlloc, kStagePrefix, kStageActive, kStageEmit, kStageFine};
     uint64_t lb_total = 0;
-    for (int i = 0; i < kStageCount; ++i) {
-        c->lb_offset[i] = (uint32_t)lb_total;
-        lb_total += lb_sizes[i];
+    for (uint32_t stage : lb_order) {
+        c->lb_offset[stage] = (uint32_t)lb_total;
+        lb_total += lb_sizes[stage];
     }
     const uint64_t L = n_lights, D = P.dom_size, S = P.shadow_map_size, K = P.K;
     const uint64_t FI = (uint64_t)I * P.F;

@@ -1,0 +1,59 @@
+"""One context whose captured frame graph serves several frames: what a replay
+must not keep of the frame it was captured for. Every fused frame is compared
+with the oracle of its own scene."""
+import numpy as np
+import pytest
+
+from bevy_strand_rasterizer_b200 import abi
+from common import build_scene, run_ref
+from test_gpu_parity import _exact
+
+pytestmark = pytest.mark.gpu
+
+DUMPS = (abi.DUMP_TASKS, abi.DUMP_PAGE_TABLE, abi.DUMP_PAGE_META, abi.DUMP_COUNTS, abi.DUMP_OFFSETS, abi.DUMP_REFS,
+         abi.DUMP_ACTIVE_TILES, abi.DUMP_WORK, abi.DUMP_RUNS, abi.DUMP_DOM_DEPTH, abi.DUMP_DOM_OPACITY,
+         abi.DUMP_SHADOW_MAP)
+
+
+def _frames(scenes, order):
+    """Renders scenes[k] for k in order in one context: the first frame node by
+    node (it sizes the buffers and captures nothing), the others fused on one
+    stream."""
+    import ctypes as C
+
+    import torch
+    from bevy_strand_rasterizer_b200.plugin import StrandRasterizerPlugin
+
+    stream = torch.cuda.Stream()
+    p = StrandRasterizerPlugin()
+    abi.check(p.lib.fiber_settings_set(p.ctx, C.byref(scenes[0].settings)), "fiber_settings_set")
+    for s in scenes:
+        p.add_geometry(*s.assets[0])
+    assets, refs = p.assets, [run_ref(s) for s in scenes]
+    for n, k in enumerate(order):
+        s, ref = scenes[k], refs[k]
+        p.assets = [assets[k]]
+        p._register()
+        p.frame_begin_raw(s.camera_cfg, s.cam, s.light_cfgs, s.lights_c, stream)
+        if n == 0:
+            p.render_nodes(stream=stream)
+        else:
+            p.frame_fused(stream=stream)
+        st, want = p.stats(), ref.stats()
+        for name in ("binning_tasks", "allocated_pages", "fine_refs", "active_tiles", "work_items", "overflow_flags"):
+            assert getattr(st, name) == getattr(want, name), f"frame {n}: {name}"
+        for what in DUMPS:
+            _exact(p.dump(what), ref.get(what), what)
+        color, ref_color = p.dump(abi.DUMP_COLOR).astype(np.float32), ref.get(abi.DUMP_COLOR).astype(np.float32)
+        assert float(np.max(np.abs(color - ref_color))) <= 2e-3, f"frame {n}: colour"
+    p.close()
+
+
+def test_fine_tiles_grow_under_a_reused_graph():
+    # With 148 SMs 60,000 strands of two frusta take 1,876 look-back tiles of
+    # the fine prepass, 19,200 take 600 (64 strands each) and 18,000 take 1,126
+    # (32 each): the third frame replays the graph captured for the second.
+    scenes = [build_scene("tiny", strands=n, points=4, cull=False,
+                          settings_overrides={"history_enabled": 0, "ref_capacity_factor": 16})
+              for n in (60_000, 19_200, 18_000)]
+    _frames(scenes, [0, 1, 2])
