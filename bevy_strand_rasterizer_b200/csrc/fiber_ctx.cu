@@ -400,7 +400,7 @@ fiber_status run_prepass(fiber_ctx* c, cudaStream_t s, const OpaqueSource* opaqu
     PrepassArgs As = A;
     set_stage(c, As, kStageActive);
     launch_compact_active(Ls, As, dp<unsigned long long>(c->d_lb) + c->lb_offset[kStageEmit]);
-    launch_emit(Ls, As, c->P.work_capacity);
+    launch_emit(Ls, As);
     launch_fill_walk(Ls, As);
     if (!csr) launch_fill(L, A);
     // The walking fill and the streaming one are one frame's alternatives: the
@@ -1151,9 +1151,10 @@ fiber_status fiber_frame_fused(fiber_ctx* c, const fiber_image* scene_color, con
         if (st == FIBER_OK && composite) st = run_composite(c, scene_color, scene_depth, out, s);
             return st;
     }
-    // Every kernel argument is stable across frames (per-frame values live in
-    // the device FrameParams), so one captured graph serves every frame of the
-    // same shape and buffers. The shape is whatever the host bakes into the
+    // Every kernel argument is stable across frames (per-frame values, the
+    // capacities among them, live in the device FrameParams), so one captured
+    // graph serves every frame of the same shape and buffers, whatever its
+    // strands. The shape is whatever the host bakes into the
     // launches: grid sizes (instances, coarse tiles), the shadow's shared
     // memory (K) and whether it runs (lights), the composite's image
     // extents, pitches and formats, and whether the walks cull against opaque

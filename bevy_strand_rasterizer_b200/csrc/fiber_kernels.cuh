@@ -208,7 +208,7 @@ void launch_fill_walk(const LaunchCtx& L, const PrepassArgs& A);
 void launch_fill(const LaunchCtx& L, const PrepassArgs& A);
 // lb_work: the look-back words of the work-item sums (stage kStageEmit).
 void launch_compact_active(const LaunchCtx& L, const PrepassArgs& A, unsigned long long* lb_work);
-void launch_emit(const LaunchCtx& L, const PrepassArgs& A, uint32_t work_capacity);
+void launch_emit(const LaunchCtx& L, const PrepassArgs& A);
 void launch_sort_cells(const LaunchCtx& L, const PrepassArgs& A);
 void launch_sort_big(const LaunchCtx& L, const PrepassArgs& A);
 void launch_telemetry(const LaunchCtx& L, const PrepassArgs& A);

@@ -1481,7 +1481,7 @@ __global__ void __launch_bounds__(kScanThreads) k_compact_active(const FramePara
 // the medium frame (3.1 M items, 62,894 tiles) and 4.7 ms on the large one
 // (22.5 M); sixteen lanes per coarse tile left the dense tiles' warps behind.
 // ===========================================================================
-__global__ void __launch_bounds__(256) k_emit(PrepassArgs A, uint32_t work_capacity) {
+__global__ void __launch_bounds__(256) k_emit(const FrameParams* __restrict__ Pp, PrepassArgs A) {
     stamp_start(A.stamps, kStampEmit);
     if (frame_failed(A.counters)) return;
     const uint32_t lt = threadIdx.x & 15u, half = threadIdx.x & 16u;
@@ -1489,6 +1489,7 @@ __global__ void __launch_bounds__(256) k_emit(PrepassArgs A, uint32_t work_capac
     const uint32_t halves = gridDim.x * (blockDim.x >> 4);
     const uint32_t first_shadow = *((volatile uint32_t*)&A.counters->camera_active);
     const uint32_t limit = heavy_limit(A.counters, A.shadow_blocks);
+    const uint32_t work_capacity = Pp->work_capacity;
     // Every lane of a warp takes every round.
     for (uint32_t p0 = 0; p0 < pages; p0 += halves) {
         const uint32_t page = p0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 4);
@@ -2243,8 +2244,8 @@ void launch_fill(const LaunchCtx& L, const PrepassArgs& A) {
 void launch_compact_active(const LaunchCtx& L, const PrepassArgs& A, unsigned long long* lb_work) {
     k_compact_active<<<L.sm_count * 4, kScanThreads, 0, L.stream>>>(L.P, A, lb_work);
 }
-void launch_emit(const LaunchCtx& L, const PrepassArgs& A, uint32_t work_capacity) {
-    k_emit<<<L.sm_count * 4, 256, 0, L.stream>>>(A, work_capacity);
+void launch_emit(const LaunchCtx& L, const PrepassArgs& A) {
+    k_emit<<<L.sm_count * 4, 256, 0, L.stream>>>(L.P, A);
 }
 void launch_sort_cells(const LaunchCtx& L, const PrepassArgs& A) {
     k_sort_cells<<<L.sm_count * 5, 256, 0, L.stream>>>(A);  // the resident blocks (5 per SM)

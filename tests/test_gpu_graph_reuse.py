@@ -1,11 +1,14 @@
 """One context whose captured frame graph serves several frames: what a replay
 must not keep of the frame it was captured for. Every fused frame is compared
 with the oracle of its own scene."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from bevy_strand_rasterizer_b200 import abi
 from common import build_scene, run_ref
+from oracle_bridge import capacities, coarse_tiles
 from test_gpu_parity import _exact
 
 pytestmark = pytest.mark.gpu
@@ -19,8 +22,6 @@ def _frames(scenes, order):
     """Renders scenes[k] for k in order in one context: the first frame node by
     node (it sizes the buffers and captures nothing), the others fused on one
     stream."""
-    import ctypes as C
-
     import torch
     from bevy_strand_rasterizer_b200.plugin import StrandRasterizerPlugin
 
@@ -57,3 +58,16 @@ def test_fine_tiles_grow_under_a_reused_graph():
                           settings_overrides={"history_enabled": 0, "ref_capacity_factor": 16})
               for n in (60_000, 19_200, 18_000)]
     _frames(scenes, [0, 1, 2])
+
+
+@pytest.mark.parametrize("backend", [0, 1])
+def test_work_items_grow_under_a_reused_graph(backend):
+    # The third frame replays the graph captured for 300 strands and has more
+    # work items than a frame of 300 strands has room for.
+    scenes = [build_scene("tiny", strands=n, points=m, width=320, height=240, dom=256, cull=False,
+                          settings_overrides={"history_enabled": 0, "ref_capacity_factor": 8,
+                                              "fine_binning_backend": backend}) for n, m in ((6_000, 16), (300, 4))]
+    cfgs = [c.to_c() for c in [scenes[1].camera_cfg] + scenes[1].light_cfgs]
+    room = capacities(300 * 3, 300, 2, coarse_tiles(cfgs), scenes[1].settings).work_capacity
+    assert run_ref(scenes[0]).stats().work_items > room
+    _frames(scenes, [0, 1, 0])
