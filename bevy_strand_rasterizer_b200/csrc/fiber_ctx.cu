@@ -84,7 +84,7 @@ __global__ void k_validate(InstanceView v, uint32_t* out) {
     atomicAdd(reinterpret_cast<unsigned long long*>(out + 2), segs);
 }
 
-constexpr int kGraphKeyWords = 12;  // what a captured frame graph depends on (fiber_frame_fused)
+constexpr int kGraphKeyWords = 13;  // what a captured frame graph depends on (fiber_frame_fused)
 
 }  // namespace
 
@@ -1156,7 +1156,8 @@ fiber_status fiber_frame_fused(fiber_ctx* c, const fiber_image* scene_color, con
     // graph serves every frame of the same shape and buffers, whatever its
     // strands. The shape is whatever the host bakes into the
     // launches: grid sizes (instances, coarse tiles), the shadow's shared
-    // memory (K) and whether it runs (lights), the composite's image
+    // memory (K) and whether it runs (lights), the deep-opacity page table's
+    // extent (lights, map size), the composite's image
     // extents, pitches and formats, and whether the walks cull against opaque
     // tiles (their kernel variant).
     auto pitch_of = [](const fiber_image* im) -> uint64_t {
@@ -1173,7 +1174,8 @@ fiber_status fiber_frame_fused(fiber_ctx* c, const fiber_image* scene_color, con
                                     scene_depth ? pitch_of(scene_depth) : 0u,
                                     ((uint64_t)c->P.width << 32) | c->P.height ^ (c->out_pixels << 1),
                                     ((uint64_t)c->P.I << 32) | c->P.total_coarse_tiles,
-                                    ((uint64_t)c->P.K << 32) | c->P.L};
+                                    ((uint64_t)c->P.K << 32) | c->P.L,
+                                    c->P.dom_size};
     bool reuse = c->graph && std::memcmp(key, c->graph_key, sizeof(key)) == 0;
     if (!reuse) {
         if (c->graph) {

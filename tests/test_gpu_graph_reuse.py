@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from bevy_strand_rasterizer_b200 import abi
+from bevy_strand_rasterizer_b200.plugin import FroxelConfig
 from common import build_scene, run_ref
 from oracle_bridge import capacities, coarse_tiles
 from test_gpu_parity import _exact
@@ -70,4 +71,13 @@ def test_work_items_grow_under_a_reused_graph(backend):
     cfgs = [c.to_c() for c in [scenes[1].camera_cfg] + scenes[1].light_cfgs]
     room = capacities(300 * 3, 300, 2, coarse_tiles(cfgs), scenes[1].settings).work_capacity
     assert run_ref(scenes[0]).stats().work_items > room
+    _frames(scenes, [0, 1, 0])
+
+
+def test_dom_size_under_a_reused_graph():
+    # 256^2 maps in 4 px tiles and 512^2 maps in 8 px tiles have the same coarse
+    # tiles; the third frame has four deep-opacity pages where the second had one.
+    scenes = [build_scene("tiny", dom=dom, settings_overrides={"history_enabled": 0, "dom_page_pool": 8})
+              for dom in (512, 256)]
+    scenes[1].light_cfgs = [FroxelConfig(256, 256, 4, 4, 16)]
     _frames(scenes, [0, 1, 0])
