@@ -479,7 +479,8 @@ __global__ void __launch_bounds__(Tile<kSplit>::threads, kSplit == 1 ? 12 : 3)
         // and fetches the following round's tasks: each warp takes 32 at a
         // time, a lane per reference (its record as k_fine wrote it for this
         // frustum, then its material), stores the entry and its candidate bits.
-        // Returns whether every entry is regular; has a block barrier.
+        // Returns whether every entry is regular and of finite opacity; has a block
+        // barrier.
         RoundTasks<T> next(s_items, n_items, R.ref_task, 0u, total, lane, warp);
         auto stage = [&](uint32_t e0, uint32_t n) -> bool {
             const float x0 = u2f(tx * fsx) + 0.5f, y0 = u2f(ty * fsy) + 0.5f;
@@ -509,6 +510,9 @@ __global__ void __launch_bounds__(Tile<kSplit>::threads, kSplit == 1 ? 12 : 3)
                         bits = ~0ull;
                         plain = true;
                     }
+                    // The regular walk deposits entries of coverage 0 too: 0 x an
+                    // infinite or NaN opacity would not leave the partials alone.
+                    plain = plain || !(fabsf(m.absorption_color[3]) <= 3.402823466e38f);
                 }
                 __syncwarp();
                 store_candidates(s_pmask, q, bits, lane);
@@ -628,7 +632,8 @@ __global__ void __launch_bounds__(Tile<kSplit>::threads, kSplit == 1 ? 12 : 3)
                             float cov0, cov1, qz0, qz1;
                             shadow_coverage2(mul2, ea, eb, pf, cov0, qz0, cov1, qz1);
                             // A coverage of 0 leaves the partials as they are
-                            // (a + (1 - a) w 0 = a), and few are: no branch.
+                            // (a + (1 - a) w 0 = a, the opacity being finite),
+                            // and few are: no branch.
                             deposit(ea, cov0, qz0);
                             if (b1 == kInvalid) break;
                             deposit(eb, cov1, qz1);
