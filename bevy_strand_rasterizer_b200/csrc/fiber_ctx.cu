@@ -553,7 +553,8 @@ fiber_status fiber_ctx_create(int device, uint64_t hbm_budget, fiber_ctx** out) 
     c->budget = hbm_budget;
     cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
     fiber_settings_default(&c->settings);
-    fiber_status st = FIBER_OK;
+    fiber_status st = configure_prepass() == cudaSuccess && configure_raster() == cudaSuccess ? FIBER_OK : FIBER_ECUDA;
+    if (st != FIBER_OK) cudaGetLastError();
     if (cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess) {
@@ -1149,7 +1150,7 @@ fiber_status fiber_frame_fused(fiber_ctx* c, const fiber_image* scene_color, con
         if (st == FIBER_OK) st = run_shading(c, s);
         if (st == FIBER_OK) st = run_raster(c, s);
         if (st == FIBER_OK && composite) st = run_composite(c, scene_color, scene_depth, out, s);
-            return st;
+        return st;
     }
     // Every kernel argument is stable across frames (per-frame values, the
     // capacities among them, live in the device FrameParams), so one captured
@@ -1190,7 +1191,7 @@ fiber_status fiber_frame_fused(fiber_ctx* c, const fiber_image* scene_color, con
         if (st == FIBER_OK) st = run_shading(c, s);
         if (st == FIBER_OK) st = run_raster(c, s);
         if (st == FIBER_OK && composite) st = run_composite(c, scene_color, scene_depth, out, s);
-            cudaError_t ce = cudaStreamEndCapture(s, &g);
+        cudaError_t ce = cudaStreamEndCapture(s, &g);
         if (st != FIBER_OK || ce != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
             c->hist_cur = hist_before;

@@ -188,6 +188,11 @@ struct LaunchCtx {
     bool telemetry;               // the prepass gathers telemetry
 };
 
+// The current device's kernel attributes (dynamic shared memory above 48 KB);
+// every context sets them before its first launch, whatever its thread.
+cudaError_t configure_prepass();
+cudaError_t configure_raster();
+
 // stamp: the launch starts the prepass (and its first span).
 void launch_opaque(const LaunchCtx& L, const PrepassArgs& A, const float* depth, uint32_t pitch, uint32_t samples,
                    uint32_t tiles, bool stamp);

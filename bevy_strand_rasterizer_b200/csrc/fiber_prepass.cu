@@ -2189,15 +2189,17 @@ void launch_lut(const LaunchCtx& L, const PrepassArgs& A) {
 void launch_fine(const LaunchCtx& L, const PrepassArgs& A) {
     k_fine<<<L.sm_count * 6, kFineThreads, 0, L.stream>>>(L.P, L.inst, A);
 }
+cudaError_t configure_prepass() {
+    const auto max_smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_visit<false, false>, max_smem, (int)kVisitSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_visit<false, true>, max_smem, (int)kVisitSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_visit<true, false>, max_smem, (int)kVisitSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_visit<true, true>, max_smem, (int)kVisitSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sort_big_cells, max_smem, (int)kBigSmemBytes);
+    return e;
+}
 template <bool kOpaque, bool kTel>
 static void launch_visit_as(const LaunchCtx& L, const PrepassArgs& A) {
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaFuncSetAttribute(k_visit<kOpaque, kTel>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVisitSmemBytes);
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
     // The resident blocks (3 per SM), each looping over warps of tasks.
     k_visit<kOpaque, kTel><<<L.sm_count * 3, kVisitThreads, kVisitSmemBytes, L.stream>>>(L.P, A);
 }
@@ -2258,13 +2260,6 @@ void launch_expand_refs(cudaStream_t s, const uint32_t* ref_task, const float4* 
     if (n) k_expand_refs<<<std::min(ceil_div_host(n, 256), 4096u), 256, 0, s>>>(ref_task, task_rec, n_tasks, n, out);
 }
 void launch_sort_big(const LaunchCtx& L, const PrepassArgs& A) {
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaFuncSetAttribute(k_sort_big_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBigSmemBytes);
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
     k_sort_big_cells<<<L.sm_count * 2, 256, kBigSmemBytes, L.stream>>>(A);
 }
 

@@ -1092,16 +1092,15 @@ __global__ void __launch_bounds__(Tile<1>::threads, 12) k_raster(const FramePara
     if (threadIdx.x == 0) stamp_end(R.stamps);
 }
 
+cudaError_t configure_raster() {
+    const auto max_smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_shadow<1>, max_smem, (int)shadow_smem_bytes<1>(kMaxDomSlices));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_shadow<4>, max_smem, (int)shadow_smem_bytes<4>(kMaxDomSlices));
+    return e;
+}
+
 template <uint32_t kSplit>
 static void launch_shadow_split(const LaunchCtx& L, const RenderArgs& R, uint32_t K) {
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaFuncSetAttribute(k_shadow<kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)shadow_smem_bytes<kSplit>(kMaxDomSlices));
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
     k_shadow<kSplit><<<L.sm_count * (kSplit == 1 ? 16 : 3), Tile<kSplit>::threads, shadow_smem_bytes<kSplit>(K), L.stream>>>(
         L.P, L.inst, R);
 }
