@@ -1537,23 +1537,26 @@ fiber_status fiber_dump(fiber_ctx* c, uint32_t what, void* host, uint64_t capaci
         case FIBER_DUMP_COUNTS: src = c->d_counts.p; bytes = (uint64_t)h.pages * kPageSize * 4; break;
         case FIBER_DUMP_OFFSETS: src = c->d_offsets.p; bytes = (uint64_t)h.pages * kPageSize * 4; break;
         case FIBER_DUMP_REFS: {
-            const uint64_t n = std::min(h.refs, P.ref_capacity);
+            const uint64_t n = std::min<uint64_t>(std::min(h.refs, P.ref_capacity), c->d_ref_task.bytes / 4u);
             bytes = n * sizeof(fiber_fine_seg_ref);
             if (host && capacity >= bytes && n) {
-                // The records live for this call only, outside the frames' buffers.
-                DevBuf refs;
-                if (cudaMalloc(&refs.p, bytes) != cudaSuccess) {
-                    cudaGetLastError();
-                    return FIBER_ENOMEM;
+                // The records, 12 B a reference, are made chunk by chunk in the
+                // cell lists' buffer, which nothing reads after the cell sort.
+                const uint64_t chunk = c->d_cells_small.bytes / sizeof(fiber_fine_seg_ref);
+                if (chunk == 0u || !c->d_task_rec.p) return FIBER_ENOTREADY;  // a frame_begin ran out of memory
+                const uint32_t tasks = std::min(h.tasks, P.task_capacity);
+                fiber_fine_seg_ref* out = static_cast<fiber_fine_seg_ref*>(host);
+                for (uint64_t at = 0; at < n; at += chunk) {
+                    const uint64_t m = std::min(chunk, n - at);
+                    launch_expand_refs(c->last_stream, dp<uint32_t>(c->d_ref_task) + at, dp<float4>(c->d_task_rec), tasks, m,
+                                       dp<fiber_fine_seg_ref>(c->d_cells_small));
+                    FIBER_CUDA(cudaGetLastError());
+                    FIBER_CUDA(cudaStreamSynchronize(c->last_stream));
+                    FIBER_CUDA(cudaMemcpy(out + at, c->d_cells_small.p, m * sizeof(fiber_fine_seg_ref),
+                                          cudaMemcpyDeviceToHost));
                 }
-                launch_expand_refs(c->last_stream, dp<uint32_t>(c->d_ref_task), dp<float4>(c->d_task_rec),
-                                   std::min(h.tasks, P.task_capacity), n, dp<fiber_fine_seg_ref>(refs));
-                cudaError_t e = cudaGetLastError();
-                if (e == cudaSuccess) e = cudaStreamSynchronize(c->last_stream);
-                if (e == cudaSuccess) e = cudaMemcpy(host, refs.p, bytes, cudaMemcpyDeviceToHost);
-                cudaFree(refs.p);
                 if (written) *written = bytes;
-                return e == cudaSuccess ? FIBER_OK : FIBER_ECUDA;
+                return FIBER_OK;
             }
             break;  // the size alone, or a buffer that is too small
         }
