@@ -92,6 +92,7 @@ struct fiber_ctx {
     int device = 0;
     uint64_t budget = 0, allocated = 0;
     int sm_count = 148;
+    uint32_t shadow_blocks = 0;  // resident blocks of the shadow raster at the settings' slices
     fiber_settings settings{};
     std::vector<Slab> slabs[5];
     // registered instances
@@ -239,7 +240,7 @@ PrepassArgs prepass_args(fiber_ctx* c) {
     A.page_items = dp<uint8_t>(c->d_page_items);
     A.active_list = dp<uint32_t>(c->d_active_list);
     A.heavy_list = dp<uint32_t>(c->d_heavy_list);
-    A.shadow_blocks = (uint32_t)c->sm_count * 12u;
+    A.shadow_blocks = c->shadow_blocks;
     A.work = dp<fiber_raster_work_item>(c->d_work);
     A.runs = dp<fiber_raster_tile_run>(c->d_runs);
     A.big_cells = dp<uint2>(c->d_big_cells);
@@ -279,7 +280,7 @@ RenderArgs render_args(fiber_ctx* c) {
     R.work = dp<fiber_raster_work_item>(c->d_work);
     R.runs = dp<fiber_raster_tile_run>(c->d_runs);
     R.heavy_list = dp<uint32_t>(c->d_heavy_list);
-    R.shadow_blocks = (uint32_t)c->sm_count * 12u;
+    R.shadow_blocks = c->shadow_blocks;
     R.ref_task = dp<uint32_t>(c->d_ref_task);
     R.task_rec = dp<float4>(c->d_task_rec);
     R.dom_depth = dp<float>(c->d_dom_depth);
@@ -555,6 +556,7 @@ fiber_status fiber_ctx_create(int device, uint64_t hbm_budget, fiber_ctx** out) 
     fiber_settings_default(&c->settings);
     fiber_status st = configure_prepass() == cudaSuccess && configure_raster() == cudaSuccess ? FIBER_OK : FIBER_ECUDA;
     if (st != FIBER_OK) cudaGetLastError();
+    c->shadow_blocks = (uint32_t)c->sm_count * shadow_blocks_per_sm(c->settings.dom_slices);
     if (cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess) {
@@ -607,7 +609,9 @@ fiber_status fiber_settings_set(fiber_ctx* c, const fiber_settings* s) {
     if (s->dom_slices == 0u || s->dom_slices > 16u) return FIBER_EINVAL;
     if (s->ref_capacity_factor == 0u || s->page_capacity_divisor == 0u) return FIBER_EINVAL;
     if (s->fine_binning_backend > 1u) return FIBER_EINVAL;  // SegmentScatter or PageCsr
+    cudaSetDevice(c->device);
     c->settings = *s;
+    c->shadow_blocks = (uint32_t)c->sm_count * shadow_blocks_per_sm(s->dom_slices);
     c->frame_ready = false;
     c->buffer_generation++;  // the captured frame graphs follow the settings' kernel sequence
     return FIBER_OK;

@@ -121,8 +121,9 @@ struct FrameCounters {
 static_assert(sizeof(FrameCounters) == 200 + 4 * (kMaxFrusta - 16), "FrameCounters layout");
 
 // A block of the shadow raster takes a run of n references in time n, so a run
-// that is large beside the references per resident block (12 per SM) is still
-// running when the other blocks have finished. Runs of kHeavyShare of that share
+// that is large beside the references per resident block (12 per SM up to 8
+// slices, 10 at 12, 8 at 16: shadow_blocks_per_sm) is still running when the
+// other blocks have finished. Runs of kHeavyShare of that share
 // or more are heavy: blocks of four threads per pixel render them.
 // Frames on both sides, one kernel against two: 177 runs of 10,145 references
 // 3.95 -> 2.55 ms a frame, 6,076 of 680 1.86 -> 1.45, 254 of 1,505 1.31 -> 0.95,

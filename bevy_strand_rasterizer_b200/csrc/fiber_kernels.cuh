@@ -193,6 +193,10 @@ struct LaunchCtx {
 cudaError_t configure_prepass();
 cudaError_t configure_raster();
 
+// Resident blocks per SM of the light runs' shadow raster at K slices (after
+// configure_raster).
+uint32_t shadow_blocks_per_sm(uint32_t K);
+
 // stamp: the launch starts the prepass (and its first span).
 void launch_opaque(const LaunchCtx& L, const PrepassArgs& A, const float* depth, uint32_t pitch, uint32_t samples,
                    uint32_t tiles, bool stamp);

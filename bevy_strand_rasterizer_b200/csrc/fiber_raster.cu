@@ -1099,6 +1099,14 @@ cudaError_t configure_raster() {
     return e;
 }
 
+uint32_t shadow_blocks_per_sm(uint32_t K) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_shadow<1>, (int)Tile<1>::threads, shadow_smem_bytes<1>(K)) !=
+        cudaSuccess)
+        cudaGetLastError();
+    return n > 0 ? (uint32_t)n : 1u;
+}
+
 template <uint32_t kSplit>
 static void launch_shadow_split(const LaunchCtx& L, const RenderArgs& R, uint32_t K) {
     k_shadow<kSplit><<<L.sm_count * (kSplit == 1 ? 16 : 3), Tile<kSplit>::threads, shadow_smem_bytes<kSplit>(K), L.stream>>>(
