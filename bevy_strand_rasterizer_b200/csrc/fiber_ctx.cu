@@ -133,6 +133,7 @@ struct fiber_ctx {
     bool epoch_dirty = false;
     // fiber_debug_stall_lookback: the next frame's look-back test hook.
     uint32_t stall_stage = 0, stall_tile = 0, stall_limit = 0;
+    uint32_t heavy_limit = 0;  // fiber_debug_heavy_limit
     // Smallest reference capacity of the next frames (the request server
     // raises it after a frame whose references overflowed).
     uint64_t ref_floor = 0;
@@ -780,6 +781,7 @@ static fiber_status frame_begin_views(fiber_ctx* c, const fiber_view* views, uin
     P.lb_stall_stage = c->stall_stage;
     P.lb_stall_tile = c->stall_tile;
     c->stall_stage = c->stall_tile = c->stall_limit = 0;
+    P.heavy_limit = c->heavy_limit;
     for (uint32_t i = 0; i < I; ++i) c->views[i].view = 0u;
     for (uint32_t v = 0; v < nv && nv > 1u; ++v)
         for (uint32_t i = views[v].instance_first; i < views[v].instance_first + views[v].instance_count; ++i)
@@ -1396,6 +1398,17 @@ fiber_status fiber_debug_stall_lookback(fiber_ctx* c, uint32_t stage, uint32_t t
     c->stall_stage = stage + 1u;
     c->stall_tile = tile;
     c->stall_limit = spin_limit;
+    return FIBER_OK;
+}
+
+fiber_status fiber_debug_heavy_limit(fiber_ctx* c, uint32_t limit, uint32_t* heavy_runs) {
+    if (!c) return FIBER_EINVAL;
+    c->heavy_limit = limit;
+    if (!heavy_runs) return FIBER_OK;
+    cudaSetDevice(c->device);
+    FIBER_CUDA(cudaStreamSynchronize(c->last_stream));
+    FIBER_CUDA(cudaMemcpy(heavy_runs, reinterpret_cast<const char*>(c->d_counters.p) + offsetof(FrameCounters, heavy_runs), 4,
+                          cudaMemcpyDeviceToHost));
     return FIBER_OK;
 }
 

@@ -459,7 +459,7 @@ fiber_status fiber_render_host(fiber_ctx* ctx, const void* scene_rgba16f_host,
 fiber_status fiber_stats_get(fiber_ctx* ctx, fiber_stats* out);
 
 /* ------------------------------------------------------------------------ */
-/* Test hook (no counterpart in the reference)                               */
+/* Test hooks (no counterpart in the reference)                              */
 /* ------------------------------------------------------------------------ */
 /* Makes the next frame's bounded device waits run out, to exercise the
  * FIBER_ETIMEDOUT path without faulting or hanging anything. In the frame of
@@ -471,6 +471,11 @@ fiber_status fiber_stats_get(fiber_ctx* ctx, fiber_stats* out);
  * after the stage then do nothing, and fiber_stats_get returns
  * FIBER_ETIMEDOUT with timeout_flags set. The frame after it is normal. */
 fiber_status fiber_debug_stall_lookback(fiber_ctx* ctx, uint32_t stage, uint32_t tile, uint32_t spin_limit);
+/* The context's next frames render shadow runs of at least `limit` references
+ * with the kernel for heavy runs (0: by the rule, 1: all runs, 0xFFFFFFFF:
+ * none); the images do not depend on it. heavy_runs, when not NULL, receives
+ * the last frame's count of heavy runs. */
+fiber_status fiber_debug_heavy_limit(fiber_ctx* ctx, uint32_t limit, uint32_t* heavy_runs);
 
 /* The last frame's prepass telemetry; EINVAL unless telemetry is enabled. */
 fiber_status fiber_telemetry_get(fiber_ctx* ctx, fiber_telemetry* out);
