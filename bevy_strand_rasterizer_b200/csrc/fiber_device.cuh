@@ -201,7 +201,8 @@ __device__ __forceinline__ F3 f3(float x, float y, float z) { return F3{x, y, z}
 //   sqrt  s0 = x y, s0 + (y / 2)(x - s0^2): equals the rounded root for every
 //         mantissa and exponent parity.
 // rcp and sqrt were compared with the operators over all 1.7e9 binary32 values
-// of magnitude 2^-100 to 2^101.
+// of magnitude 2^-100 to 2^101 (tests/exact_arithmetic.cu repeats this, the
+// quotients of odd divisors near a boundary and random ones).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float rcp_estimate(float x) {
     float r;
