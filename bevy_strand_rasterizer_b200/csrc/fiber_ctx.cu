@@ -23,6 +23,7 @@ using namespace fiber;
 namespace {
 
 constexpr int kSpanCount = 14;
+constexpr uint32_t kSpanEmit = 8, kSpanComposite = 12;
 const char* kSpanNames[kSpanCount] = {
     "strand_prepass/broad_instances",     // broad + depth-warp LUT
     "strand_prepass/fine",
@@ -30,9 +31,9 @@ const char* kSpanNames[kSpanCount] = {
     "strand_prepass/allocate_count_pages",
     "strand_prepass/binning",              // count
     "strand_prepass/prefix_fine_pages",
-    "strand_prepass/fill_segment_refs",
+    "strand_prepass/fill_segment_refs",     // until the cell sort starts, which waits for the emit too
     "strand_prepass/compact_active_tiles",  // beside the fill, as the emit is
-    "strand_prepass/emit_raster_work",      // canonical cell order
+    "strand_prepass/emit_raster_work",      // emit + canonical cell order, the sum of both
     "strand_shadow_rasterizer/rasterize",  // incl. fused stampback
     "strand_shading/shade",
     "strand_rasterizer/rasterize",
@@ -1660,16 +1661,26 @@ fiber_status fiber_span_times(fiber_ctx* c, float* ms, uint32_t n) {
     // without a composite after it the raster ends the frame.
     if (c->P.L == 0u) t[kStampShadow] = t[kStampShade];
     const bool composite = t[kStampComposite] > t[kStampRaster];
-    const uint32_t begin[kSpanCount] = {kStampBroad, kStampFine,    kStampVisit, kStampAlloc, kStampCount,
-                                        kStampPrefix, kStampFill,   kStampCompact, kStampSort, kStampShadow,
-                                        kStampShade,  kStampRaster, kStampComposite, kStampBroad};
-    const uint32_t end[kSpanCount] = {kStampFine,   kStampVisit, kStampAlloc, kStampCount,  kStampPrefix,
-                                      kStampFill,   kStampSort,  kStampEmit,  kStampShadow, kStampShade,
-                                      kStampRaster, composite ? kStampComposite : kStampEnd, kStampEnd, kStampEnd};
+    // The emit runs beside the fill, before the cell sort: its span is the sum
+    // of the two (the emit and the order of its references).
+    struct Interval { uint32_t begin, end; };
+    const Interval spans[kSpanCount] = {
+        {kStampBroad, kStampFine},   {kStampFine, kStampVisit},    {kStampVisit, kStampAlloc},
+        {kStampAlloc, kStampCount},  {kStampCount, kStampPrefix},  {kStampPrefix, kStampFill},
+        {kStampFill, kStampSort},    {kStampCompact, kStampCompactEnd}, {kStampSort, kStampSortEnd},
+        {kStampShadow, kStampShade}, {kStampShade, kStampRaster},
+        {kStampRaster, composite ? kStampComposite : kStampEnd},
+        {kStampComposite, kStampEnd}, {kStampBroad, kStampEnd}};
+    auto elapsed = [&](Interval x) -> float {
+        const unsigned long long b = t[x.begin], e = t[x.end];
+        return b != 0u && e >= b ? (float)((double)(e - b) * 1e-6) : -1.0f;
+    };
     for (uint32_t i = 0; i < n && i < (uint32_t)kSpanCount; ++i) {
-        const unsigned long long b = t[begin[i]], e = t[end[i]];
-        const bool ran = b != 0u && e >= b && (i != 12u || composite);
-        ms[i] = ran ? (float)((double)(e - b) * 1e-6) : -1.0f;
+        ms[i] = i == kSpanComposite && !composite ? -1.0f : elapsed(spans[i]);
+        if (i == kSpanEmit) {
+            const float emit = elapsed({kStampEmit, kStampEmitEnd});
+            ms[i] = emit >= 0.0f && ms[i] >= 0.0f ? ms[i] + emit : -1.0f;
+        }
     }
     return FIBER_OK;
 }

@@ -149,13 +149,15 @@ constexpr uint32_t kShadowRunCounter = 5, kCameraRunCounter = 6, kHeavyRunCounte
 
 // ---------------------------------------------------------------------------
 // Span stamps: each stage's first kernel writes the device clock (ns) when its
-// first block starts, the last ones keep the latest block's end, and the span
-// times are their differences. Event records between the kernels measured the
+// first block starts; stages whose end is not the next one's start (those beside
+// the main chain, the cell sort and the frame's last) keep their latest block's
+// end. The span times are their differences. Event records between the kernels measured the
 // same but cost 49 us of the tiny frame's 287 (a graph node each).
 // ---------------------------------------------------------------------------
 enum Stamp : uint32_t {
     kStampBroad = 0, kStampFine, kStampVisit, kStampAlloc, kStampCount, kStampPrefix, kStampFill, kStampCompact,
-    kStampEmit, kStampSort, kStampShadow, kStampShade, kStampRaster, kStampComposite, kStampEnd, kStampCount_
+    kStampEmit, kStampSort, kStampShadow, kStampShade, kStampRaster, kStampComposite, kStampEnd, kStampCompactEnd,
+    kStampEmitEnd, kStampSortEnd, kStampCount_
 };
 __device__ __forceinline__ unsigned long long device_clock_ns() {
     unsigned long long t;
@@ -165,8 +167,9 @@ __device__ __forceinline__ unsigned long long device_clock_ns() {
 __device__ __forceinline__ void stamp_start(unsigned long long* stamps, Stamp s) {
     if (blockIdx.x == 0u && threadIdx.x == 0u) stamps[s] = device_clock_ns();
 }
-// One thread of each block, when the block is done.
-__device__ __forceinline__ void stamp_end(unsigned long long* stamps) { atomicMax(stamps + kStampEnd, device_clock_ns()); }
+// One thread of each block that had work (the first one in any case), when the
+// block is done.
+__device__ __forceinline__ void stamp_end(unsigned long long* stamps, Stamp s) { atomicMax(stamps + s, device_clock_ns()); }
 
 // ---------------------------------------------------------------------------
 // WGSL builtin semantics

@@ -1404,11 +1404,13 @@ __global__ void __launch_bounds__(kScanThreads) k_compact_active(const FramePara
     const uint32_t cam_end = P.camera_tile_end * 16u;
     const uint32_t per_tile = kScanThreads * kScanItems;
     const uint32_t n_tiles = ceil_div(n, per_tile);
+    bool worked = blockIdx.x == 0u;
     for (;;) {
         if (threadIdx.x == 0) s_tile = atomicAdd(A.tile_counter, 1u);
         __syncthreads();
         const uint32_t tile = s_tile;
         if (tile >= n_tiles) break;
+        worked = true;
         const uint32_t e0 = tile * per_tile + threadIdx.x * kScanItems;  // n is a multiple of 16
         uint4 w = make_uint4(0u, 0u, 0u, 0u);
         if (e0 < n) w = *reinterpret_cast<const uint4*>(A.tile_work + e0);
@@ -1465,6 +1467,7 @@ __global__ void __launch_bounds__(kScanThreads) k_compact_active(const FramePara
         }
         __syncthreads();
     }
+    if (worked && threadIdx.x == 0u) stamp_end(A.stamps, kStampCompactEnd);
 }
 
 // ===========================================================================
@@ -1544,6 +1547,8 @@ __global__ void __launch_bounds__(256) k_emit(const FrameParams* __restrict__ Pp
         if (slot.x >= first_shadow && before < limit && before + load >= limit)
             A.heavy_list[atomicAdd(&A.counters->heavy_runs, 1u)] = slot.x;
     }
+    if ((blockIdx.x == 0u || blockIdx.x * (blockDim.x >> 4) < pages) && threadIdx.x == 0u)
+        stamp_end(A.stamps, kStampEmitEnd);
 }
 
 // A cell's entries are binning task indices; the canonical order is by depth key
@@ -2109,6 +2114,7 @@ __global__ void __launch_bounds__(256) k_sort_big_cells(PrepassArgs A) {
             __syncthreads();
         }
     }
+    if ((blockIdx.x == 0u || blockIdx.x < n_cells) && threadIdx.x == 0u) stamp_end(A.stamps, kStampSortEnd);
 }
 
 // finalize_telemetry (:2145-2188): totals, per-page candidate statistics and

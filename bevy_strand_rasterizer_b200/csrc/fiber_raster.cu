@@ -1089,7 +1089,7 @@ __global__ void __launch_bounds__(Tile<1>::threads, 12) k_raster(const FramePara
             if (P.fragment_counts) R.fragments[pi] = frags;
         }
     }
-    if (threadIdx.x == 0) stamp_end(R.stamps);
+    if (threadIdx.x == 0) stamp_end(R.stamps, kStampEnd);
 }
 
 cudaError_t configure_raster() {

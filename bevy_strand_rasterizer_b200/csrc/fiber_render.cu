@@ -406,7 +406,7 @@ __global__ void k_composite(CompositeArgs C) {
                                frag.z * frag.w + dst.z * oma, frag.w * 1.0f + dst.w * oma);
         store_px(C.out, C.out_pitch, C.out_format, x, y, o);
     }
-    if (threadIdx.x == 0) stamp_end(C.stamps);
+    if (threadIdx.x == 0) stamp_end(C.stamps, kStampEnd);
 }
 
 void launch_shade(const LaunchCtx& L, const RenderArgs& R) {
