@@ -86,6 +86,7 @@ fiber_status capture(fiber_batch* b, cudaStream_t s0) {
     for (uint32_t v = 0; v < n; ++v) costs[v] = (float)fiber_ctx_frame_cost(b->views[v]);
     std::vector<uint32_t> assign(n), seq(n);
     plan(costs.data(), n, nb, b->tuning.order, assign.data(), seq.data());
+    std::shared_lock<std::shared_mutex> capturing(g_capture_lock);
     BATCH_CUDA(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
     fiber_status st = FIBER_OK;
     cudaError_t ce = cudaEventRecord(b->fork, s0);
@@ -100,6 +101,7 @@ fiber_status capture(fiber_batch* b, cudaStream_t s0) {
     }
     cudaGraph_t g = nullptr;
     ce = cudaStreamEndCapture(s0, &g);
+    capturing.unlock();
     if (st == FIBER_OK && ce != cudaSuccess) st = FIBER_ECUDA;
     if (st == FIBER_OK && cudaGraphInstantiate(&b->graph, g, 0) != cudaSuccess) st = FIBER_ECUDA;
     if (g) cudaGraphDestroy(g);

@@ -12,6 +12,8 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
+#include <shared_mutex>
 #include <string>
 #include <vector>
 
@@ -173,6 +175,7 @@ fiber_status ensure(fiber_ctx* c, DevBuf& b, size_t bytes, bool zero = false) {
     if (b.p && b.bytes >= bytes) return FIBER_OK;
     if (c->budget && c->allocated - b.bytes + bytes > c->budget) return FIBER_ENOMEM;
     if (b.p) {
+        const std::unique_lock<std::shared_mutex> alone(g_capture_lock);
         cudaFree(b.p);
         c->allocated -= b.bytes;
         b.p = nullptr;
@@ -579,6 +582,7 @@ fiber_status fiber_ctx_create(int device, uint64_t hbm_budget, fiber_ctx** out) 
 fiber_status fiber_ctx_destroy(fiber_ctx* c) {
     if (!c) return FIBER_EINVAL;
     cudaSetDevice(c->device);
+    const std::unique_lock<std::shared_mutex> alone(g_capture_lock);
     cudaDeviceSynchronize();
     if (c->graph) cudaGraphExecDestroy(c->graph);
     for (auto& v : c->slabs)
@@ -658,6 +662,7 @@ fiber_status fiber_slab_free(fiber_ctx* c, uint32_t kind, uint32_t alloc_id) {
     int k = kind_slot(kind);
     if (k < 0 || alloc_id >= c->slabs[k].size() || !c->slabs[k][alloc_id].live) return FIBER_EINVAL;
     cudaSetDevice(c->device);
+    const std::unique_lock<std::shared_mutex> alone(g_capture_lock);
     cudaDeviceSynchronize();
     Slab& s = c->slabs[k][alloc_id];
     cudaFree(s.ptr);
@@ -671,7 +676,10 @@ fiber_status fiber_instance_set(fiber_ctx* c, const fiber_strand_instance* rows,
     if (!c || (n && !rows)) return FIBER_EINVAL;
     if (n >= 32768u) return FIBER_EINVAL;  // instance ids are 15 bits in the cell sort key
     cudaSetDevice(c->device);
-    FIBER_CUDA(cudaDeviceSynchronize());
+    {
+        const std::unique_lock<std::shared_mutex> alone(g_capture_lock);
+        FIBER_CUDA(cudaDeviceSynchronize());
+    }
     std::vector<InstanceView> views(n);
     std::vector<uint64_t> segs(n, 0);
     uint64_t tot_seg = 0, tot_pts = 0, tot_str = 0;
@@ -1191,6 +1199,7 @@ fiber_status fiber_frame_fused(fiber_ctx* c, const fiber_image* scene_color, con
             c->graph = nullptr;
         }
         cudaGraph_t g = nullptr;
+        std::shared_lock<std::shared_mutex> capturing(g_capture_lock);
         FIBER_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         const int hist_before = c->hist_cur;
         fiber_status st = run_prepass(c, s, op);
@@ -1199,6 +1208,7 @@ fiber_status fiber_frame_fused(fiber_ctx* c, const fiber_image* scene_color, con
         if (st == FIBER_OK) st = run_raster(c, s);
         if (st == FIBER_OK && composite) st = run_composite(c, scene_color, scene_depth, out, s);
         cudaError_t ce = cudaStreamEndCapture(s, &g);
+        capturing.unlock();
         if (st != FIBER_OK || ce != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
             c->hist_cur = hist_before;

@@ -5,8 +5,14 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <shared_mutex>
 
 #include "fiber.h"
+
+// Contexts of several threads: a device-wide synchronisation (and what frees
+// memory) fails while another thread captures a frame graph, and spoils the
+// capture. Captures hold this lock shared, device-wide synchronisations alone.
+inline std::shared_mutex g_capture_lock;
 
 // A context's instance table with everything fiber_instance_set derives from
 // it (validated device views, segment totals). Saving one per resident scene
