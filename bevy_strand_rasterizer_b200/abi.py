@@ -201,7 +201,7 @@ EXPORTS = [
     "fiber_server_start", "fiber_server_submit", "fiber_server_wait", "fiber_server_destroy", "fiber_server_now_ns",
     "fiber_batch_create", "fiber_batch_set_tuning", "fiber_batch_get_tuning", "fiber_batch_launch",
     "fiber_batch_tune", "fiber_batch_destroy", "fiber_batch_plan",
-    "fiber_prefix_pages_noalloc", "fiber_debug_stall_lookback", "fiber_debug_heavy_limit",
+    "fiber_prefix_pages_noalloc", "fiber_debug_stall_lookback", "fiber_debug_shadow_kernel",
 ]
 
 _LIB = None
@@ -244,7 +244,7 @@ def load_library(path: Path | str | None = None) -> C.CDLL:
         "fiber_render_host": (C.c_int, [vp, vp, vp, vp, vp]),
         "fiber_stats_get": (C.c_int, [vp, pp(Stats)]),
         "fiber_debug_stall_lookback": (C.c_int, [vp, u32, u32, u32]),
-        "fiber_debug_heavy_limit": (C.c_int, [vp, u32, pp(u32)]),
+        "fiber_debug_shadow_kernel": (C.c_int, [vp, u32, pp(u32)]),
         "fiber_telemetry_get": (C.c_int, [vp, pp(Telemetry)]),
         "fiber_dump": (C.c_int, [vp, u32, vp, C.c_uint64, pp(C.c_uint64)]),
         "fiber_output_image": (C.c_int, [vp, u32, pp(Image)]),

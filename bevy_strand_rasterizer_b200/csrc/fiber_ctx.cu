@@ -136,7 +136,7 @@ struct fiber_ctx {
     bool epoch_dirty = false;
     // fiber_debug_stall_lookback: the next frame's look-back test hook.
     uint32_t stall_stage = 0, stall_tile = 0, stall_limit = 0;
-    uint32_t heavy_limit = 0;  // fiber_debug_heavy_limit
+    uint32_t shadow_kernel = 0;  // fiber_debug_shadow_kernel
     // Smallest reference capacity of the next frames (the request server
     // raises it after a frame whose references overflowed).
     uint64_t ref_floor = 0;
@@ -222,6 +222,11 @@ LaunchCtx launch_ctx(fiber_ctx* c, cudaStream_t s) {
     return L;
 }
 
+// What heavy_limit takes: the resident blocks, or the test hook's extremes.
+uint32_t shadow_blocks(const fiber_ctx* c) {
+    return c->shadow_kernel == 0u ? c->shadow_blocks : c->shadow_kernel == 1u ? 0u : 0xFFFFFFFFu;
+}
+
 PrepassArgs prepass_args(fiber_ctx* c) {
     PrepassArgs A{};
     A.counters = dp<FrameCounters>(c->d_counters);
@@ -245,7 +250,7 @@ PrepassArgs prepass_args(fiber_ctx* c) {
     A.page_items = dp<uint8_t>(c->d_page_items);
     A.active_list = dp<uint32_t>(c->d_active_list);
     A.heavy_list = dp<uint32_t>(c->d_heavy_list);
-    A.shadow_blocks = c->shadow_blocks;
+    A.shadow_blocks = shadow_blocks(c);
     A.work = dp<fiber_raster_work_item>(c->d_work);
     A.runs = dp<fiber_raster_tile_run>(c->d_runs);
     A.big_cells = dp<uint2>(c->d_big_cells);
@@ -285,7 +290,7 @@ RenderArgs render_args(fiber_ctx* c) {
     R.work = dp<fiber_raster_work_item>(c->d_work);
     R.runs = dp<fiber_raster_tile_run>(c->d_runs);
     R.heavy_list = dp<uint32_t>(c->d_heavy_list);
-    R.shadow_blocks = c->shadow_blocks;
+    R.shadow_blocks = shadow_blocks(c);
     R.ref_task = dp<uint32_t>(c->d_ref_task);
     R.task_rec = dp<float4>(c->d_task_rec);
     R.dom_depth = dp<float>(c->d_dom_depth);
@@ -790,7 +795,6 @@ static fiber_status frame_begin_views(fiber_ctx* c, const fiber_view* views, uin
     P.lb_stall_stage = c->stall_stage;
     P.lb_stall_tile = c->stall_tile;
     c->stall_stage = c->stall_tile = c->stall_limit = 0;
-    P.heavy_limit = c->heavy_limit;
     for (uint32_t i = 0; i < I; ++i) c->views[i].view = 0u;
     for (uint32_t v = 0; v < nv && nv > 1u; ++v)
         for (uint32_t i = views[v].instance_first; i < views[v].instance_first + views[v].instance_count; ++i)
@@ -1412,9 +1416,10 @@ fiber_status fiber_debug_stall_lookback(fiber_ctx* c, uint32_t stage, uint32_t t
     return FIBER_OK;
 }
 
-fiber_status fiber_debug_heavy_limit(fiber_ctx* c, uint32_t limit, uint32_t* heavy_runs) {
-    if (!c) return FIBER_EINVAL;
-    c->heavy_limit = limit;
+fiber_status fiber_debug_shadow_kernel(fiber_ctx* c, uint32_t which, uint32_t* heavy_runs) {
+    if (!c || which > 2u) return FIBER_EINVAL;
+    if (which != c->shadow_kernel) c->buffer_generation++;  // captured frame graphs hold the old choice
+    c->shadow_kernel = which;
     if (!heavy_runs) return FIBER_OK;
     cudaSetDevice(c->device);
     FIBER_CUDA(cudaStreamSynchronize(c->last_stream));

@@ -87,7 +87,6 @@ struct FrameParams {
     uint32_t layer_frustum[kMaxFrusta];  // frustum of each DOM layer
     uint32_t out_base[kMaxFrusta];       // first pixel of a camera's colour / depth / fragment image
     uint32_t fine_per_warp;              // strands per warp of k_fine's tiles
-    uint32_t heavy_limit;                // fiber_debug_heavy_limit: references of a heavy shadow run (0: heavy_limit())
     uint32_t fine_tile_base[kMaxFrusta + 1];  // k_fine's tiles of each frustum (prefix)
     uint32_t view_strand0[kMaxViews], view_strands[kMaxViews];  // a view's strands (global strand indices)
     uint32_t view_layer0[kMaxViews], view_layers[kMaxViews];    // a view's lights (DOM layers, light indices)
@@ -133,8 +132,9 @@ static_assert(sizeof(FrameCounters) == 200 + 4 * (kMaxFrusta - 16), "FrameCounte
 // medium frame took 4.15, 4.05 and 3.91 ms (four threads a pixel do the walk's
 // work at half its rate), at 1.5 the close-up 2.07 against 1.95.
 constexpr float kHeavyShare = 0.5f;
-__device__ __forceinline__ uint32_t heavy_limit(const FrameParams& P, const FrameCounters* c, uint32_t shadow_blocks) {
-    if (P.heavy_limit != 0u) return P.heavy_limit;
+// With 0xFFFFFFFF blocks the limit is 1 (every run is heavy), with 0 blocks it is
+// 0xFFFFFFFF (none): fiber_debug_shadow_kernel.
+__device__ __forceinline__ uint32_t heavy_limit(const FrameCounters* c, uint32_t shadow_blocks) {
     const float share = (float)*((const volatile unsigned long long*)&c->shadow_refs) / (float)shadow_blocks;
     return __float2uint_rz(fmaxf(kHeavyShare * share, 1.0f));
 }

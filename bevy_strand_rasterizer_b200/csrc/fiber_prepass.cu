@@ -1491,7 +1491,7 @@ __global__ void __launch_bounds__(256) k_emit(const FrameParams* __restrict__ Pp
     const uint32_t pages = *((volatile uint32_t*)&A.counters->pages);
     const uint32_t halves = gridDim.x * (blockDim.x >> 4);
     const uint32_t first_shadow = *((volatile uint32_t*)&A.counters->camera_active);
-    const uint32_t limit = heavy_limit(*Pp, A.counters, A.shadow_blocks);
+    const uint32_t limit = heavy_limit(A.counters, A.shadow_blocks);
     const uint32_t work_capacity = Pp->work_capacity;
     // Every lane of a warp takes every round.
     for (uint32_t p0 = 0; p0 < pages; p0 += halves) {

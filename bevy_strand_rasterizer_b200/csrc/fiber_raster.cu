@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(Tile<kSplit>::threads, kSplit == 1 ? 12 : 3)
     const uint32_t first = *((volatile uint32_t*)&R.counters->camera_active);
     const uint32_t n_runs = kSplit == 1 ? *((volatile uint32_t*)&R.counters->active_tiles) - first
                                         : *((volatile uint32_t*)&R.counters->heavy_runs);
-    const uint32_t limit = heavy_limit(P, R.counters, R.shadow_blocks);
+    const uint32_t limit = heavy_limit(R.counters, R.shadow_blocks);
     uint32_t* counter = &R.counters->tile_counter[kSplit == 1 ? kShadowRunCounter : kHeavyRunCounter];
     uint32_t claim = 0u;
     if (threadIdx.x == 0) claim = atomicAdd(counter, 1u);

@@ -471,11 +471,11 @@ fiber_status fiber_stats_get(fiber_ctx* ctx, fiber_stats* out);
  * after the stage then do nothing, and fiber_stats_get returns
  * FIBER_ETIMEDOUT with timeout_flags set. The frame after it is normal. */
 fiber_status fiber_debug_stall_lookback(fiber_ctx* ctx, uint32_t stage, uint32_t tile, uint32_t spin_limit);
-/* The context's next frames render shadow runs of at least `limit` references
- * with the kernel for heavy runs (0: by the rule, 1: all runs, 0xFFFFFFFF:
- * none); the images do not depend on it. heavy_runs, when not NULL, receives
- * the last frame's count of heavy runs. */
-fiber_status fiber_debug_heavy_limit(fiber_ctx* ctx, uint32_t limit, uint32_t* heavy_runs);
+/* The context's next frames render their shadow runs with the kernel that the
+ * rule gives each run (which = 0), all with the one for light runs (1) or all
+ * with the one for heavy runs (2); the images do not depend on it. heavy_runs,
+ * when not NULL, receives the last frame's count of heavy runs. */
+fiber_status fiber_debug_shadow_kernel(fiber_ctx* ctx, uint32_t which, uint32_t* heavy_runs);
 
 /* The last frame's prepass telemetry; EINVAL unless telemetry is enabled. */
 fiber_status fiber_telemetry_get(fiber_ctx* ctx, fiber_telemetry* out);

@@ -15,27 +15,27 @@ from test_gpu_parity import _compare
 
 pytestmark = pytest.mark.gpu
 
-NONE = 0xFFFFFFFF
+LIGHT, HEAVY = 1, 2
 
 
-def _heavy_runs(p, limit=0):
+def _heavy_runs(p, which=0):
     n = C.c_uint32()
-    abi.check(p.lib.fiber_debug_heavy_limit(p.ctx, limit, C.byref(n)), "fiber_debug_heavy_limit")
+    abi.check(p.lib.fiber_debug_shadow_kernel(p.ctx, which, C.byref(n)), "fiber_debug_shadow_kernel")
     return n.value
 
 
-@pytest.fixture(params=[NONE, 1], ids=["light", "heavy"])
+@pytest.fixture(params=[LIGHT, HEAVY], ids=["light", "heavy"])
 def kernel(request, monkeypatch):
     """Every frame's shadow runs by one kernel; checks that it was that one."""
-    limit, begin, stats = request.param, StrandRasterizerPlugin.frame_begin_raw, StrandRasterizerPlugin.stats
+    which, begin, stats = request.param, StrandRasterizerPlugin.frame_begin_raw, StrandRasterizerPlugin.stats
 
     def begin_raw(self, *args, **kw):
-        _heavy_runs(self, limit)
+        _heavy_runs(self, which)
         return begin(self, *args, **kw)
 
     def checked(self, *args, **kw):
         s = stats(self, *args, **kw)
-        assert _heavy_runs(self, limit) == (s.shadow_runs if limit == 1 else 0)
+        assert _heavy_runs(self, which) == (s.shadow_runs if which == HEAVY else 0)
         return s
 
     monkeypatch.setattr(StrandRasterizerPlugin, "frame_begin_raw", begin_raw)
