@@ -127,7 +127,9 @@ static_assert(sizeof(FrameCounters) == 200 + 4 * (kMaxFrusta - 16), "FrameCounte
 // or more are heavy: blocks of four threads per pixel render them.
 // Frames on both sides, one kernel against two: 177 runs of 10,145 references
 // 3.95 -> 2.55 ms a frame, 6,076 of 680 1.86 -> 1.45, 254 of 1,505 1.31 -> 0.95,
-// tiny (124 of 100) 0.47 -> 0.45; frames whose runs are even keep their times
+// tiny (124 of 100) 0.47 -> 0.45 (one frame of a few hundred heavy runs, which
+// all run at once, varies by the SMs they share: 400 runs 0.72 to 1.2 ms of
+// raster, 0.9 on average); frames whose runs are even keep their times
 // (medium 3.86 / 3.87, large 52.5 / 52.7). At shares of 0.06, 0.125 and 0.25 the
 // medium frame took 4.15, 4.05 and 3.91 ms (four threads a pixel do the walk's
 // work at half its rate), at 1.5 the close-up 2.07 against 1.95.

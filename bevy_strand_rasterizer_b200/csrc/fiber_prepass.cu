@@ -849,8 +849,8 @@ __device__ __forceinline__ bool visits_unused(const PrepassArgs& A) {
 // (which is walked again to write the rest), are written directly. When the
 // records do not fit (or slots exceed 24 bits) the pass still marks every page and
 // raises visit_overflow, which hands count and fill to the walking kernels.
-// Bound by instruction issue: a task has 1.5 coarse tiles on average and 2.8 in
-// the longest of 32, so a lane that walked its own task's tiles (two clips, a
+// Bound by instruction issue (62 % of the slots, 24 of 32 lanes) and the loads
+// between them: a task has 1.5 coarse tiles on average and 2.8 in the longest of 32, so a lane that walked its own task's tiles (two clips, a
 // slice lookup and a cell walk each) idled half of the time. Medium frame 674 ->
 // 550 us, large 7.4 -> 6.5 ms, 16 views 3.3 -> 2.7, close-up 228 -> 175 us. What it
 // takes: the reservations are atomics on one address, which the device takes at
@@ -1815,10 +1815,11 @@ __device__ __forceinline__ void sort_cells(const PrepassArgs& A, SortSpanSmem* s
 // lists k_prefix_pages made: a warp per 32 cells of 2..8 references (a lane per
 // cell), eight cells of 9..16 references per warp (four lanes each), four of
 // 17..32 (eight lanes each), then a warp per larger cell of up to 256. Bound by the networks' 64-bit compares and selects (ALU pipe
-// 71 % busy); the key gathers hide behind them (2 % of the time). The start
-// wrote 20 B of reference, key and task per entry and sorted a word beside its
-// task by branches: 0.57 -> 0.19 ms for the medium frame, 11.8 -> 4.9 ms for
-// the large frame's 349 M references.
+// 71 % busy). An earlier form wrote 20 B of reference, key and task per entry and
+// sorted a word beside its task by branches: 0.57 -> 0.19 ms for the medium frame,
+// 11.0 -> 4.3 ms for the large frame's 349 M references. Frames with strands out
+// of order (ByRecord: 16 B more gathered per entry, small cells one by one) take
+// about 0.38 and 10.4 ms.
 __global__ void __launch_bounds__(256, 5) k_sort_cells(PrepassArgs A) {
     stamp_start(A.stamps, kStampSort);
     if (frame_failed(A.counters)) return;

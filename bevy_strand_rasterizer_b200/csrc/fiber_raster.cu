@@ -17,9 +17,11 @@
 // 4 from each item's start, (w0 over w1) over (w2 over w3), early out after each
 // item once alpha > 0.98.
 //
-// Both rasters are bound by instruction issue, so the walk is written for few
-// instructions with the results of the plain binary32 formulas, bit for bit:
-// packed pairs (.f32x2) for what comes in pairs, and quotients and square roots
+// Both rasters are bound by the walk's instructions: on the benchmark's medium
+// frame 71 and 72 % of the issue slots are taken, by 24 and 18 of 32 lanes, and
+// what is left are fixed-latency waits, staging loads and barriers at 24 warps
+// per SM. So the walk is written for few instructions, with the results of the
+// plain binary32 formulas bit for bit: packed pairs (.f32x2) for what comes in pairs, and quotients and square roots
 // by a reciprocal estimate and fused corrections (fiber_device.cuh) instead of
 // the general-range division and square root.
 #include "fiber_kernels.cuh"
@@ -353,9 +355,9 @@ struct Walk {
 // worker's partial sees its entries in the reference's order; the four
 // partials combine in worker order as the reference does.
 //
-// Medium frame (30,499 runs, 128 M covered pairs): 1.145 G -> 0.716 G warp
-// instructions, 1.54 -> 1.09 ms; large (226,793 runs, 2.97 G pairs): 29.2 ->
-// 20.1 ms. About a third of it is staging (364 warp instructions per 32
+// The benchmark's medium frame (21,988 runs): 1.145 G -> 0.715 G warp
+// instructions, 1.31 -> 0.99 ms of the light runs' launch; large (226,793 runs,
+// 2.97 G covered pairs): 29.2 -> 17.5 ms. About a third of it is staging (364 warp instructions per 32
 // references), the rest the walk. Rounds of 64, 192 and 256 references were
 // slower (1.20, 1.17, 1.26 ms against 1.14), 14 and 16 blocks per SM too (shared
 // memory holds 12 at 8 slices).
@@ -793,8 +795,8 @@ void launch_dom_paging(const LaunchCtx& L, const RenderArgs& R, uint32_t table_e
 // group is held as at most two halves and most groups, which hold one covered
 // entry, are that entry. Group and item state carry over from round to round.
 //
-// Medium frame (32,395 runs, 29 M covered pairs): 620 M -> 385 M warp
-// instructions, 0.80 -> 0.56 ms; large: 3.50 -> 2.48 ms.
+// The benchmark's medium frame (25,918 runs): 620 M -> 382 M warp instructions,
+// 0.68 -> 0.49 ms; large: 3.50 -> 1.84 ms.
 // ===========================================================================
 constexpr uint32_t kCamEntry = 5;  // float4 words of a staged entry
 
